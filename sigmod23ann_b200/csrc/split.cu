@@ -10,8 +10,8 @@
 //                      of its whole range (:195-197, :273-278), eight lanes
 //                      per point in the reference's FMA-chain order
 //   k_lloyd_seq        per-side double sums in the Lloyd set's order and the
-//                      new centres (:170-186, :227-259), one CTA per node fed
-//                      by bulk copies
+//                      new centres (:170-186, :227-259), one CTA per node and
+//                      32 dimensions
 //   k_scan_items       exclusive scan of per-tile side-true counts
 //   k_scatter          stable partition, side-true first (std::stable_partition
 //                      at :195, the group memcpy at :301-304)
@@ -331,126 +331,215 @@ __global__ void __launch_bounds__(kSideThreads) k_side(const Item* __restrict__ 
 // double one point at a time in the set's order (src/SolutionKmeans.hpp:
 // 170-175, :227-238 -- under a serial scheduler the large-node combinable
 // holds one partial, so that order is the sample's).  Rounding makes that
-// sum order-dependent, so it is not split: one CTA per node walks the set in
-// order.  A producer warp streams the rows into shared memory with bulk
-// copies (one per row, into a ring of kSeqStages tiles on mbarriers); warp 0
-// sums the side-true rows and warp 1 the side-false rows, each lane owning
-// dims lane, lane+32, ... so a node's 2*D sums advance together.
-constexpr int kSeqRows = 64;
-constexpr int kSeqStages = 4;
-constexpr int kSeqThreads = 3 * kWarp;
+// sum order-dependent, so it is not split over the points; it is split over
+// dimensions: one CTA per node and up to 32 dimensions walks the set in order.
+// Copier warps stream those dimensions of the rows into shared memory (16-byte
+// copies into a ring of 64-row tiles on mbarriers), a tile's side-true rows
+// first and its side-false rows after them, each in order; one warp per side
+// sums its rows, a dimension a lane.
+//
+// What bounds it is the chain of dependent double adds of a large node's
+// longer side (8.3 cycles each), so little else may sit on that chain or in
+// its warp's issue slots: a side's rows are consecutive (no flag to test, no
+// list, addresses are immediates), the next group's values are loaded before
+// this group's are added, and the conversion to double is folded into the add
+// (scaled_double).  The copies set the other limit, which is why a node's
+// dimensions go to several CTAs: a bulk copy of a 400-byte row takes about 70
+// cycles of an SM's copy engine and 16-byte copies of it 18 cycles, each more
+// than the adds.  Measured over one build, against one CTA per node fed by bulk
+// copies with one warp per side over all dimensions: 100k x 100 (232 launches)
+// 4.9 ms from 32.0, 2M x 100 (154) 12.6 from 77.4, 217k x 128 2.8 from 20.2.
+constexpr uint32_t kSeqRows = 64;
+constexpr uint32_t kSeqGroup = 8;                       // rows a consumer loads at a time
+constexpr uint32_t kSeqCopiers = 4;                     // warps that copy rows
+constexpr uint32_t kSeqShare = kSeqRows / kSeqCopiers;  // rows of a tile one of them copies
+constexpr uint32_t kSeqAhead = kWarp / kSeqShare;       // tiles whose ids one load brings
+constexpr uint32_t kSeqStages = 4;
+constexpr int kSeqThreads = (2 + kSeqCopiers) * kWarp;
+// CTAs per node, and the dimensions of each (whole 16-byte pieces).
+__host__ __device__ constexpr uint32_t seq_groups(int D) { return (D + kWarp - 1) / kWarp; }
+__host__ __device__ constexpr uint32_t seq_dims(int D) { return (D / 4 + seq_groups(D) - 1) / seq_groups(D) * 4; }
+
+constexpr uint32_t kSeqGrid = 148 * 6;  // CTAs: as many as fit on the SMs
 
 struct SeqNode {
-    uint64_t fbase;  // first entry of the node in the flag / id arrays (16-byte aligned)
+    uint64_t fbase;  // first entry of the node in the flag / id arrays
     uint32_t len;    // entries
     uint32_t pad;
 };
 
-__host__ __device__ constexpr size_t seq_smem_bytes(int D) {
-    return static_cast<size_t>(kSeqStages) * kSeqRows * D * sizeof(float) + kSeqStages * kSeqRows;
+// x * 2^-896 as a double, for finite x: the float's sign, exponent and mantissa
+// fields at the double's places, the exponent not re-biased (1023 - 127 = 896;
+// a subnormal float becomes the subnormal double of the same scale, so zero
+// and subnormals are exact too).  fma(scaled_double(x), 2^896, sum) rounds
+// sum + x once, as the add of the converted value does; the conversion
+// instruction itself takes 16 cycles a warp and scheduler, this a multiply
+// (both shifts at once) and a mask.
+constexpr double kUnscale = 0x1p896;
+__device__ __forceinline__ double scaled_double(float x) {
+    const long long w = static_cast<long long>(__float_as_int(x)) * (1 << 29);
+    return __hiloint2double(static_cast<int>(w >> 32) & static_cast<int>(0x8fffffffu), static_cast<int>(w));
 }
 
 template <int D>
-__global__ void __launch_bounds__(kSeqThreads) k_lloyd_seq(const SeqNode* __restrict__ nodes,
-                                                           const uint8_t* __restrict__ flags,
-                                                           const uint32_t* __restrict__ ids,
-                                                           const float* __restrict__ pts, int ld, float* __restrict__ c1,
-                                                           float* __restrict__ c2, int32_t* __restrict__ ok,
-                                                           int32_t* __restrict__ error_flag,
-                                                           const uint32_t* __restrict__ dcount) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    float* tiles = reinterpret_cast<float*>(smem);                                   // [stage][row][D]
-    uint8_t* tflags = smem + static_cast<size_t>(kSeqStages) * kSeqRows * D * 4;  // [stage][row]
-    __shared__ uint64_t full[kSeqStages], empty[kSeqStages];
+__global__ void __launch_bounds__(kSeqThreads)
+    k_lloyd_seq(const SeqNode* __restrict__ nodes, const uint8_t* __restrict__ flags, const uint32_t* __restrict__ ids,
+                const float* __restrict__ pts, int ld, float* __restrict__ c1, float* __restrict__ c2,
+                int32_t* __restrict__ ok, int32_t* __restrict__ error_flag, uint32_t count,
+                const uint32_t* __restrict__ dcount) {
+    constexpr uint32_t G = seq_groups(D), DG = seq_dims(D), S = kSeqStages;
+    // [stage][row][DG], and the rows past them that a last group may read (and drop)
+    __shared__ __align__(16) float tiles[(S * kSeqRows + kSeqGroup) * DG];
+    __shared__ uint64_t full[S], empty[S];
+    __shared__ uint32_t counts[S][2];  // side-true rows, side-false rows of the tile
     const int lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
-    // Nodes blockIdx.x, blockIdx.x + gridDim.x, ... of [0, count); their
-    // tiles run through one ring, tile g of the CTA in stage g % kSeqStages.
-    const uint32_t count = dcount ? *dcount : gridDim.x;
+    // Units (node, dimension group) blockIdx.x, blockIdx.x + gridDim.x, ...;
+    // their tiles run through one ring, tile g of the CTA in stage g % S.
+    if (dcount) count = *dcount;
+    const uint32_t units = count * G;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kSeqStages; ++s) {
-            tc::mbar_init(&full[s], 1);
+        for (uint32_t s = 0; s < S; ++s) {
+            tc::mbar_init(&full[s], kSeqCopiers * kWarp + 1);
             tc::mbar_init(&empty[s], 2);
         }
         tc::fence_barrier_init();
     }
     __syncthreads();
-    constexpr uint32_t kRowBytes = D * sizeof(float);
-    if (warp == 2) {
-        // Producer: a node's ids of the next tile are loaded while this one is issued.
+    if (warp >= 2) {
+        // Copiers: warp w copies rows w * kSeqShare ... of every tile.  The ids
+        // of kSeqAhead tiles are one load (lane / kSeqShare the tile), made as
+        // many tiles ahead, and so are the flags of whole tiles.
+        const int w = warp - 2;
+        constexpr uint32_t R = 4, P = kWarp / R;  // rows copied at once, lanes (16-byte pieces) of each
+        constexpr int U = kSeqRows / kWarp;
+        static_assert(DG <= 4 * P, "a row's share fits its lanes");
+        const uint32_t q = lane % P, sub = lane / P;
+        const uint32_t tiles_at = tc::smem_u32(tiles) + 16 * q;
         uint32_t g = 0;
         bool failed = false;
-        for (uint32_t node = blockIdx.x; node < count && !failed; node += gridDim.x) {
-            const SeqNode nd = nodes[node];
+        for (uint32_t unit = blockIdx.x; unit < units && !failed; unit += gridDim.x) {
+            const SeqNode nd = nodes[unit / G];
+            const uint32_t dim0 = (unit % G) * DG;
+            const float* from = pts + dim0 + 4 * q;
+            const bool piece = 4 * q < DG && dim0 + 4 * q < D;
             const uint32_t ntiles = (nd.len + kSeqRows - 1) / kSeqRows;
-            uint32_t next[kSeqRows / kWarp];
-            auto load_ids = [&](uint32_t t) {
+            auto load_ids = [&](uint32_t t0) {
+                const uint32_t e = (t0 + lane / kSeqShare) * kSeqRows + w * kSeqShare + lane % kSeqShare;
+                return e < nd.len ? ids[nd.fbase + e] : 0u;
+            };
+            auto load_flags = [&](uint32_t t, uint8_t (&to)[U]) {
 #pragma unroll
-                for (int u = 0; u < kSeqRows / kWarp; ++u) {
-                    const uint32_t e = t * kSeqRows + lane + u * kWarp;
-                    next[u] = (t < ntiles && e < nd.len) ? ids[nd.fbase + e] : 0u;
+                for (int u = 0; u < U; ++u) {
+                    const uint32_t e = t * kSeqRows + u * kWarp + lane;
+                    to[u] = e < nd.len ? flags[nd.fbase + e] : 0;
                 }
             };
-            load_ids(0);
-            for (uint32_t t = 0; t < ntiles; ++t, ++g) {
-                uint32_t cur[kSeqRows / kWarp];
+            uint32_t next = load_ids(0);
+            uint8_t f[kSeqAhead][U];
 #pragma unroll
-                for (int u = 0; u < kSeqRows / kWarp; ++u) cur[u] = next[u];
-                load_ids(t + 1);
-                const uint32_t s = g % kSeqStages;
-                if (g >= kSeqStages && !tc::mbar_wait_limited(&empty[s], ((g / kSeqStages) - 1) & 1u)) {
-                    if (lane == 0) atomicExch(error_flag, 1);
-                    failed = true;
-                    break;
-                }
-                const uint32_t rows = min(static_cast<uint32_t>(kSeqRows), nd.len - t * kSeqRows);
-                const uint32_t fbytes = (rows + 15u) & ~15u;
-                if (lane == 0) tc::mbar_arrive_expect_tx(&full[s], rows * kRowBytes + fbytes);
-                __syncwarp();
+            for (uint32_t a = 0; a < kSeqAhead; ++a) load_flags(a, f[a]);
+            for (uint32_t t0 = 0; t0 < ntiles && !failed; t0 += kSeqAhead) {
+                const uint32_t cur = next;
+                next = load_ids(t0 + kSeqAhead);
 #pragma unroll
-                for (int u = 0; u < kSeqRows / kWarp; ++u) {
-                    const uint32_t r = lane + u * kWarp;
-                    if (r < rows)
-                        tc::bulk_g2s(tiles + (static_cast<size_t>(s) * kSeqRows + r) * D,
-                                     pts + static_cast<size_t>(cur[u]) * ld, kRowBytes, &full[s]);
+                for (uint32_t a = 0; a < kSeqAhead; ++a) {
+                    const uint32_t t = t0 + a;
+                    if (t >= ntiles) break;
+                    unsigned long long mask = 0;  // side-true rows of the tile
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+                        mask |= static_cast<unsigned long long>(__ballot_sync(kFull, f[a][u] == 1)) << (u * kWarp);
+                    load_flags(t + kSeqAhead, f[a]);
+                    const uint32_t s = g % S;
+                    if (g >= S && !tc::mbar_wait_limited(&empty[s], ((g / S) - 1) & 1u)) {
+                        if (lane == 0) atomicExch(error_flag, 1);
+                        failed = true;
+                        break;
+                    }
+                    const uint32_t rows = min(kSeqRows, nd.len - t * kSeqRows);
+                    const uint32_t trues = __popcll(mask);
+                    // Lane l works out where row l % kSeqShare of the share goes, as a
+                    // byte offset; rows past the end copy nothing.
+                    const uint32_t r = w * kSeqShare + lane % kSeqShare;
+                    const uint32_t before = __popcll(mask & ((1ull << r) - 1ull));
+                    const uint32_t to = ((mask >> r) & 1ull ? before : trues + r - before) * (DG * 4);
+                    const uint32_t put = r < rows ? to : ~0u;
+                    const uint32_t tile = tiles_at + s * (kSeqRows * DG * 4);
+#pragma unroll
+                    for (uint32_t i = 0; i < kSeqShare; i += R) {
+                        const uint32_t id = __shfl_sync(kFull, cur, (a * kSeqShare + i + sub) % kWarp);
+                        const uint32_t off = __shfl_sync(kFull, put, (i + sub) % kWarp);
+                        if (piece && off != ~0u) tc::cp_async16(tile + off, from + static_cast<size_t>(id) * ld);
+                    }
+                    tc::cp_async_arrive(&full[s]);
+                    if (w == 0 && lane == 0) {
+                        counts[s][0] = trues;
+                        counts[s][1] = rows - trues;
+                        tc::mbar_arrive(&full[s]);
+                    }
+                    ++g;
                 }
-                if (lane == 0) tc::bulk_g2s(tflags + s * kSeqRows, flags + nd.fbase + t * kSeqRows, fbytes, &full[s]);
             }
         }
-        // No copy may be in flight when the CTA exits.
-        const uint32_t first = g > kSeqStages ? g - kSeqStages : 0u;
-        for (uint32_t t = first; t < g; ++t)
-            if (!tc::mbar_wait(&full[t % kSeqStages], (t / kSeqStages) & 1u) && lane == 0) atomicExch(error_flag, 1);
+        tc::cp_async_wait_all();  // no copy may be in flight when the CTA exits
         return;
     }
     // Consumers: warp 0 sums the side-true rows, warp 1 the side-false rows.
-    const uint8_t want = warp == 0 ? 1 : 0;
-    constexpr int PER = (D + kWarp - 1) / kWarp;
+    const int side = warp;
     uint32_t g = 0;
-    for (uint32_t node = blockIdx.x; node < count; node += gridDim.x) {
-        const SeqNode nd = nodes[node];
-        const uint32_t ntiles = (nd.len + kSeqRows - 1) / kSeqRows;
-        double acc[PER];
-#pragma unroll
-        for (int j = 0; j < PER; ++j) acc[j] = 0.0;
+    for (uint32_t unit = blockIdx.x; unit < units; unit += gridDim.x) {
+        const uint32_t node = unit / G, dim = (unit % G) * DG + lane;
+        const bool live = lane < DG && dim < D;
+        const float* col = tiles + (lane < DG ? lane : 0);
+        const uint32_t ntiles = (nodes[node].len + kSeqRows - 1) / kSeqRows;
+        double acc = 0.0;
+        float odd = 0.0f;  // NaN once a value was not finite
         uint32_t cnt = 0;
         for (uint32_t t = 0; t < ntiles; ++t, ++g) {
-            const uint32_t s = g % kSeqStages;
-            if (!tc::mbar_wait_limited(&full[s], (g / kSeqStages) & 1u)) {
+            const uint32_t s = g % S;
+            if (!tc::mbar_wait_limited(&full[s], (g / S) & 1u)) {
                 if (lane == 0) atomicExch(error_flag, 1);
                 return;
             }
-            const uint32_t rows = min(static_cast<uint32_t>(kSeqRows), nd.len - t * kSeqRows);
-            const float* tile = tiles + static_cast<size_t>(s) * kSeqRows * D;
-            const uint8_t* tf = tflags + s * kSeqRows;
-#pragma unroll 4
-            for (uint32_t r = 0; r < rows; ++r) {
-                if (tf[r] == want) {
+            const uint32_t mine = counts[s][side];
+            const float* at = col + (s * kSeqRows + (side == 0 ? 0u : counts[s][0])) * DG;
+            cnt += mine;
+            float v[kSeqGroup], w[kSeqGroup];
+            auto load = [&](float (&to)[kSeqGroup]) {
 #pragma unroll
-                    for (int j = 0; j < PER; ++j)
-                        if (lane + j * kWarp < D)
-                            acc[j] = __dadd_rn(acc[j], static_cast<double>(tile[r * D + lane + j * kWarp]));
-                    ++cnt;
+                for (uint32_t u = 0; u < kSeqGroup; ++u) to[u] = live ? at[u * DG] : 0.0f;
+                at += kSeqGroup * DG;
+            };
+            auto add = [&](const float (&x)[kSeqGroup]) {
+#pragma unroll
+                for (uint32_t u = 0; u < kSeqGroup; ++u) {
+                    acc = __fma_rn(scaled_double(x[u]), kUnscale, acc);
+                    odd = __fmaf_rn(x[u], 0.0f, odd);
                 }
+            };
+            // Rows past the side's last read as +0.0, which leaves a sum that
+            // started at +0.0 as it is.
+            auto drop = [&](float (&x)[kSeqGroup], uint32_t keep) {
+#pragma unroll
+                for (uint32_t u = 0; u < kSeqGroup; ++u) x[u] = u < keep ? x[u] : 0.0f;
+            };
+            uint32_t left = mine;
+            load(v);
+            while (left > 2 * kSeqGroup) {
+                load(w);
+                add(v);
+                load(v);
+                add(w);
+                left -= 2 * kSeqGroup;
+            }
+            if (left > kSeqGroup) {
+                load(w);
+                add(v);
+                drop(w, left - kSeqGroup);
+                add(w);
+            } else if (left > 0) {
+                drop(v, left);
+                add(v);
             }
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(&empty[s]);
@@ -459,11 +548,18 @@ __global__ void __launch_bounds__(kSeqThreads) k_lloyd_seq(const SeqNode* __rest
             if (lane == 0) ok[node] = 0;
             continue;
         }
-        float* c = (warp == 0 ? c1 : c2) + static_cast<size_t>(node) * ld;
-        const double nn = static_cast<double>(cnt);
-#pragma unroll
-        for (int j = 0; j < PER; ++j)
-            if (lane + j * kWarp < D) c[lane + j * kWarp] = __double2float_rn(__ddiv_rn(acc[j], nn));
+        if (odd != 0.0f) {
+            // Infinities or NaN among the values: their sum once more, by the
+            // conversion, from global memory.
+            const SeqNode nd = nodes[node];
+            acc = 0.0;
+            for (uint32_t e = 0; e < nd.len; ++e)
+                if (flags[nd.fbase + e] == 1 - side)
+                    acc = __dadd_rn(acc, static_cast<double>(
+                                             pts[static_cast<size_t>(ids[nd.fbase + e]) * ld + (live ? dim : 0)]));
+        }
+        float* c = (side == 0 ? c1 : c2) + static_cast<size_t>(node) * ld;
+        if (live) c[dim] = __double2float_rn(__ddiv_rn(acc, static_cast<double>(cnt)));
     }
 }
 
@@ -954,14 +1050,12 @@ void launch_lloyd(Context& c, uint32_t count, const uint32_t* h_starts, const ui
     int32_t* err = d_ok + count;
     KNNG_CUDA(cudaMemsetAsync(err, 0, sizeof(int32_t), c.stream));
     KNNG_DISPATCH_D(c.d, {
-        auto seq = k_lloyd_seq<D>;
-        allow_max_smem(c, seq);
         for (uint32_t iter = 0; iter < iters; ++iter) {
             launch_plane(c, count, d_c1, d_c2, d_coefs, d_offsets);
             k_side<D><<<ni, kSideThreads, 0, c.stream>>>(d_items, d_lloyd_positions, c.indices, c.points, c.ld,
                                                          d_coefs, d_offsets, flags, ids, item_true, nullptr);
-            seq<<<count, kSeqThreads, seq_smem_bytes(D), c.stream>>>(d_nodes, flags, ids, c.points, c.ld, d_c1, d_c2,
-                                                                     d_ok, err, nullptr);
+            k_lloyd_seq<D><<<std::min(count * seq_groups(D), kSeqGrid), kSeqThreads, 0, c.stream>>>(
+                d_nodes, flags, ids, c.points, c.ld, d_c1, d_c2, d_ok, err, count, nullptr);
             c.launches += 2;
             KNNG_CUDA(cudaGetLastError());
         }
@@ -1223,15 +1317,13 @@ void enqueue_level(Context& c, DevRep& r, uint32_t lloyd_iters, cudaGraphConditi
         allow_max_smem(c, fp);
         fp<<<kNodeGrid, kPairThreads, fp_smem, c.stream>>>(r.seed_off, r.seeds, c.indices, c.points, c.ld, r.first,
                                                            r.second, r.ok, r.c1, r.c2, cur);
-        auto seqk = k_lloyd_seq<D>;
-        allow_max_smem(c, seqk);
         for (uint32_t iter = 0; iter < lloyd_iters; ++iter) {
             k_plane<D><<<kNodeGrid, 256, 0, c.stream>>>(r.c1, r.c2, c.ld, 0, r.coefs, r.offs, cur);
             k_side<D><<<kItemGrid, kSideThreads, 0, c.stream>>>(r.litems, r.lloyd, c.indices, c.points, c.ld, r.coefs,
                                                                 r.offs, r.lflags, r.lids, r.litem_true,
                                                                 &r.cnt->lloyd_items);
-            seqk<<<kThreadGrid, kSeqThreads, seq_smem_bytes(D), c.stream>>>(r.seq, r.lflags, r.lids, c.points, c.ld,
-                                                                              r.c1, r.c2, r.ok, r.error, cur);
+            k_lloyd_seq<D><<<kSeqGrid, kSeqThreads, 0, c.stream>>>(r.seq, r.lflags, r.lids, c.points, c.ld, r.c1, r.c2,
+                                                                   r.ok, r.error, 0, cur);
         }
         k_plane<D><<<kNodeGrid, 256, 0, c.stream>>>(r.c1, r.c2, c.ld, 0, r.coefs, r.offs, cur);
         k_part_plan<<<1, kPlanThreads, 0, c.stream>>>(r.start, r.end, r.cnt, r.ok, r.ib, r.ie);
@@ -1279,7 +1371,6 @@ DevRep::Graph& rep_graph(Context& c, DevRep& r, uint32_t max_leaf, uint32_t lloy
     // Attributes first: nothing but stream work may happen during the capture.
     KNNG_DISPATCH_D(c.d, {
         allow_max_smem(c, k_farthest_pair<D>);
-        allow_max_smem(c, k_lloyd_seq<D>);
     });
     if (precision == KNNG_PRECISION_BF16_RERANK)
         prepare_leaves_bf16_list(c);

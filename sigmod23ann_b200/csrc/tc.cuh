@@ -170,9 +170,20 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc, boo
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(gsrc), "r"(sz) : "memory");
 }
 
+// The same to a shared-memory address, always reading.
+__device__ __forceinline__ void cp_async16(uint32_t smem_dst, const void* gsrc) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_dst), "l"(gsrc) : "memory");
+}
+
 // Waits until every cp.async this thread issued has landed (visible to this
 // thread; other threads need a barrier after it).
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// One arrival on the barrier once every cp.async this thread issued so far has
+// landed (the barrier's count includes it).
+__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 
 // ---------------------------------------------------------------- MMA
 
