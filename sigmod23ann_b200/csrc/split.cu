@@ -42,6 +42,11 @@ constexpr int kSideThreads = 256;
 constexpr int kSidePer = 8;  // positions per thread in the side / scatter kernels
 constexpr int kChunk = kSideThreads * kSidePer;
 constexpr int kPairThreads = 256;
+// Grids of the level's kernels (grid-stride loops): over nodes, over items,
+// over one thread per node or item.
+constexpr uint32_t kNodeGrid = 148 * 4;
+constexpr uint32_t kItemGrid = 148 * 8;
+constexpr uint32_t kThreadGrid = 148 * 2;
 constexpr uint32_t kListItem = 0x80000000u;  // Item::node flag: entries come from a position list
 
 // A chunk of one node's entries: positions begin .. begin+count (range item)
@@ -264,40 +269,50 @@ __device__ __forceinline__ float group_dot(const ChainPlane<D>& p, const float* 
     return acc;
 }
 
-// Side flags of one item (up to kChunk entries of one node): entry r reads
-// position begin + r, or list[begin + r] for a list item; its flag goes to
-// flags[fbase + r] and, when `ids_out` is given, its point id to
-// ids_out[fbase + r].  item_true[item] = the item's side-true count.
+// Side flags of the items (up to kChunk entries of one node each): entry r
+// reads position begin + r, or list[begin + r] for a list item; its flag goes
+// to flags[fbase + r] and, when `ids_out` is given, its point id to
+// ids_out[fbase + r].  With `item_true` (zeroed before) each item's side-true
+// count is added up there.
+//
+// A warp takes 32 entries at a time (a unit: kChunk / 32 of them an item, an
+// item's past its count are empty), the loads of several groups of four rows in
+// flight.  What bounds the small levels is latency -- item, position, id and
+// row are dependent loads -- so a level of few items must still reach every SM:
+// a CTA per 2,048-entry item left a 100k x 100 level to 49 CTAs that walked
+// 64 units' latency each in turn (42 us a launch, now 9).  Units go to warps
+// unit-major, so that the empty ones of short items fall together at the end.
 template <int D>
 __global__ void __launch_bounds__(kSideThreads) k_side(const Item* __restrict__ items, const uint32_t* __restrict__ list,
                                                        const uint32_t* __restrict__ idx, const float* __restrict__ pts,
                                                        int ld, const float* __restrict__ coefs,
                                                        const float* __restrict__ offsets, uint8_t* __restrict__ flags,
                                                        uint32_t* __restrict__ ids_out,
-                                                       uint32_t* __restrict__ item_true,
+                                                       uint32_t* __restrict__ item_true, uint32_t n_items,
                                                        const uint32_t* __restrict__ dcount) {
-    __shared__ uint32_t warp_sum[kSideThreads / kWarp];
-    const uint32_t n_items = dcount ? *dcount : gridDim.x;
-    for (uint32_t item = blockIdx.x; item < n_items; item += gridDim.x) {
-    const Item it = items[item];
-    const bool from_list = (it.node & kListItem) != 0;
-    const uint32_t node = it.node & ~kListItem;
-    const int lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
+    if (dcount) n_items = *dcount;
+    const int lane = threadIdx.x % kWarp;
     const int l = lane & 7, grp = lane >> 3, g0 = lane & ~7;
-    ChainPlane<D> plane;
-    load_chain_plane<D>(plane, coefs + static_cast<size_t>(node) * ld, l);
-    const float off = offsets[node];
-    uint32_t cnt = 0;
-    // Each warp takes 32 consecutive entries at a time.
-    for (uint32_t r0 = warp * kWarp; r0 < it.count; r0 += kSideThreads) {
+    const uint64_t units = static_cast<uint64_t>(n_items) * (kChunk / kWarp);
+    for (uint64_t unit = (blockIdx.x * kSideThreads + threadIdx.x) / kWarp; unit < units;
+         unit += gridDim.x * (kSideThreads / kWarp)) {
+        const uint32_t item = static_cast<uint32_t>(unit % n_items);
+        const uint32_t r0 = static_cast<uint32_t>(unit / n_items) * kWarp;
+        const Item it = items[item];
+        if (r0 >= it.count) continue;
+        const bool from_list = (it.node & kListItem) != 0;
+        const uint32_t node = it.node & ~kListItem;
         const uint32_t r = r0 + lane;
         uint32_t id = 0;
         if (r < it.count) {
             const uint64_t e = it.begin + r;
             id = idx[from_list ? list[e] : static_cast<uint32_t>(e)];
         }
+        ChainPlane<D> plane;
+        load_chain_plane<D>(plane, coefs + static_cast<size_t>(node) * ld, l);
+        const float off = offsets[node];
         uint32_t mask = 0;  // bit j: entry r0 + j is side-true
-#pragma unroll 1
+#pragma unroll 4
         for (int b = 0; b < 8; ++b) {
             const int j = 4 * b + grp;
             const uint32_t pid = __shfl_sync(kFull, id, j);
@@ -308,20 +323,10 @@ __global__ void __launch_bounds__(kSideThreads) k_side(const Item* __restrict__ 
             for (int q = 0; q < 4; ++q) mask |= ((bal >> (8 * q)) & 1u) << (4 * b + q);
         }
         if (r < it.count) {
-            const uint8_t f = (mask >> lane) & 1u;
-            flags[it.fbase + r] = f;
+            flags[it.fbase + r] = (mask >> lane) & 1u;
             if (ids_out) ids_out[it.fbase + r] = id;
         }
-        cnt += __popc(mask);  // warp-uniform
-    }
-    if (lane == 0) warp_sum[warp] = cnt;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t s = 0;
-        for (int w = 0; w < kSideThreads / kWarp; ++w) s += warp_sum[w];
-        item_true[item] = s;
-    }
-    __syncthreads();  // warp_sum is reused by the next item
+        if (item_true && lane == 0) atomicAdd(&item_true[item], static_cast<uint32_t>(__popc(mask)));
     }
 }
 
@@ -832,13 +837,14 @@ __global__ void __launch_bounds__(kPlanThreads)
 
 __global__ void k_part_items(const LevelCounts* __restrict__ cnt, const uint32_t* __restrict__ start,
                              const uint32_t* __restrict__ end, const uint32_t* __restrict__ ib,
-                             Item* __restrict__ items) {
+                             Item* __restrict__ items, uint32_t* __restrict__ item_true) {
     const uint32_t count = cnt->cur, total = cnt->part_items;
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
         const uint32_t i = owner_of(ib, count, t);
         const uint64_t o = static_cast<uint64_t>(start[i]) + static_cast<uint64_t>(t - ib[i]) * kChunk;
         const uint64_t left = end[i] - o;
         items[t] = {i, static_cast<uint32_t>(left < kChunk ? left : kChunk), o, o};
+        item_true[t] = 0;  // the side test adds to it
     }
 }
 
@@ -967,6 +973,11 @@ __global__ void k_rep_init(const uint32_t* __restrict__ set_offsets, uint32_t ns
 
 void set_split_wait_limit(uint32_t polls) { KNNG_CUDA(cudaMemcpyToSymbol(tc::g_wait_limit, &polls, sizeof(polls))); }
 
+// CTAs of a side test over n_items items: a warp per unit, up to the grid of a level.
+static uint32_t side_grid(uint32_t n_items) {
+    return static_cast<uint32_t>(std::min<uint64_t>(static_cast<uint64_t>(n_items) * kChunk / kSideThreads, kItemGrid));
+}
+
 void launch_iota(Context& c) {
     if (c.n == 0) return;
     k_iota<<<std::min<uint32_t>((c.n + 255) / 256, 148 * 16), 256, 0, c.stream>>>(c.indices, c.n);
@@ -1046,14 +1057,14 @@ void launch_lloyd(Context& c, uint32_t count, const uint32_t* h_starts, const ui
     const SeqNode* d_nodes = upload(c, "lloyd_nodes", nodes.data(), count);
     uint8_t* flags = static_cast<uint8_t*>(scratch(c, "lloyd_flags", fnext + 64));
     uint32_t* ids = static_cast<uint32_t*>(scratch(c, "lloyd_ids", (fnext + 64) * sizeof(uint32_t)));
-    uint32_t* item_true = static_cast<uint32_t*>(scratch(c, "lloyd_item_true", (ni + 1) * sizeof(uint32_t)));
     int32_t* err = d_ok + count;
     KNNG_CUDA(cudaMemsetAsync(err, 0, sizeof(int32_t), c.stream));
     KNNG_DISPATCH_D(c.d, {
         for (uint32_t iter = 0; iter < iters; ++iter) {
             launch_plane(c, count, d_c1, d_c2, d_coefs, d_offsets);
-            k_side<D><<<ni, kSideThreads, 0, c.stream>>>(d_items, d_lloyd_positions, c.indices, c.points, c.ld,
-                                                         d_coefs, d_offsets, flags, ids, item_true, nullptr);
+            k_side<D><<<side_grid(ni), kSideThreads, 0, c.stream>>>(d_items, d_lloyd_positions, c.indices, c.points, c.ld,
+                                                                    d_coefs, d_offsets, flags, ids, nullptr, ni,
+                                                                    nullptr);
             k_lloyd_seq<D><<<std::min(count * seq_groups(D), kSeqGrid), kSeqThreads, 0, c.stream>>>(
                 d_nodes, flags, ids, c.points, c.ld, d_c1, d_c2, d_ok, err, count, nullptr);
             c.launches += 2;
@@ -1081,9 +1092,10 @@ void launch_partition(Context& c, uint32_t count, const uint32_t* h_starts, cons
     uint8_t* flags = static_cast<uint8_t*>(scratch(c, "side_flags", c.n + 16));
     uint32_t* item_true = static_cast<uint32_t*>(scratch(c, "item_true", (ni + 1) * sizeof(uint32_t)));
     uint32_t* prefix = static_cast<uint32_t*>(scratch(c, "item_prefix", (ni + 1) * sizeof(uint32_t)));
+    KNNG_CUDA(cudaMemsetAsync(item_true, 0, ni * sizeof(uint32_t), c.stream));
     KNNG_DISPATCH_D(c.d, {
-        k_side<D><<<ni, kSideThreads, 0, c.stream>>>(d_items, nullptr, c.indices, c.points, c.ld, d_coefs, d_offsets,
-                                                     flags, nullptr, item_true, nullptr);
+        k_side<D><<<side_grid(ni), kSideThreads, 0, c.stream>>>(d_items, nullptr, c.indices, c.points, c.ld, d_coefs,
+                                                                d_offsets, flags, nullptr, item_true, ni, nullptr);
     });
     k_scan_items<<<1, 1024, 0, c.stream>>>(item_true, ni, prefix, nullptr);
     k_node_true<<<(count + 255) / 256, 256, 0, c.stream>>>(d_ib, d_ie, prefix, count, d_true, nullptr);
@@ -1114,7 +1126,7 @@ struct DevRep {
     uint32_t *seeds, *lloyd;
     SeqNode* seq;
     uint64_t* lbegin;
-    uint32_t *lfrom, *item_off, *lids, *litem_true;
+    uint32_t *lfrom, *item_off, *lids;
     Item* litems;
     uint8_t* lflags;
     uint32_t *first, *second;
@@ -1268,7 +1280,6 @@ DevRep& ensure_devrep(Context& c, uint32_t max_leaf, uint32_t small_threshold) {
     r.litems = rep_alloc<Item>(c, r, r.lloyd_item_cap);
     r.lflags = rep_alloc<uint8_t>(c, r, r.entry_cap);
     r.lids = rep_alloc<uint32_t>(c, r, r.entry_cap);
-    r.litem_true = rep_alloc<uint32_t>(c, r, r.lloyd_item_cap + 1);
     r.first = rep_alloc<uint32_t>(c, r, nc);
     r.second = rep_alloc<uint32_t>(c, r, nc);
     r.ok = rep_alloc<int32_t>(c, r, nc);
@@ -1286,10 +1297,6 @@ DevRep& ensure_devrep(Context& c, uint32_t max_leaf, uint32_t small_threshold) {
     KNNG_CUDA(cudaStreamSynchronize(c.stream));
     return r;
 }
-
-constexpr uint32_t kNodeGrid = 148 * 4;
-constexpr uint32_t kItemGrid = 148 * 8;
-constexpr uint32_t kThreadGrid = 148 * 2;
 
 // Start of a repetition: the error words cleared, indices 0..n-1, the sets'
 // roots as the first level.
@@ -1320,16 +1327,16 @@ void enqueue_level(Context& c, DevRep& r, uint32_t lloyd_iters, cudaGraphConditi
         for (uint32_t iter = 0; iter < lloyd_iters; ++iter) {
             k_plane<D><<<kNodeGrid, 256, 0, c.stream>>>(r.c1, r.c2, c.ld, 0, r.coefs, r.offs, cur);
             k_side<D><<<kItemGrid, kSideThreads, 0, c.stream>>>(r.litems, r.lloyd, c.indices, c.points, c.ld, r.coefs,
-                                                                r.offs, r.lflags, r.lids, r.litem_true,
+                                                                r.offs, r.lflags, r.lids, nullptr, 0,
                                                                 &r.cnt->lloyd_items);
             k_lloyd_seq<D><<<kSeqGrid, kSeqThreads, 0, c.stream>>>(r.seq, r.lflags, r.lids, c.points, c.ld, r.c1, r.c2,
                                                                    r.ok, r.error, 0, cur);
         }
         k_plane<D><<<kNodeGrid, 256, 0, c.stream>>>(r.c1, r.c2, c.ld, 0, r.coefs, r.offs, cur);
         k_part_plan<<<1, kPlanThreads, 0, c.stream>>>(r.start, r.end, r.cnt, r.ok, r.ib, r.ie);
-        k_part_items<<<kThreadGrid, 256, 0, c.stream>>>(r.cnt, r.start, r.end, r.ib, r.pitems);
+        k_part_items<<<kThreadGrid, 256, 0, c.stream>>>(r.cnt, r.start, r.end, r.ib, r.pitems, r.item_true);
         k_side<D><<<kItemGrid, kSideThreads, 0, c.stream>>>(r.pitems, nullptr, c.indices, c.points, c.ld, r.coefs,
-                                                            r.offs, r.side_flags, nullptr, r.item_true,
+                                                            r.offs, r.side_flags, nullptr, r.item_true, 0,
                                                             &r.cnt->part_items);
     });
     k_scan_items<<<1, 1024, 0, c.stream>>>(r.item_true, 0, r.prefix, &r.cnt->part_items);
