@@ -93,17 +93,17 @@ typedef struct knng_stats {
     uint64_t kernel_launches; /* all kernels launched by the call */
     uint64_t refine_changed;  /* points whose set changed in the refinement pass */
     double ms_refine_join;    /* refinement: tensor-core join, direct pass (every point) */
-    double ms_refine_apply;   /* refinement: survivor lists + sorted replay */
-    double ms_refine_fallback;/* refinement: per-point pass for points with a lost record */
+    double ms_refine_apply;   /* refinement: candidates, exact distances, sorted replay */
+    double ms_refine_fallback;/* refinement: per-point pass for points with too many candidates */
     uint64_t refine_pairs;    /* (point, candidate) pairs the join evaluated */
     uint64_t refine_filter_pass; /* pairs the tensor-core bound could not reject */
     uint64_t refine_member_skip; /* of those, candidates already in the point's list */
-    uint64_t refine_exact;    /* exact FP32 distances computed by the join */
-    uint64_t refine_emits;    /* survivor records written (before de-duplication) */
-    uint64_t refine_overflow; /* survivor records past their point's slots (pooled) */
+    uint64_t refine_exact;    /* exact FP32 distances computed (each candidate of a point once) */
+    uint64_t refine_emits;    /* candidate records: passing pairs that are no members, repeats included */
+    uint64_t refine_overflow; /* points whose candidates a warp's tables did not hold (redone by a CTA) */
     double ms_refine_prep;    /* refinement: snapshot, reverse lists, scans */
-    uint64_t refine_join_launches; /* join-kernel launches */
-    uint64_t refine_lost;     /* points redone by the per-point pass (pool region full) */
+    uint64_t refine_join_launches; /* join-kernel launches (one per range of points) */
+    uint64_t refine_lost;     /* points redone by the per-point pass (past a CTA's tables) */
     uint64_t refine_passes_done; /* neighbour-of-neighbour passes run, whichever kernel ran them */
     double recall_estimate;   /* knng_build_adaptive: recall on its sample at the end */
     uint64_t estimate_queries;/* knng_build_adaptive: sampled points */

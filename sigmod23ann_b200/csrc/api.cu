@@ -1119,6 +1119,7 @@ knng_status knng_set_sets(knng_context* ctx, const float* dist, const uint32_t* 
             if (sizes[i] == c.k && maxslot[i] >= c.k) knng::fail(KNNG_ERR_INVALID_ARGUMENT, "full set without a max slot");
         }
         c.snap_prev_valid = false;  // the sets change other than by offers
+        c.dists_own = false;
         const size_t nk = static_cast<size_t>(c.n) * c.k;
         KNNG_CUDA(cudaMemcpyAsync(c.set_dist, dist, nk * sizeof(float), cudaMemcpyHostToDevice, c.stream));
         KNNG_CUDA(cudaMemcpyAsync(c.set_id, ids, nk * sizeof(uint32_t), cudaMemcpyHostToDevice, c.stream));
@@ -1190,6 +1191,7 @@ knng_status knng_load_sets(knng_context* ctx, const char* path) {
         }
         knng::alloc_sets(c, k);
         c.snap_prev_valid = false;  // the sets change other than by offers
+        c.dists_own = false;
         KNNG_CUDA(cudaMemcpyAsync(c.set_dist, dist.data(), nk * sizeof(float), cudaMemcpyHostToDevice, c.stream));
         KNNG_CUDA(cudaMemcpyAsync(c.set_id, ids.data(), nk * sizeof(uint32_t), cudaMemcpyHostToDevice, c.stream));
         KNNG_CUDA(cudaMemcpyAsync(c.set_size, size.data(), c.n * sizeof(uint32_t), cudaMemcpyHostToDevice, c.stream));

@@ -92,9 +92,9 @@ struct Context {
     // Neighbour-of-neighbour pass: 0 = local join on the tensor cores,
     // 1 = one warp per point (environment KNNG_REFINE=pointwise at creation).
     int refine_mode = 0;
-    // Survivor storage of the join (environment at creation overrides the
-    // sizes taken from the free budget): KNNG_REFINE_SLOTS = slots per point,
-    // KNNG_REFINE_POOL = pool records per CTA region; -1 = from the budget.
+    // Candidates of a point that the replay's warp, and its CTA, take before
+    // the point goes on to the CTA, and to the per-point pass (environment at
+    // creation: KNNG_REFINE_SLOTS, KNNG_REFINE_POOL; -1 = what the kernels hold).
     int refine_slots = -1;
     // The join takes points in the leaf order of the last repetition; true
     // (environment KNNG_JOIN_ORDER=id at creation): in id order.
@@ -109,11 +109,15 @@ struct Context {
     uint32_t leaf_ctas = 2;
     // A join pass skips the pairs the previous join pass offered (both edges
     // already in its lists; offering them again changes nothing): the lists
-    // of the last pass are kept while snap_prev_valid.  Any change to the sets
+    // of the last pass (snapshot buffer snap_flip) are kept while snap_prev_valid.  Any change to the sets
     // other than offers clears it.  false (environment KNNG_REFINE_SKIP=0 at
     // creation): every pass offers every pair.
     bool refine_skip_old = true;
     bool snap_prev_valid = false;
+    uint32_t snap_flip = 0;
+    // The sets' distances are those this context's kernels computed from its
+    // points; false once sets were handed over or read from a file.
+    bool dists_own = true;
     int64_t refine_pool = -1;
     // Breakdown of the last refinement pass.
     struct RefineRecord {

@@ -43,25 +43,9 @@ __device__ __forceinline__ void fence_barrier_init() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
-// Arrives once on the barrier and raises its expected transaction bytes.
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-
 // Arrives once on the barrier.
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-// Bulk copy (the TMA engine's untiled form, this CTA's shared memory, no
-// multicast) of `bytes` from global memory; completes `bytes` transactions on
-// the barrier.  Both addresses 16-byte aligned, bytes a multiple of 16.
-__device__ __forceinline__ void bulk_g2s(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(smem_dst)),
-                 "l"(gsrc), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
 }
 
 // Poll limit of the waits for work in progress (mbar_wait_limited) in this
@@ -162,15 +146,7 @@ __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.
 
 // ---------------------------------------------------------- cp.async
 
-// 16-byte global -> shared copy that does not pass through registers; with
-// `valid` false it writes 16 zero bytes and reads nothing.
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc, bool valid) {
-    const uint32_t d = smem_u32(smem_dst);
-    const uint32_t sz = valid ? 16u : 0u;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(gsrc), "r"(sz) : "memory");
-}
-
-// The same to a shared-memory address, always reading.
+// 16-byte global -> shared copy that does not pass through registers.
 __device__ __forceinline__ void cp_async16(uint32_t smem_dst, const void* gsrc) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_dst), "l"(gsrc) : "memory");
 }
@@ -273,15 +249,22 @@ __host__ __device__ constexpr uint32_t idesc_f16(uint32_t M, uint32_t N) {
 
 // Issues the K/16 MMAs of one 128 x N 16-bit tile (call from a single thread).
 // The operand tiles (FP16 or BF16, as idesc says) use the same chunk-major
-// layout as the TF32 ones, a 16-byte chunk holding 8 values; one MMA consumes
-// K = 16 (two chunks).
-__device__ __forceinline__ void issue_tile_16bit(uint32_t tmem_d, uint32_t a_base, uint32_t b_base, uint32_t a_rows,
-                                                 uint32_t b_rows, uint32_t kpad, uint32_t idesc) {
+// layout as the TF32 ones, a 16-byte chunk holding 8 values, chunks a_stride /
+// b_stride bytes apart (at least rows * 16); one MMA consumes K = 16 (two
+// chunks).
+__device__ __forceinline__ void issue_tile_strided(uint32_t tmem_d, uint32_t a_base, uint32_t b_base, uint32_t a_stride,
+                                                   uint32_t b_stride, uint32_t kpad, uint32_t idesc) {
     for (uint32_t s = 0; s < kpad / 16; ++s) {
-        const uint64_t da = smem_desc(a_base + 2 * s * a_rows * 16, a_rows * 16, 128);
-        const uint64_t db = smem_desc(b_base + 2 * s * b_rows * 16, b_rows * 16, 128);
+        const uint64_t da = smem_desc(a_base + 2 * s * a_stride, a_stride, 128);
+        const uint64_t db = smem_desc(b_base + 2 * s * b_stride, b_stride, 128);
         mma_bf16(tmem_d, da, db, idesc, s > 0);
     }
+}
+
+// The same for tiles whose chunks follow one another without a gap.
+__device__ __forceinline__ void issue_tile_16bit(uint32_t tmem_d, uint32_t a_base, uint32_t b_base, uint32_t a_rows,
+                                                 uint32_t b_rows, uint32_t kpad, uint32_t idesc) {
+    issue_tile_strided(tmem_d, a_base, b_base, a_rows * 16, b_rows * 16, kpad, idesc);
 }
 
 // Byte offset of element (row r, k) in a chunk-major tile with `rows` rows.

@@ -1,0 +1,91 @@
+"""The join and its replay against the one-warp-per-point pass: list lengths
+around the tile's column steps, every dimension, unfilled lists, ranges of
+points when the budget is small, and sets handed over with distances that are
+not those of the points."""
+from __future__ import annotations
+
+import os
+
+import numpy as np
+import pytest
+
+from helpers import assert_sets_equal
+from sigmod23ann_b200 import KnngContext, Stats, workloads
+
+pytestmark = pytest.mark.gpu
+
+
+def _sets_after_reps(pts, k, leaf, reps=2):
+    with KnngContext(0) as c:
+        c.load_points(pts)
+        c.reset_sets(k)
+        for r in range(reps):
+            c.run_rep(leaf, 1, 3000, seed=5, rep_index=r)
+        return c.sets()
+
+
+def _pass_from(pts, k, sets, budget=0, pointwise=False, passes=1):
+    if pointwise:
+        os.environ["KNNG_REFINE"] = "pointwise"
+    try:
+        with KnngContext(0, budget) as c:
+            c.load_points(pts)
+            c.reset_sets(k)
+            c.set_sets(sets)
+            st = Stats()
+            changed = [c.refine(st) for _ in range(passes)]
+            return c.sets(), changed, st
+    finally:
+        os.environ.pop("KNNG_REFINE", None)
+
+
+@pytest.mark.parametrize("n,d,k,leaf", [(700, 64, 1, 90), (3001, 64, 10, 65), (2999, 100, 16, 129), (2500, 128, 17, 129),
+                                        (3000, 100, 32, 257), (2777, 128, 64, 200), (2500, 64, 65, 257),
+                                        (2100, 128, 100, 90), (3000, 100, 127, 300), (2500, 128, 128, 300), (129, 100, 100, 400)])
+def test_pass_equals_pointwise(knng_lib, n, d, k, leaf):
+    pts = workloads.gaussian_mixture(n=n, d=d, clusters=8, sigma=0.2, seed=n + d)
+    # With the sets a build holds (its own distances) and handed over.
+    with KnngContext(0) as c:
+        c.load_points(pts)
+        c.reset_sets(k)
+        for r in range(2):
+            c.run_rep(leaf, 1, 3000, seed=5, rep_index=r)
+        before = c.sets()
+        changed = [c.refine(), c.refine()]
+        own = c.sets()
+    want, want_changed, _ = _pass_from(pts, k, before, pointwise=True, passes=2)
+    assert_sets_equal(own, want, "own sets")
+    assert changed == want_changed
+    given, given_changed, _ = _pass_from(pts, k, before, passes=2)
+    assert_sets_equal(given, want, "handed over")
+    assert given_changed == want_changed
+
+
+def test_small_budgets_take_ranges_of_points(knng_lib):
+    """With room for some of the points' bits only, the pass goes range by
+    range; with room for none, point by point.  The sets are the same."""
+    n, d, k = 40_000, 64, 50
+    pts = workloads.gaussian_mixture(n=n, d=d, clusters=16, sigma=0.2, seed=8)
+    before = _sets_after_reps(pts, k, 129)
+    want, want_changed, _ = _pass_from(pts, k, before)
+    held = n * (4 * d + 8 + 8 * k + 12)  # points, order, sets
+    lists = n * k * 8                    # snapshot and its distances
+    seen = set()
+    for extra in (64 << 20, 40 << 20, 20 << 20):
+        got, changed, st = _pass_from(pts, k, before, budget=held + lists + extra)
+        assert_sets_equal(got, want, f"extra {extra}")
+        assert changed == want_changed
+        seen.add(int(st.refine_join_launches))
+    assert max(seen) > 1, seen
+
+
+def test_distances_of_given_sets_do_not_steer_the_filter(knng_lib):
+    """Sets handed over may hold any distances (here a thousandth of the real
+    ones, with the real bounds): the filter's norms come from the points."""
+    pts = workloads.gaussian_mixture(n=4000, d=100, clusters=8, sigma=0.2, seed=9)
+    before = _sets_after_reps(pts, 100, 300)
+    before["dist"] = before["dist"] * np.float32(1e-3)
+    want, want_changed, _ = _pass_from(pts, 100, before, pointwise=True)
+    got, changed, _ = _pass_from(pts, 100, before)
+    assert_sets_equal(got, want, "scaled distances")
+    assert changed == want_changed
