@@ -246,11 +246,12 @@ uint32_t start_count(uint32_t n);
 // leaf.cu
 void launch_leaves(Context& c, uint32_t count, const uint32_t* d_starts, const uint32_t* d_ends,
                    uint32_t max_bucket, uint64_t* evals);
-// Persistent bucket pass over a device list of *d_count buckets taken from
-// the work counter *d_work (zeroed beforehand); *d_error is set when a
-// tensor-core wait gives up.
+// Persistent bucket pass over a device list of *d_count buckets; d_items
+// (leaf_items_bytes of it) receives its work items, *d_n_items and *d_work are
+// zeroed beforehand; *d_error is set when a tensor-core wait gives up.
+size_t leaf_items_bytes(uint32_t n);
 void launch_leaves_list(Context& c, const uint32_t* d_starts, const uint32_t* d_ends, const uint32_t* d_count,
-                        uint32_t* d_work, uint32_t max_bucket, uint32_t* d_error);
+                        void* d_items, uint32_t* d_n_items, uint32_t* d_work, uint32_t max_bucket, uint32_t* d_error);
 void launch_leaves_bf16_list(Context& c, const uint32_t* d_starts, const uint32_t* d_ends, const uint32_t* d_count,
                              uint32_t* d_work, uint32_t* d_error);
 // Exact k nearest points (FP32 distances in the reference's order) of the

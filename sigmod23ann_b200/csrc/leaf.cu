@@ -1,16 +1,16 @@
 // Bucket all-pairs kernel: addCandidatesLessThan (src/KnnSets.hpp:131-160)
-// for every bucket of a repetition at once, one CTA per bucket.
+// for every bucket of a repetition at once.
 //
 // The reference offers, for a point at bucket position q, the other members
 // in position order (0..q-1 from the outer loop, then q+1..b-1 from its own
 // inner loop), each offer gated by dist < bound and applied with
 // KnnSetScannableSimd::addCandidateLessThan.  This kernel keeps that order
-// exactly: for a block of 64 points (4 per warp, sets held in registers) it
+// exactly: for a block of rows (a few per warp, sets held in registers) it
 // walks the bucket in 64-point column blocks in ascending order, computes the
-// 64x64 distance block in the reference's FP32 order from dim-major shared
-// memory tiles, then each warp replays its points' 64 offers in column order
-// (set_offer_batch).  Distances are computed for the full b x b matrix (both
-// triangles); each (i, j) and (j, i) evaluation gives the same bits.
+// block's distances in the reference's FP32 order from dim-major shared
+// memory tiles, then each warp replays its points' 64 offers in column order.
+// Distances are computed for the full b x b matrix (both triangles); each
+// (i, j) and (j, i) evaluation gives the same bits.
 // k_leaf_tc makes the same offers but computes distances only for the pairs
 // a tensor-core filter cannot rule out (see below); it is the slower of the
 // two at 10M points, where the sequential set updates dominate.
@@ -30,145 +30,240 @@ namespace {
 
 constexpr int kLeafThreads = 512;
 constexpr int kLeafWarps = kLeafThreads / kWarp;  // 16
-constexpr int kBI = 64;                            // points updated per row block
+constexpr int kBI = 64;                            // rows of the sample k-NN's and k_leaf_tc's blocks (4 a warp)
 constexpr int kBJ = 64;                            // candidates per column block
 constexpr int kPtsPerWarp = kBI / kLeafWarps;      // 4
-constexpr int kJPerThread = kBI * kBJ / kLeafThreads;  // 8
 constexpr int kDmStride = kBJ + 1;
+constexpr uint32_t kMarkCols = 1024;               // bucket positions whose member marks are held at a time
+constexpr uint32_t kMarkWords = kMarkCols / kWarp;
 
-// rows [base, base+64) of the bucket -> tile[dim][r] (zeros past the bucket end)
-template <int D>
+// rows [base, base + R) of the bucket -> tile[dim][r] (zeros past the bucket
+// end); kNegate: their negatives.
+template <int D, int R, bool kNegate = false>
 __device__ __forceinline__ void load_tile(float* __restrict__ tile, const uint32_t* __restrict__ ids, uint32_t base,
                                           uint32_t b, const float* __restrict__ pts, int ld) {
     constexpr int Q = D / 4;
-    for (int f = threadIdx.x; f < kBI * Q; f += kLeafThreads) {
-        const int r = f % kBI, q = f / kBI;
+    for (int f = threadIdx.x; f < R * Q; f += kLeafThreads) {
+        const int r = f % R, q = f / R;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (base + r < b) v = __ldg(reinterpret_cast<const float4*>(pts + static_cast<size_t>(ids[base + r]) * ld) + q);
-        tile[(4 * q + 0) * kBI + r] = v.x;
-        tile[(4 * q + 1) * kBI + r] = v.y;
-        tile[(4 * q + 2) * kBI + r] = v.z;
-        tile[(4 * q + 3) * kBI + r] = v.w;
+        tile[(4 * q + 0) * R + r] = kNegate ? -v.x : v.x;
+        tile[(4 * q + 1) * R + r] = kNegate ? -v.y : v.y;
+        tile[(4 * q + 2) * R + r] = kNegate ? -v.z : v.z;
+        tile[(4 * q + 3) * R + r] = kNegate ? -v.w : v.w;
     }
 }
 
-// Dm[i][j] = canonical distance(I row i, J row j), thread -> (i, 8 columns).
-template <int D>
+// Two FP32 operations in one instruction (each half rounded as the single
+// operation rounds).
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// Dm[i][j] = canonical distance(I row i, J row j) of R rows and 64 columns,
+// thread -> (i, R / 8 consecutive columns).  I holds the negated rows, so a
+// difference is an add (its sign does not matter to its square); two columns
+// share an instruction.
+template <int D, int R>
 __device__ __forceinline__ void distance_block(const float* __restrict__ I, const float* __restrict__ J,
                                                float* __restrict__ Dm) {
     constexpr int M = D / 8 * 8;
-    const int i = threadIdx.x % kBI;
-    const int jg = threadIdx.x / kBI;  // 0..7
-    const float4* J4 = reinterpret_cast<const float4*>(J);
-    float tot[kJPerThread];
+    constexpr int C = R * kBJ / kLeafThreads;  // columns of a thread
+    constexpr int H = C / 2;
+    static_assert(C == 8 || C == 4 || C == 2, "two to eight columns a thread");
+    const int i = threadIdx.x % R;
+    const int j0 = threadIdx.x / R * C;
+    auto columns = [&](int dim, unsigned long long (&v)[H]) {
+        const float* at = J + dim * kBJ + j0;
+        if constexpr (C == 2) {
+            v[0] = *reinterpret_cast<const unsigned long long*>(at);
+        } else {
 #pragma unroll
-    for (int q = 0; q < kJPerThread; ++q) tot[q] = 0.0f;
+            for (int q = 0; q < C / 4; ++q) {
+                const ulonglong2 x = reinterpret_cast<const ulonglong2*>(at)[q];
+                v[2 * q] = x.x;
+                v[2 * q + 1] = x.y;
+            }
+        }
+    };
+    unsigned long long tot[H];
+#pragma unroll
+    for (int q = 0; q < H; ++q) tot[q] = 0ull;
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
-        float ch[kJPerThread];
+        unsigned long long ch[H];
 #pragma unroll
-        for (int q = 0; q < kJPerThread; ++q) ch[q] = 0.0f;
+        for (int q = 0; q < H; ++q) ch[q] = 0ull;
 #pragma unroll
         for (int dim = c; dim < M; dim += 8) {
-            const float a = I[dim * kBI + i];
-            const float4 v0 = J4[dim * (kBJ / 4) + jg * 2 + 0];
-            const float4 v1 = J4[dim * (kBJ / 4) + jg * 2 + 1];
-            const float bv[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+            const float a = I[dim * R + i];
+            const unsigned long long aa = pack2(a, a);
+            unsigned long long v[H];
+            columns(dim, v);
 #pragma unroll
-            for (int q = 0; q < kJPerThread; ++q) {
-                const float diff = __fsub_rn(a, bv[q]);
-                ch[q] = __fmaf_rn(diff, diff, ch[q]);
+            for (int q = 0; q < H; ++q) {
+                const unsigned long long diff = add2(v[q], aa);
+                ch[q] = fma2(diff, diff, ch[q]);
             }
         }
 #pragma unroll
-        for (int q = 0; q < kJPerThread; ++q) tot[q] = __fadd_rn(tot[q], ch[q]);
+        for (int q = 0; q < H; ++q) tot[q] = add2(tot[q], ch[q]);
     }
 #pragma unroll
     for (int dim = M; dim < D; ++dim) {
-        const float a = I[dim * kBI + i];
-        const float4 v0 = J4[dim * (kBJ / 4) + jg * 2 + 0];
-        const float4 v1 = J4[dim * (kBJ / 4) + jg * 2 + 1];
-        const float bv[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+        const float a = I[dim * R + i];
+        const unsigned long long aa = pack2(a, a);
+        unsigned long long v[H];
+        columns(dim, v);
 #pragma unroll
-        for (int q = 0; q < kJPerThread; ++q) {
-            const float diff = __fsub_rn(a, bv[q]);
-            tot[q] = __fadd_rn(tot[q], __fmul_rn(diff, diff));
+        for (int q = 0; q < H; ++q) {
+            // The product and the sum are rounded one after the other: single
+            // operations, which are never fused.
+            float dx, dy, tx, ty;
+            unpack2(add2(v[q], aa), dx, dy);
+            unpack2(tot[q], tx, ty);
+            tot[q] = pack2(__fadd_rn(tx, __fmul_rn(dx, dx)), __fadd_rn(ty, __fmul_rn(dy, dy)));
         }
     }
 #pragma unroll
-    for (int q = 0; q < kJPerThread; ++q) Dm[i * kDmStride + jg * kJPerThread + q] = tot[q];
+    for (int q = 0; q < H; ++q) unpack2(tot[q], Dm[i * kDmStride + j0 + 2 * q], Dm[i * kDmStride + j0 + 2 * q + 1]);
 }
 
-template <int D>
+// Work of a bucket pass: pos[id] = bucket position array's index of point id
+// (the inverse of idx), and the row blocks of the buckets of at least two
+// points, items[0 .. *n_items) = (bucket, first row), in no particular order.
+__global__ void k_leaf_items(const uint32_t* __restrict__ starts, const uint32_t* __restrict__ ends, uint32_t count,
+                             const uint32_t* __restrict__ dcount, uint32_t rows, const uint32_t* __restrict__ idx,
+                             uint32_t n, uint32_t* __restrict__ pos, uint2* __restrict__ items,
+                             uint32_t* __restrict__ n_items) {
+    if (dcount) count = *dcount;
+    const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    for (uint32_t i = first; i < n; i += stride) pos[idx[i]] = i;
+    for (uint32_t l = first; l < count; l += stride) {
+        const uint32_t b = ends[l] - starts[l];
+        if (b < 2) continue;
+        const uint32_t blocks = (b + rows - 1) / rows;
+        uint32_t at = atomicAdd(n_items, blocks);
+        for (uint32_t k = 0; k < blocks; ++k) items[at++] = make_uint2(l, k * rows);
+    }
+}
+
+// A persistent grid takes row blocks of P * 16 rows (P rows a warp) from the
+// work counter.
+//
+// kOwn: the sets hold distances of these points.  A set's members are then
+// left out of its offers, marked beforehand by their bucket positions (`pos`):
+// every other point of a bucket is offered once, so no offer needs a
+// containment check.  Sets handed over with other distances keep the check.
+//
+// What bounds it: issue slots, shared by the distances (two columns an
+// instruction; FP32 pipe 3,200 cycles a block of 32 x 64 pairs at d = 100) and
+// the set updates (one accepted offer at a time), and in small passes the
+// number of work items: a CTA per bucket left a single 1,000-point bucket to one
+// SM (11.7 ms for four repetitions, now 0.3) and the 156 buckets of a 100k set to
+// half of them (two repetitions 20.7 ms, now 4.5).  Measured on 2M x 100 (four
+// repetitions): 125 ms, from 189 with a CTA per bucket, the check in every
+// offer and one column an instruction.
+template <int D, int P, bool kOwn>
 __global__ void __launch_bounds__(kLeafThreads, 2)
     k_leaf(const uint32_t* __restrict__ starts, const uint32_t* __restrict__ ends, const uint32_t* __restrict__ idx,
-           const float* __restrict__ pts, int ld, float* __restrict__ set_dist, uint32_t* __restrict__ set_id,
-           uint32_t* __restrict__ set_size, uint32_t* __restrict__ set_maxslot, float* __restrict__ set_bound,
-           int K, const uint32_t* __restrict__ dcount, uint32_t* __restrict__ work) {
+           const uint32_t* __restrict__ pos, const float* __restrict__ pts, int ld, float* __restrict__ set_dist,
+           uint32_t* __restrict__ set_id, uint32_t* __restrict__ set_size, uint32_t* __restrict__ set_maxslot,
+           float* __restrict__ set_bound, int K, const uint2* __restrict__ items, const uint32_t* __restrict__ n_items,
+           uint32_t* __restrict__ work) {
+    constexpr int R = P * kLeafWarps;
     extern __shared__ float4 smem4[];
     float* I = reinterpret_cast<float*>(smem4);
-    float* J = I + D * kBI;
+    float* J = I + D * R;
     float* Dm = J + D * kBJ;
-    uint32_t* ids = reinterpret_cast<uint32_t*>(Dm + kBI * kDmStride);
+    uint32_t* marks = reinterpret_cast<uint32_t*>(Dm + R * kDmStride);  // [row][kMarkWords]
+    uint32_t* ids = marks + R * kMarkWords;
     __shared__ uint32_t next_s;
     const int lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
-    // One bucket per CTA, or (with `work`) buckets [0, *dcount) taken one at a
-    // time from the work counter by a persistent grid.
-    for (uint32_t round = 0;; ++round) {
-    uint32_t leaf;
-    if (work) {
+    const uint32_t total = *n_items;
+    for (;;) {
         if (threadIdx.x == 0) next_s = atomicAdd(work, 1u);
         __syncthreads();
-        leaf = next_s;
+        const uint32_t w = next_s;
+        if (w >= total) break;
+        const uint2 item = items[w];
+        const uint32_t s = starts[item.x], b = ends[item.x] - s, ib = item.y;
+        for (uint32_t t = threadIdx.x; t < b; t += kLeafThreads) ids[t] = idx[s + t];
         __syncthreads();
-        if (leaf >= *dcount) break;
-    } else {
-        if (round > 0) break;
-        leaf = blockIdx.x;
-    }
-    const uint32_t s = starts[leaf];
-    const uint32_t b = ends[leaf] - s;
-    if (b < 2) continue;
-    for (uint32_t t = threadIdx.x; t < b; t += kLeafThreads) ids[t] = idx[s + t];
-    __syncthreads();
-    for (uint32_t ib = 0; ib < b; ib += kBI) {
-        load_tile<D>(I, ids, ib, b, pts, ld);
-        WarpSet sets[kPtsPerWarp];
+        load_tile<D, R, true>(I, ids, ib, b, pts, ld);
+        WarpSet sets[P];
 #pragma unroll
-        for (int u = 0; u < kPtsPerWarp; ++u) {
-            const uint32_t p = ib + warp * kPtsPerWarp + u;
+        for (int u = 0; u < P; ++u) {
+            const uint32_t p = ib + warp * P + u;
             if (p < b) set_load(sets[u], set_dist, set_id, set_size, set_maxslot, set_bound, ids[p], K, lane);
         }
         for (uint32_t jb = 0; jb < b; jb += kBJ) {
+            if (kOwn && jb % kMarkCols == 0) {
+                // Member marks of the next kMarkCols positions (this warp's rows).
+#pragma unroll
+                for (int u = 0; u < P; ++u) {
+                    uint32_t* row = marks + (warp * P + u) * kMarkWords;
+                    for (uint32_t t = lane; t < kMarkWords; t += kWarp) row[t] = 0u;
+                    __syncwarp();
+                    if (ib + warp * P + u < b) {
+#pragma unroll
+                        for (int r = 0; r < kSlotsPerLane; ++r) {
+                            if (lane + r * kWarp < static_cast<int>(sets[u].size)) {
+                                const uint32_t at = pos[sets[u].id[r]] - s - jb;
+                                if (at < kMarkCols) atomicOr(&row[at / kWarp], 1u << (at % kWarp));
+                            }
+                        }
+                    }
+                }
+                __syncwarp();
+            }
             __syncthreads();  // previous block's readers of J / Dm are done; I is written
-            load_tile<D>(J, ids, jb, b, pts, ld);
+            load_tile<D, kBJ>(J, ids, jb, b, pts, ld);
             __syncthreads();
-            distance_block<D>(I, J, Dm);
+            distance_block<D, R>(I, J, Dm);
             __syncthreads();
 #pragma unroll
-            for (int u = 0; u < kPtsPerWarp; ++u) {
-                const int row = warp * kPtsPerWarp + u;
+            for (int u = 0; u < P; ++u) {
+                const int row = warp * P + u;
                 const uint32_t p = ib + row;
                 if (p < b) {
 #pragma unroll
                     for (int h = 0; h < kBJ / kWarp; ++h) {
                         const int jj = h * kWarp + lane;
                         const uint32_t j = jb + jj;
-                        const bool valid = j < b && j != p;
                         const float d = Dm[row * kDmStride + jj];
-                        const uint32_t cand = valid ? ids[j] : 0u;
-                        set_offer_batch(sets[u], cand, d, valid, K, lane);
+                        bool valid = j < b && j != p;
+                        if (kOwn) {
+                            valid = valid && !((marks[row * kMarkWords + (jb % kMarkCols) / kWarp + h] >> lane) & 1u);
+                            set_offer_new_batch(sets[u], valid ? ids[j] : 0u, d, valid, K, lane);
+                        } else {
+                            set_offer_batch(sets[u], valid ? ids[j] : 0u, d, valid, K, lane);
+                        }
                     }
                 }
             }
         }
 #pragma unroll
-        for (int u = 0; u < kPtsPerWarp; ++u) {
-            const uint32_t p = ib + warp * kPtsPerWarp + u;
+        for (int u = 0; u < P; ++u) {
+            const uint32_t p = ib + warp * P + u;
             if (p < b) set_store(sets[u], set_dist, set_id, set_size, set_maxslot, set_bound, ids[p], K, lane);
         }
-        __syncthreads();  // everyone is done with I before it is reloaded
-    }
+        __syncthreads();  // everyone is done with ids, I and the work word
     }
 }
 
@@ -212,7 +307,7 @@ __global__ void __launch_bounds__(kLeafThreads, 2)
     const uint32_t q0 = qb * kBI, rows = min(static_cast<uint32_t>(kBI), nq - q0);
     for (uint32_t t = threadIdx.x; t < static_cast<uint32_t>(kBI); t += kLeafThreads) qid[t] = t < rows ? queries[q0 + t] : 0u;
     __syncthreads();
-    load_tile<D>(I, qid, 0, rows, pts, ld);
+    load_tile<D, kBI, true>(I, qid, 0, rows, pts, ld);
     const int lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
     WarpSet sets[kPtsPerWarp];
 #pragma unroll
@@ -230,7 +325,7 @@ __global__ void __launch_bounds__(kLeafThreads, 2)
         __syncthreads();
         load_range_tile<D>(J, jb, c1, pts, ld);
         __syncthreads();
-        distance_block<D>(I, J, Dm);
+        distance_block<D, kBI>(I, J, Dm);
         __syncthreads();
 #pragma unroll
         for (int u = 0; u < kPtsPerWarp; ++u) {
@@ -240,7 +335,8 @@ __global__ void __launch_bounds__(kLeafThreads, 2)
                 for (int h = 0; h < kBJ / kWarp; ++h) {
                     const uint32_t j = jb + h * kWarp + lane;
                     const bool valid = j < c1 && j != qid[row];
-                    set_offer_batch(sets[u], valid ? j : 0u, Dm[row * kDmStride + h * kWarp + lane], valid, K, lane);
+                    set_offer_new_batch(sets[u], valid ? j : 0u, Dm[row * kDmStride + h * kWarp + lane], valid, K,
+                                        lane);
                 }
             }
         }
@@ -495,7 +591,7 @@ __global__ void __launch_bounds__(kLeafThreads, 2)
         for (int k = tid; k < D; k += kLeafThreads) centre[k] = pts[static_cast<size_t>(ids[0]) * ld + k];
         for (uint32_t ib = 0; ib < b && healthy; ib += kBI) {
             __syncthreads();  // the centre is written; the last row block's readers of I are done
-            load_tile<D>(I, ids, ib, b, pts, ld);
+            load_tile<D, kBI>(I, ids, ib, b, pts, ld);
             WarpSet sets[kPtsPerWarp];
 #pragma unroll
             for (int u = 0; u < kPtsPerWarp; ++u) {
@@ -509,7 +605,7 @@ __global__ void __launch_bounds__(kLeafThreads, 2)
                                              rt_a, tid);
             for (uint32_t jb = 0; jb < b; jb += kBJ) {
                 __syncthreads();  // the last column block's readers of J, B and the masks are done
-                load_tile<D>(J, ids, jb, b, pts, ld);
+                load_tile<D, kBJ>(J, ids, jb, b, pts, ld);
                 __syncthreads();
                 if (tid < 2 * kBJ)
                     convert_dm<D>(J, min(static_cast<uint32_t>(kBJ), b - jb), kBJ, Bt, centre, norm_b, rt_b, tid);
@@ -650,6 +746,43 @@ double sample_recall(Context& c, const uint32_t* d_queries, uint32_t nq, const u
     return static_cast<double>(h) / (static_cast<double>(nq) * c.k);
 }
 
+namespace {
+
+// Rows of a block of the FP32 pass: 32 (two a warp) once the points make a block
+// for each of two CTAs an SM, else 16.  64 loads the fewest column tiles per
+// pair, but four sets a warp spill and short buckets waste rows: 2M x 100
+// 130 ms against 125 (four repetitions), 100k x 100 5.6 against 4.7 (eight).
+uint32_t leaf_rows(const Context& c) { return c.n >= 2u * c.sms * 2u * kLeafWarps ? 2u * kLeafWarps : kLeafWarps; }
+
+// The bucket pass over the buckets [0, count) or [0, *dcount): its items, then
+// a persistent grid of leaf_ctas CTAs per SM.  *n_items and *work start at 0.
+void enqueue_leaves(Context& c, uint32_t count, const uint32_t* d_starts, const uint32_t* d_ends, const uint32_t* dcount,
+                    uint2* items, uint32_t* n_items, uint32_t* work, uint32_t max_bucket) {
+    const uint32_t rows = leaf_rows(c);
+    uint32_t* pos = c.indices_tmp;  // the partition's second buffer is free during the pass
+    k_leaf_items<<<std::min<uint32_t>((c.n + 255) / 256, 148 * 8), 256, 0, c.stream>>>(
+        d_starts, d_ends, count, dcount, rows, c.indices, c.n, pos, items, n_items);
+    ++c.launches;
+    KNNG_CUDA(cudaGetLastError());
+    KNNG_DISPATCH_D(c.d, {
+        const size_t smem = static_cast<size_t>(D) * (rows + kBJ) * sizeof(float) +
+                            static_cast<size_t>(rows) * kDmStride * sizeof(float) +
+                            static_cast<size_t>(rows) * kMarkWords * sizeof(uint32_t) +
+                            static_cast<size_t>(std::max<uint32_t>(max_bucket, 1)) * sizeof(uint32_t);
+        if (smem > 227 * 1024) fail(KNNG_ERR_INVALID_ARGUMENT, "bucket too large for the bucket kernel");
+        auto kern = rows == kLeafWarps ? (c.dists_own ? k_leaf<D, 1, true> : k_leaf<D, 1, false>)
+                                       : (c.dists_own ? k_leaf<D, 2, true> : k_leaf<D, 2, false>);
+        allow_max_smem(c, kern);
+        kern<<<c.leaf_ctas * c.sms, kLeafThreads, smem, c.stream>>>(
+            d_starts, d_ends, c.indices, pos, c.points, c.ld, c.set_dist, c.set_id, c.set_size, c.set_maxslot,
+            c.set_bound, static_cast<int>(c.k), items, n_items, work);
+    });
+    ++c.launches;
+    KNNG_CUDA(cudaGetLastError());
+}
+
+}  // namespace
+
 void launch_leaves(Context& c, uint32_t count, const uint32_t* d_starts, const uint32_t* d_ends,
                    uint32_t max_bucket, uint64_t* evals) {
     if (count == 0) return;
@@ -673,30 +806,31 @@ void launch_leaves(Context& c, uint32_t count, const uint32_t* d_starts, const u
         if (h) fail(KNNG_ERR_CUDA, "bucket pass: the MMA completion wait gave up");
         return;
     }
-    KNNG_DISPATCH_D(c.d, {
-        const size_t smem = static_cast<size_t>(D) * (kBI + kBJ) * sizeof(float) +
-                            static_cast<size_t>(kBI) * kDmStride * sizeof(float) +
-                            static_cast<size_t>(std::max<uint32_t>(max_bucket, 1)) * sizeof(uint32_t);
-        if (smem > 227 * 1024) fail(KNNG_ERR_INVALID_ARGUMENT, "bucket too large for the bucket kernel");
-        auto kern = k_leaf<D>;
-        allow_max_smem(c, kern);
-        kern<<<count, kLeafThreads, smem, c.stream>>>(d_starts, d_ends, c.indices, c.points, c.ld, c.set_dist,
-                                                      c.set_id, c.set_size, c.set_maxslot, c.set_bound,
-                                                      static_cast<int>(c.k), nullptr, nullptr);
-    });
-    ++c.launches;
-    KNNG_CUDA(cudaGetLastError());
+    // Row blocks: at most one more than n / rows of each bucket.
+    const uint32_t rows = leaf_rows(c);
+    auto* items = static_cast<uint2*>(scratch(c, "leaf_items", (c.n / rows + static_cast<size_t>(count) + 1) * sizeof(uint2)));
+    auto* counters = static_cast<uint32_t*>(scratch(c, "leaf_counters", 2 * sizeof(uint32_t)));
+    KNNG_CUDA(cudaMemsetAsync(counters, 0, 2 * sizeof(uint32_t), c.stream));
+    enqueue_leaves(c, count, d_starts, d_ends, nullptr, items, counters, counters + 1, max_bucket);
 }
 
 void prepare_leaves_list(Context& c) {
     KNNG_DISPATCH_D(c.d, {
-        allow_max_smem(c, k_leaf<D>);
+        allow_max_smem(c, k_leaf<D, 1, true>);
+        allow_max_smem(c, k_leaf<D, 2, true>);
+        allow_max_smem(c, k_leaf<D, 1, false>);
+        allow_max_smem(c, k_leaf<D, 2, false>);
         allow_max_smem(c, k_leaf_tc<D>);
     });
 }
 
+size_t leaf_items_bytes(uint32_t n) {
+    // Buckets of at least two points, and rows of at least 16 a block.
+    return (static_cast<size_t>(n) / kLeafWarps + n / 2 + 1) * sizeof(uint2);
+}
+
 void launch_leaves_list(Context& c, const uint32_t* d_starts, const uint32_t* d_ends, const uint32_t* d_count,
-                        uint32_t* d_work, uint32_t max_bucket, uint32_t* d_error) {
+                        void* d_items, uint32_t* d_n_items, uint32_t* d_work, uint32_t max_bucket, uint32_t* d_error) {
     if (c.leaf_tc) {
         KNNG_DISPATCH_D(c.d, {
             const size_t smem = LeafTc<D>::bytes(max_bucket);
@@ -712,21 +846,7 @@ void launch_leaves_list(Context& c, const uint32_t* d_starts, const uint32_t* d_
         KNNG_CUDA(cudaGetLastError());
         return;
     }
-    KNNG_DISPATCH_D(c.d, {
-        const size_t smem = static_cast<size_t>(D) * (kBI + kBJ) * sizeof(float) +
-                            static_cast<size_t>(kBI) * kDmStride * sizeof(float) +
-                            static_cast<size_t>(std::max<uint32_t>(max_bucket, 1)) * sizeof(uint32_t);
-        if (smem > 227 * 1024) fail(KNNG_ERR_INVALID_ARGUMENT, "bucket too large for the bucket kernel");
-        auto kern = k_leaf<D>;
-        allow_max_smem(c, kern);
-        const int sms = c.sms;
-        // Persistent: leaf_ctas CTAs per SM take the buckets from the work counter.
-        kern<<<c.leaf_ctas * sms, kLeafThreads, smem, c.stream>>>(d_starts, d_ends, c.indices, c.points, c.ld, c.set_dist,
-                                                        c.set_id, c.set_size, c.set_maxslot, c.set_bound,
-                                                        static_cast<int>(c.k), d_count, d_work);
-    });
-    ++c.launches;
-    KNNG_CUDA(cudaGetLastError());
+    enqueue_leaves(c, 0, d_starts, d_ends, d_count, static_cast<uint2*>(d_items), d_n_items, d_work, max_bucket);
 }
 
 }  // namespace knng

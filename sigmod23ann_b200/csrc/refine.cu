@@ -789,8 +789,9 @@ __device__ __forceinline__ void survivor_keys(const ChainRow<D>& mine, const uin
     }
 }
 
-// Replays a point's survivors buf[0..S), sorted by candidate id, through the
-// sequential set update; returns the number of changes.  One warp.
+// Replays a point's survivors buf[0..S), sorted by candidate id (each once, none
+// a member), through the sequential set update; returns the number of changes.
+// One warp.
 __device__ __forceinline__ uint32_t replay_keys(WarpSet& s, const unsigned long long* buf, uint32_t S, int K, int lane) {
     uint32_t changed = 0;
     for (uint32_t t0 = 0; t0 < S; t0 += kWarp) {
@@ -798,7 +799,7 @@ __device__ __forceinline__ uint32_t replay_keys(WarpSet& s, const unsigned long 
         const unsigned long long key = t < S ? buf[t] : ~0ull;
         const uint32_t cid = static_cast<uint32_t>(key >> 32);
         const float d = __uint_as_float(static_cast<uint32_t>(key & 0xFFFFFFFFu));
-        changed += set_offer_batch(s, cid, d, t < S, K, lane);
+        changed += set_offer_new_batch(s, cid, d, t < S, K, lane);
     }
     return changed;
 }

@@ -694,7 +694,7 @@ constexpr uint32_t kMaxSplitAttempts = 64;
 constexpr uint32_t kMaxLevelIterations = 8192;
 
 struct LevelCounts {
-    uint32_t cur, next, leaves, lloyd_items, part_items, iterations, restarts, fallbacks, nodes, leaf_work;
+    uint32_t cur, next, leaves, lloyd_items, part_items, iterations, restarts, fallbacks, nodes, leaf_work, leaf_items, pad;
     unsigned long long pairs;  // sum of b (b - 1) / 2 over the leaves
 };
 
@@ -1119,6 +1119,7 @@ struct DevRep {
     std::vector<std::pair<void*, size_t>> allocs;
     uint32_t *set_offsets, *table;
     uint32_t *start, *end, *base, *attempt, *nstart, *nend, *nbase, *nattempt, *leaf_start, *leaf_end;
+    uint8_t* leaf_items;  // work items of the bucket pass
     LevelCounts* cnt;
     uint64_t* params;  // seed, repetition, max_leaf, 0
     int32_t* error;    // [0] Lloyd sums, [1] BF16 bucket pass
@@ -1265,6 +1266,7 @@ DevRep& ensure_devrep(Context& c, uint32_t max_leaf, uint32_t small_threshold) {
     r.nattempt = rep_alloc<uint32_t>(c, r, nc);
     r.leaf_start = rep_alloc<uint32_t>(c, r, r.n + r.nsets);
     r.leaf_end = rep_alloc<uint32_t>(c, r, r.n + r.nsets);
+    r.leaf_items = rep_alloc<uint8_t>(c, r, leaf_items_bytes(r.n));
     r.cnt = rep_alloc<LevelCounts>(c, r, 1);
     r.params = rep_alloc<uint64_t>(c, r, 4);
     r.error = rep_alloc<int32_t>(c, r, 4);
@@ -1358,8 +1360,8 @@ void enqueue_buckets(Context& c, DevRep& r, uint32_t max_leaf, uint32_t precisio
         launch_leaves_bf16_list(c, r.leaf_start, r.leaf_end, &r.cnt->leaves, &r.cnt->leaf_work,
                                 reinterpret_cast<uint32_t*>(r.error + 1));
     else
-        launch_leaves_list(c, r.leaf_start, r.leaf_end, &r.cnt->leaves, &r.cnt->leaf_work, max_leaf - 1,
-                           reinterpret_cast<uint32_t*>(r.error + 1));
+        launch_leaves_list(c, r.leaf_start, r.leaf_end, &r.cnt->leaves, r.leaf_items, &r.cnt->leaf_items,
+                           &r.cnt->leaf_work, max_leaf - 1, reinterpret_cast<uint32_t*>(r.error + 1));
 }
 
 // The repetition as one graph: prologue, WHILE (nodes left) { level },
@@ -1367,7 +1369,7 @@ void enqueue_buckets(Context& c, DevRep& r, uint32_t max_leaf, uint32_t precisio
 DevRep::Graph& rep_graph(Context& c, DevRep& r, uint32_t max_leaf, uint32_t lloyd_iters, uint32_t precision) {
     const void* ptrs[8] = {c.points, c.indices, c.indices_tmp, c.set_dist, c.set_id, c.set_size, c.set_bound,
                            reinterpret_cast<const void*>(static_cast<uintptr_t>(c.k))};
-    const uint32_t variant = (c.leaf_tc ? 4u : 0u) | c.leaf_ctas;
+    const uint32_t variant = (c.leaf_tc ? 4u : 0u) | (c.dists_own ? 0u : 8u) | c.leaf_ctas;
     for (auto& g : r.graphs)
         if (g.max_leaf == max_leaf && g.lloyd_iters == lloyd_iters && g.precision == precision &&
             g.leaf_variant == variant && std::equal(ptrs, ptrs + 8, g.ptrs))
@@ -1495,8 +1497,10 @@ void run_rep_device(Context& c, uint32_t max_leaf, uint32_t lloyd_iters, uint32_
     }
     LevelCounts h{};
     download(c, &h, r.cnt, 1);
-    // Kernels the graph ran: prologue (2), every level, the bucket pass.
-    if (graph) c.launches += 3 + static_cast<uint64_t>(h.iterations) * (14 + 3 * lloyd_iters);
+    // Kernels the graph ran: prologue (2), every level, the bucket pass (with
+    // its items in the plain FP32 form).
+    const bool with_items = precision != KNNG_PRECISION_BF16_RERANK && !c.leaf_tc;
+    if (graph) c.launches += (with_items ? 4 : 3) + static_cast<uint64_t>(h.iterations) * (14 + 3 * lloyd_iters);
     int32_t err[4] = {0, 0, 0, 0};
     download(c, err, r.error, 4);
     if (err[0]) fail(KNNG_ERR_CUDA, "Lloyd sums: a bulk-copy wait gave up");
