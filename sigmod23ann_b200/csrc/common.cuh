@@ -301,49 +301,94 @@ __device__ __forceinline__ uint32_t set_offer_batch(WarpSet& s, uint32_t cand, f
     return changed;
 }
 
-// warp_argmax with the common case first: the lanes whose largest slot is the
-// maximum are found by one vote, and if there is one such lane its slot is the
-// answer (slots of one lane share slot % 8, so the first of them wins); ties
-// between lanes go through the full order.
-__device__ __forceinline__ void warp_argmax_quick(WarpSet& s, int K, int lane) {
-    const uint32_t b0 = __float_as_uint(s.dist[0]), b1 = __float_as_uint(s.dist[1]);
-    const uint32_t b2 = __float_as_uint(s.dist[2]), b3 = __float_as_uint(s.dist[3]);
-    static_assert(kSlotsPerLane == 4, "four slots a lane");
-    const uint32_t mine = max(max(b0, b1), max(b2, b3));  // slots past K hold 0
-    const uint32_t top = __reduce_max_sync(kFull, mine);
-    const unsigned holders = __ballot_sync(kFull, mine == top);
-    if ((holders & (holders - 1)) == 0) {
-        const uint32_t r = b0 == mine ? 0u : b1 == mine ? 1u : b2 == mine ? 2u : 3u;
-        s.maxslot = __shfl_sync(kFull, r * kWarp + lane, __ffs(holders) - 1);
-        s.bound = __uint_as_float(top);
-    } else {
-        warp_argmax(s, K, lane);
-    }
-}
-
 // set_offer_batch for candidates that are not in the set and that are offered
 // once: the containment check falls away.  (A caller leaves out the members of
 // the set as it found it; one that is evicted later is at least as far as every
 // later bound, so leaving it out is what offering it would do.)
-__device__ __forceinline__ uint32_t set_offer_new_batch(WarpSet& s, uint32_t cand, float d, bool valid, int K, int lane) {
-    uint32_t changed = 0;
+//
+// Offers that only fill free slots are placed together, by rank; `scratch` is 32
+// bytes of shared memory for that (null: one by one).  A full set's arg-max
+// takes the common case first: the lanes whose largest slot is the maximum are
+// found by one vote, and if there is one such lane its first slot holding it is
+// the answer (slots of one lane share slot % 8); ties between lanes go through
+// the full order.  The slot stays with its lane (its number there in `mine`)
+// until the batch is done.
+__device__ __forceinline__ uint32_t set_offer_new_batch(WarpSet& s, uint32_t cand, float d, bool valid, int K, int lane,
+                                                        uint8_t* scratch = nullptr) {
+    static_assert(kSlotsPerLane == 4, "four slots a lane");
     unsigned pending = __ballot_sync(kFull, valid && d < s.bound);
-    while (pending) {
+    if (pending == 0) return 0;
+    uint32_t changed = 0;
+    if (s.size < static_cast<uint32_t>(K)) {
+        const uint32_t count = __popc(pending);
+        if (scratch && s.size + count <= static_cast<uint32_t>(K)) {
+            if ((pending >> lane) & 1u) scratch[__popc(pending & ((1u << lane) - 1u))] = static_cast<uint8_t>(lane);
+            __syncwarp();
+            const uint32_t rank = (lane - s.size) % kWarp;  // of the slot this lane gets
+            const bool gets = rank < count;
+            const int src = gets ? scratch[rank] : 0;
+            const float dj = __shfl_sync(kFull, d, src);
+            const uint32_t cj = __shfl_sync(kFull, cand, src);
+            const uint32_t at = (s.size + rank) / kWarp;
+#pragma unroll
+            for (uint32_t r = 0; r < kSlotsPerLane; ++r) {
+                if (gets && at == r) {
+                    s.dist[r] = dj;
+                    s.id[r] = cj;
+                }
+            }
+            s.size += count;
+            if (s.size == static_cast<uint32_t>(K)) warp_argmax(s, K, lane);
+            __syncwarp();  // the scratch is read
+            return count;
+        }
+        while (pending && s.size < static_cast<uint32_t>(K)) {
+            const int src = __ffs(pending) - 1;
+            pending &= pending - 1;
+            const float dj = __shfl_sync(kFull, d, src);
+            const uint32_t cj = __shfl_sync(kFull, cand, src);
+            set_write_slot(s, s.size, cj, dj, lane);
+            s.size += 1;
+            ++changed;
+        }
+        if (s.size < static_cast<uint32_t>(K)) return changed;
+        warp_argmax(s, K, lane);
+        pending &= __ballot_sync(kFull, d < s.bound);
+    }
+    if (pending == 0) return changed;
+    int owner = s.maxslot % kWarp;
+    uint32_t mine = s.maxslot / kWarp;
+    do {
         const int src = __ffs(pending) - 1;
         pending &= pending - 1;
         const float dj = __shfl_sync(kFull, d, src);
         const uint32_t cj = __shfl_sync(kFull, cand, src);
-        const bool full = s.size == static_cast<uint32_t>(K);
-        set_write_slot(s, full ? s.maxslot : s.size, cj, dj, lane);
-        ++changed;
-        if (!full) {
-            s.size += 1;
-            if (s.size < static_cast<uint32_t>(K)) continue;  // the bound is still FLT_MAX
+        const bool here = lane == owner;
+#pragma unroll
+        for (uint32_t r = 0; r < kSlotsPerLane; ++r) {
+            if (here && mine == r) {
+                s.dist[r] = dj;
+                s.id[r] = cj;
+            }
         }
-        warp_argmax_quick(s, K, lane);
+        ++changed;
+        const uint32_t b0 = __float_as_uint(s.dist[0]), b1 = __float_as_uint(s.dist[1]);
+        const uint32_t b2 = __float_as_uint(s.dist[2]), b3 = __float_as_uint(s.dist[3]);
+        const uint32_t most = max(max(b0, b1), max(b2, b3));  // slots past K hold 0
+        const uint32_t top = __reduce_max_sync(kFull, most);
+        const unsigned holders = __ballot_sync(kFull, most == top);
+        mine = b0 == most ? 0u : b1 == most ? 1u : b2 == most ? 2u : 3u;
+        owner = 31 - __clz(holders);
+        s.bound = __uint_as_float(top);
+        if (holders != (1u << owner)) {
+            warp_argmax(s, K, lane);
+            owner = s.maxslot % kWarp;
+            mine = s.maxslot / kWarp;
+        }
         // The bound only decreases: drop the candidates it now excludes.
         pending &= __ballot_sync(kFull, d < s.bound);
-    }
+    } while (pending);
+    s.maxslot = __shfl_sync(kFull, mine * kWarp + lane, owner);
     return changed;
 }
 

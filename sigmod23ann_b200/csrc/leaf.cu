@@ -6,9 +6,9 @@
 // inner loop), each offer gated by dist < bound and applied with
 // KnnSetScannableSimd::addCandidateLessThan.  This kernel keeps that order
 // exactly: for a block of rows (a few per warp, sets held in registers) it
-// walks the bucket in 64-point column blocks in ascending order, computes the
+// walks the bucket in 128-point column blocks in ascending order, computes the
 // block's distances in the reference's FP32 order from dim-major shared
-// memory tiles, then each warp replays its points' 64 offers in column order.
+// memory tiles, then each warp replays its points' offers in column order.
 // Distances are computed for the full b x b matrix (both triangles); each
 // (i, j) and (j, i) evaluation gives the same bits.
 // k_leaf_tc makes the same offers but computes distances only for the pairs
@@ -31,26 +31,56 @@ namespace {
 constexpr int kLeafThreads = 512;
 constexpr int kLeafWarps = kLeafThreads / kWarp;  // 16
 constexpr int kBI = 64;                            // rows of the sample k-NN's and k_leaf_tc's blocks (4 a warp)
-constexpr int kBJ = 64;                            // candidates per column block
+constexpr int kBJ = 64;                            // k_leaf_tc's columns per block
 constexpr int kPtsPerWarp = kBI / kLeafWarps;      // 4
-constexpr int kDmStride = kBJ + 1;
+constexpr int kCols = 128;                         // candidates per column block
+constexpr int kDmStride = kCols + 4;               // whole 16-byte stores
 constexpr uint32_t kMarkCols = 1024;               // bucket positions whose member marks are held at a time
 constexpr uint32_t kMarkWords = kMarkCols / kWarp;
 
-// rows [base, base + R) of the bucket -> tile[dim][r] (zeros past the bucket
-// end); kNegate: their negatives.
-template <int D, int R, bool kNegate = false>
+// rows [base, base + 64) of the bucket -> tile[dim][r] (zeros past the bucket
+// end), the layout of k_leaf_tc.
+template <int D>
 __device__ __forceinline__ void load_tile(float* __restrict__ tile, const uint32_t* __restrict__ ids, uint32_t base,
                                           uint32_t b, const float* __restrict__ pts, int ld) {
     constexpr int Q = D / 4;
-    for (int f = threadIdx.x; f < R * Q; f += kLeafThreads) {
-        const int r = f % R, q = f / R;
+    for (int f = threadIdx.x; f < kBI * Q; f += kLeafThreads) {
+        const int r = f % kBI, q = f / kBI;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (base + r < b) v = __ldg(reinterpret_cast<const float4*>(pts + static_cast<size_t>(ids[base + r]) * ld) + q);
-        tile[(4 * q + 0) * R + r] = kNegate ? -v.x : v.x;
-        tile[(4 * q + 1) * R + r] = kNegate ? -v.y : v.y;
-        tile[(4 * q + 2) * R + r] = kNegate ? -v.z : v.z;
-        tile[(4 * q + 3) * R + r] = kNegate ? -v.w : v.w;
+        tile[(4 * q + 0) * kBI + r] = v.x;
+        tile[(4 * q + 1) * kBI + r] = v.y;
+        tile[(4 * q + 2) * kBI + r] = v.z;
+        tile[(4 * q + 3) * kBI + r] = v.w;
+    }
+}
+
+// Dim-major tiles of the distance blocks: dimension `dim` of row r at
+// dim * R + (r ^ tile_swizzle(dim) % R).  A warp fills four rows by eight 16-byte
+// pieces at a time: it reads whole 128-byte lines, and the swizzle (the piece's
+// number in the row index's bits 2-4) sends its 32 values to 32 banks.
+__host__ __device__ constexpr int tile_swizzle(int dim) { return (dim / 4 % 8) * 4; }
+
+// The rows row_id(r), r < count, -> tile of R rows (rows past `count` keep what
+// they hold: no one uses their distances); kNegate: their negatives.
+template <int D, int R, bool kNegate, class RowId>
+__device__ __forceinline__ void fill_tile(float* __restrict__ tile, const float* __restrict__ pts, int ld,
+                                          uint32_t count, RowId row_id) {
+    constexpr int Q = D / 4, QG = (Q + 7) / 8;  // pieces of a row, groups of eight
+    const int lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
+    const int r0 = lane / 8, qq = lane % 8;
+    const int groups = static_cast<int>((min(count, static_cast<uint32_t>(R)) + 3) / 4) * QG;
+#pragma unroll 2
+    for (int g = warp; g < groups; g += kLeafWarps) {
+        const int r = g / QG * 4 + r0, q = g % QG * 8 + qq;
+        if (q < Q && static_cast<uint32_t>(r) < count) {
+            const float4 v = __ldg(reinterpret_cast<const float4*>(pts + static_cast<size_t>(row_id(r)) * ld) + q);
+            float* at = tile + 4 * q * R + (r ^ (qq * 4 % R));
+            at[0] = kNegate ? -v.x : v.x;
+            at[R] = kNegate ? -v.y : v.y;
+            at[2 * R] = kNegate ? -v.z : v.z;
+            at[3 * R] = kNegate ? -v.w : v.w;
+        }
     }
 }
 
@@ -75,73 +105,90 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
     return r;
 }
 
-// Dm[i][j] = canonical distance(I row i, J row j) of R rows and 64 columns,
-// thread -> (i, R / 8 consecutive columns).  I holds the negated rows, so a
-// difference is an add (its sign does not matter to its square); two columns
-// share an instruction.
+// Dm[i][j] = canonical distance(I row i, J row j) of R rows and kCols columns.
+// A thread computes two rows by C columns; a warp covers 16 rows by 4 C
+// columns, so that both operands' loads are one wavefront each (the operands of
+// 16 or 32 distances a lane pair): with a row by four columns a thread, shared
+// memory bandwidth was what the later repetitions waited for (81% of its
+// peak).  I holds the negated rows, so a difference is an add (its sign does not
+// matter to its square); two columns share an instruction.
+// Warps whose rows or columns lie past the block's have nothing to do.
 template <int D, int R>
 __device__ __forceinline__ void distance_block(const float* __restrict__ I, const float* __restrict__ J,
-                                               float* __restrict__ Dm) {
+                                               float* __restrict__ Dm, uint32_t rows, uint32_t cols) {
     constexpr int M = D / 8 * 8;
-    constexpr int C = R * kBJ / kLeafThreads;  // columns of a thread
+    constexpr int C = R * kCols / kLeafThreads / 2;  // columns of a thread
     constexpr int H = C / 2;
-    static_assert(C == 8 || C == 4 || C == 2, "two to eight columns a thread");
-    const int i = threadIdx.x % R;
-    const int j0 = threadIdx.x / R * C;
-    auto columns = [&](int dim, unsigned long long (&v)[H]) {
-        const float* at = J + dim * kBJ + j0;
+    static_assert(C == 4 || C == 2, "two or four columns a thread");
+    static_assert(R % 16 == 0 && R / 16 * (kCols / (4 * C)) == kLeafWarps, "the warps cover the block");
+    const int lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
+    if (static_cast<uint32_t>(warp % (R / 16) * 16) >= rows || static_cast<uint32_t>(warp / (R / 16) * (4 * C)) >= cols) return;
+    const int i0 = warp % (R / 16) * 16 + lane % 8 * 2;
+    const int j0 = warp / (R / 16) * (4 * C) + lane / 8 * C;
+    auto load = [&](int dim, unsigned long long& a0, unsigned long long& a1, unsigned long long (&v)[H]) {
+        const float2 a = *reinterpret_cast<const float2*>(I + dim * R + (i0 ^ (tile_swizzle(dim) % R)));
+        a0 = pack2(a.x, a.x);
+        a1 = pack2(a.y, a.y);
+        const float* at = J + dim * kCols + (j0 ^ (tile_swizzle(dim) % kCols));
         if constexpr (C == 2) {
             v[0] = *reinterpret_cast<const unsigned long long*>(at);
         } else {
-#pragma unroll
-            for (int q = 0; q < C / 4; ++q) {
-                const ulonglong2 x = reinterpret_cast<const ulonglong2*>(at)[q];
-                v[2 * q] = x.x;
-                v[2 * q + 1] = x.y;
-            }
+            const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(at);
+            v[0] = x.x;
+            v[H - 1] = x.y;
         }
     };
-    unsigned long long tot[H];
+    unsigned long long tot[2][H];
 #pragma unroll
-    for (int q = 0; q < H; ++q) tot[q] = 0ull;
+    for (int q = 0; q < H; ++q) tot[0][q] = tot[1][q] = 0ull;
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
-        unsigned long long ch[H];
+        unsigned long long ch[2][H];
 #pragma unroll
-        for (int q = 0; q < H; ++q) ch[q] = 0ull;
+        for (int q = 0; q < H; ++q) ch[0][q] = ch[1][q] = 0ull;
 #pragma unroll
         for (int dim = c; dim < M; dim += 8) {
-            const float a = I[dim * R + i];
-            const unsigned long long aa = pack2(a, a);
-            unsigned long long v[H];
-            columns(dim, v);
+            unsigned long long a0, a1, v[H];
+            load(dim, a0, a1, v);
 #pragma unroll
             for (int q = 0; q < H; ++q) {
-                const unsigned long long diff = add2(v[q], aa);
-                ch[q] = fma2(diff, diff, ch[q]);
+                const unsigned long long d0 = add2(v[q], a0), d1 = add2(v[q], a1);
+                ch[0][q] = fma2(d0, d0, ch[0][q]);
+                ch[1][q] = fma2(d1, d1, ch[1][q]);
             }
         }
 #pragma unroll
-        for (int q = 0; q < H; ++q) tot[q] = add2(tot[q], ch[q]);
+        for (int q = 0; q < H; ++q) {
+            tot[0][q] = add2(tot[0][q], ch[0][q]);
+            tot[1][q] = add2(tot[1][q], ch[1][q]);
+        }
     }
 #pragma unroll
     for (int dim = M; dim < D; ++dim) {
-        const float a = I[dim * R + i];
-        const unsigned long long aa = pack2(a, a);
-        unsigned long long v[H];
-        columns(dim, v);
+        unsigned long long a0, a1, v[H];
+        load(dim, a0, a1, v);
 #pragma unroll
-        for (int q = 0; q < H; ++q) {
-            // The product and the sum are rounded one after the other: single
-            // operations, which are never fused.
-            float dx, dy, tx, ty;
-            unpack2(add2(v[q], aa), dx, dy);
-            unpack2(tot[q], tx, ty);
-            tot[q] = pack2(__fadd_rn(tx, __fmul_rn(dx, dx)), __fadd_rn(ty, __fmul_rn(dy, dy)));
+        for (int r = 0; r < 2; ++r) {
+#pragma unroll
+            for (int q = 0; q < H; ++q) {
+                // The product and the sum are rounded one after the other: single
+                // operations, which are never fused.
+                float dx, dy, tx, ty;
+                unpack2(add2(v[q], r == 0 ? a0 : a1), dx, dy);
+                unpack2(tot[r][q], tx, ty);
+                tot[r][q] = pack2(__fadd_rn(tx, __fmul_rn(dx, dx)), __fadd_rn(ty, __fmul_rn(dy, dy)));
+            }
         }
     }
 #pragma unroll
-    for (int q = 0; q < H; ++q) unpack2(tot[q], Dm[i * kDmStride + j0 + 2 * q], Dm[i * kDmStride + j0 + 2 * q + 1]);
+    for (int r = 0; r < 2; ++r) {
+        float* out = Dm + (i0 + r) * kDmStride + j0;
+        if constexpr (C == 2) {
+            *reinterpret_cast<unsigned long long*>(out) = tot[r][0];
+        } else {
+            *reinterpret_cast<ulonglong2*>(out) = make_ulonglong2(tot[r][0], tot[r][H - 1]);
+        }
+    }
 }
 
 // Work of a bucket pass: pos[id] = bucket position array's index of point id
@@ -171,14 +218,16 @@ __global__ void k_leaf_items(const uint32_t* __restrict__ starts, const uint32_t
 // every other point of a bucket is offered once, so no offer needs a
 // containment check.  Sets handed over with other distances keep the check.
 //
-// What bounds it: issue slots, shared by the distances (two columns an
-// instruction; FP32 pipe 3,200 cycles a block of 32 x 64 pairs at d = 100) and
-// the set updates (one accepted offer at a time), and in small passes the
+// What bounds it: in a first repetition issue slots (0.72 of them used), most
+// of them the accepted offers, which follow one another; later the distances
+// (paired FP32 instructions at 54% of their pipe's peak, shared memory at 67%)
+// and the barriers between a column block's steps.  In small passes it is the
 // number of work items: a CTA per bucket left a single 1,000-point bucket to one
-// SM (11.7 ms for four repetitions, now 0.3) and the 156 buckets of a 100k set to
-// half of them (two repetitions 20.7 ms, now 4.5).  Measured on 2M x 100 (four
-// repetitions): 125 ms, from 189 with a CTA per bucket, the check in every
-// offer and one column an instruction.
+// SM (11.7 ms for four repetitions, now 0.2) and the 156 buckets of a 100k set to
+// half of them (two repetitions 20.7 ms, now 3.3).  Measured on 2M x 100 (four
+// repetitions): 106 ms, from 189 with a CTA per bucket, the check in every
+// offer and one column an instruction; 125 with blocks of 32 x 64 and a row by
+// four columns a thread.
 template <int D, int P, bool kOwn>
 __global__ void __launch_bounds__(kLeafThreads, 2)
     k_leaf(const uint32_t* __restrict__ starts, const uint32_t* __restrict__ ends, const uint32_t* __restrict__ idx,
@@ -190,10 +239,11 @@ __global__ void __launch_bounds__(kLeafThreads, 2)
     extern __shared__ float4 smem4[];
     float* I = reinterpret_cast<float*>(smem4);
     float* J = I + D * R;
-    float* Dm = J + D * kBJ;
+    float* Dm = J + D * kCols;
     uint32_t* marks = reinterpret_cast<uint32_t*>(Dm + R * kDmStride);  // [row][kMarkWords]
     uint32_t* ids = marks + R * kMarkWords;
     __shared__ uint32_t next_s;
+    __shared__ uint8_t place_s[kLeafWarps][kWarp];
     const int lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
     const uint32_t total = *n_items;
     for (;;) {
@@ -205,14 +255,14 @@ __global__ void __launch_bounds__(kLeafThreads, 2)
         const uint32_t s = starts[item.x], b = ends[item.x] - s, ib = item.y;
         for (uint32_t t = threadIdx.x; t < b; t += kLeafThreads) ids[t] = idx[s + t];
         __syncthreads();
-        load_tile<D, R, true>(I, ids, ib, b, pts, ld);
+        fill_tile<D, R, true>(I, pts, ld, b - ib, [&](uint32_t r) { return ids[ib + r]; });
         WarpSet sets[P];
 #pragma unroll
         for (int u = 0; u < P; ++u) {
             const uint32_t p = ib + warp * P + u;
             if (p < b) set_load(sets[u], set_dist, set_id, set_size, set_maxslot, set_bound, ids[p], K, lane);
         }
-        for (uint32_t jb = 0; jb < b; jb += kBJ) {
+        for (uint32_t jb = 0; jb < b; jb += kCols) {
             if (kOwn && jb % kMarkCols == 0) {
                 // Member marks of the next kMarkCols positions (this warp's rows).
 #pragma unroll
@@ -233,9 +283,9 @@ __global__ void __launch_bounds__(kLeafThreads, 2)
                 __syncwarp();
             }
             __syncthreads();  // previous block's readers of J / Dm are done; I is written
-            load_tile<D, kBJ>(J, ids, jb, b, pts, ld);
+            fill_tile<D, kCols, false>(J, pts, ld, b - jb, [&](uint32_t r) { return ids[jb + r]; });
             __syncthreads();
-            distance_block<D, R>(I, J, Dm);
+            distance_block<D, R>(I, J, Dm, b - ib, b - jb);
             __syncthreads();
 #pragma unroll
             for (int u = 0; u < P; ++u) {
@@ -243,14 +293,15 @@ __global__ void __launch_bounds__(kLeafThreads, 2)
                 const uint32_t p = ib + row;
                 if (p < b) {
 #pragma unroll
-                    for (int h = 0; h < kBJ / kWarp; ++h) {
+                    for (int h = 0; h < kCols / kWarp; ++h) {
+                        if (jb + h * kWarp >= b) break;  // warp-uniform
                         const int jj = h * kWarp + lane;
                         const uint32_t j = jb + jj;
                         const float d = Dm[row * kDmStride + jj];
                         bool valid = j < b && j != p;
                         if (kOwn) {
                             valid = valid && !((marks[row * kMarkWords + (jb % kMarkCols) / kWarp + h] >> lane) & 1u);
-                            set_offer_new_batch(sets[u], valid ? ids[j] : 0u, d, valid, K, lane);
+                            set_offer_new_batch(sets[u], valid ? ids[j] : 0u, d, valid, K, lane, place_s[warp]);
                         } else {
                             set_offer_batch(sets[u], valid ? ids[j] : 0u, d, valid, K, lane);
                         }
@@ -271,47 +322,35 @@ __global__ void __launch_bounds__(kLeafThreads, 2)
 //
 // The k nearest points of a sample of query points, by the same FP32
 // distances and set update as the bucket kernel, for the build's recall
-// estimate: CTA (query block of 64, column range) offers its range's points
-// to the 64 queries' sets in point order; k_sample_merge keeps each query's k
+// estimate: CTA (query block of 32, column range) offers its range's points
+// to the 32 queries' sets in point order; k_sample_merge keeps each query's k
 // best (distance, id) over the ranges.
 
-// rows [first, first+64) of [first, last) -> tile[dim][r] (zeros past last)
-template <int D>
-__device__ __forceinline__ void load_range_tile(float* __restrict__ tile, uint32_t first, uint32_t last,
-                                                const float* __restrict__ pts, int ld) {
-    constexpr int Q = D / 4;
-    for (int f = threadIdx.x; f < kBI * Q; f += kLeafThreads) {
-        const int r = f % kBI, q = f / kBI;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (first + r < last) v = __ldg(reinterpret_cast<const float4*>(pts + static_cast<size_t>(first + r) * ld) + q);
-        tile[(4 * q + 0) * kBI + r] = v.x;
-        tile[(4 * q + 1) * kBI + r] = v.y;
-        tile[(4 * q + 2) * kBI + r] = v.z;
-        tile[(4 * q + 3) * kBI + r] = v.w;
-    }
-}
+constexpr int kQueries = 2 * kLeafWarps;  // queries of a block, two a warp
 
 template <int D>
 __global__ void __launch_bounds__(kLeafThreads, 2)
     k_sample_knn(const uint32_t* __restrict__ queries, uint32_t nq, const float* __restrict__ pts, int ld, uint32_t n,
                  uint32_t splits, int K, float* __restrict__ part_dist, uint32_t* __restrict__ part_id,
                  uint32_t* __restrict__ part_size) {
+    constexpr int P = kQueries / kLeafWarps;
     extern __shared__ float4 smem4[];
     float* I = reinterpret_cast<float*>(smem4);
-    float* J = I + D * kBI;
-    float* Dm = J + D * kBJ;
-    uint32_t* qid = reinterpret_cast<uint32_t*>(Dm + kBI * kDmStride);
+    float* J = I + D * kQueries;
+    float* Dm = J + D * kCols;
+    uint32_t* qid = reinterpret_cast<uint32_t*>(Dm + kQueries * kDmStride);
     const uint32_t qb = blockIdx.x / splits, sp = blockIdx.x % splits;
     const uint32_t chunk = (n + splits - 1) / splits;
     const uint32_t c0 = min(n, sp * chunk), c1 = min(n, c0 + chunk);
-    const uint32_t q0 = qb * kBI, rows = min(static_cast<uint32_t>(kBI), nq - q0);
-    for (uint32_t t = threadIdx.x; t < static_cast<uint32_t>(kBI); t += kLeafThreads) qid[t] = t < rows ? queries[q0 + t] : 0u;
+    const uint32_t q0 = qb * kQueries, rows = min(static_cast<uint32_t>(kQueries), nq - q0);
+    for (uint32_t t = threadIdx.x; t < static_cast<uint32_t>(kQueries); t += kLeafThreads)
+        qid[t] = t < rows ? queries[q0 + t] : 0u;
     __syncthreads();
-    load_tile<D, kBI, true>(I, qid, 0, rows, pts, ld);
+    fill_tile<D, kQueries, true>(I, pts, ld, rows, [&](uint32_t r) { return qid[r]; });
     const int lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
-    WarpSet sets[kPtsPerWarp];
+    WarpSet sets[P];
 #pragma unroll
-    for (int u = 0; u < kPtsPerWarp; ++u) {
+    for (int u = 0; u < P; ++u) {
 #pragma unroll
         for (int r = 0; r < kSlotsPerLane; ++r) {
             sets[u].dist[r] = 0.0f;
@@ -321,18 +360,18 @@ __global__ void __launch_bounds__(kLeafThreads, 2)
         sets[u].maxslot = 0;
         sets[u].bound = FLT_MAX;
     }
-    for (uint32_t jb = c0; jb < c1; jb += kBJ) {
+    for (uint32_t jb = c0; jb < c1; jb += kCols) {
         __syncthreads();
-        load_range_tile<D>(J, jb, c1, pts, ld);
+        fill_tile<D, kCols, false>(J, pts, ld, c1 - jb, [&](uint32_t r) { return jb + r; });
         __syncthreads();
-        distance_block<D, kBI>(I, J, Dm);
+        distance_block<D, kQueries>(I, J, Dm, rows, c1 - jb);
         __syncthreads();
 #pragma unroll
-        for (int u = 0; u < kPtsPerWarp; ++u) {
-            const int row = warp * kPtsPerWarp + u;
+        for (int u = 0; u < P; ++u) {
+            const int row = warp * P + u;
             if (static_cast<uint32_t>(row) < rows) {
 #pragma unroll
-                for (int h = 0; h < kBJ / kWarp; ++h) {
+                for (int h = 0; h < kCols / kWarp; ++h) {
                     const uint32_t j = jb + h * kWarp + lane;
                     const bool valid = j < c1 && j != qid[row];
                     set_offer_new_batch(sets[u], valid ? j : 0u, Dm[row * kDmStride + h * kWarp + lane], valid, K,
@@ -342,8 +381,8 @@ __global__ void __launch_bounds__(kLeafThreads, 2)
         }
     }
 #pragma unroll
-    for (int u = 0; u < kPtsPerWarp; ++u) {
-        const uint32_t row = warp * kPtsPerWarp + u;
+    for (int u = 0; u < P; ++u) {
+        const uint32_t row = warp * P + u;
         if (row < rows) {
             const size_t at = static_cast<size_t>(q0 + row) * splits + sp;
 #pragma unroll
@@ -591,7 +630,7 @@ __global__ void __launch_bounds__(kLeafThreads, 2)
         for (int k = tid; k < D; k += kLeafThreads) centre[k] = pts[static_cast<size_t>(ids[0]) * ld + k];
         for (uint32_t ib = 0; ib < b && healthy; ib += kBI) {
             __syncthreads();  // the centre is written; the last row block's readers of I are done
-            load_tile<D, kBI>(I, ids, ib, b, pts, ld);
+            load_tile<D>(I, ids, ib, b, pts, ld);
             WarpSet sets[kPtsPerWarp];
 #pragma unroll
             for (int u = 0; u < kPtsPerWarp; ++u) {
@@ -605,7 +644,7 @@ __global__ void __launch_bounds__(kLeafThreads, 2)
                                              rt_a, tid);
             for (uint32_t jb = 0; jb < b; jb += kBJ) {
                 __syncthreads();  // the last column block's readers of J, B and the masks are done
-                load_tile<D, kBJ>(J, ids, jb, b, pts, ld);
+                load_tile<D>(J, ids, jb, b, pts, ld);
                 __syncthreads();
                 if (tid < 2 * kBJ)
                     convert_dm<D>(J, min(static_cast<uint32_t>(kBJ), b - jb), kBJ, Bt, centre, norm_b, rt_b, tid);
@@ -710,9 +749,9 @@ __global__ void __launch_bounds__(kLeafThreads, 2)
 void sample_knn(Context& c, const uint32_t* d_queries, uint32_t nq, uint32_t* d_truth) {
     if (nq == 0) return;
     const int K = static_cast<int>(c.k);
-    const uint32_t qblocks = (nq + kBI - 1) / kBI;
+    const uint32_t qblocks = (nq + kQueries - 1) / kQueries;
     const uint32_t splits = std::max<uint32_t>(1, std::min<uint32_t>((2u * c.sms + qblocks - 1) / qblocks,
-                                                                      (c.n + kBJ - 1) / kBJ));
+                                                                      (c.n + kCols - 1) / kCols));
     auto* pd = static_cast<float*>(scratch(c, "sknn_dist", static_cast<size_t>(nq) * splits * K * sizeof(float)));
     auto* pi = static_cast<uint32_t*>(scratch(c, "sknn_id", static_cast<size_t>(nq) * splits * K * sizeof(uint32_t)));
     auto* ps = static_cast<uint32_t*>(scratch(c, "sknn_size", static_cast<size_t>(nq) * splits * sizeof(uint32_t)));
@@ -721,8 +760,8 @@ void sample_knn(Context& c, const uint32_t* d_queries, uint32_t nq, uint32_t* d_
     auto* keys = static_cast<unsigned long long*>(
         scratch(c, "sknn_keys", static_cast<size_t>(nq) * cap * sizeof(unsigned long long)));
     KNNG_DISPATCH_D(c.d, {
-        const size_t smem = static_cast<size_t>(D) * (kBI + kBJ) * sizeof(float) +
-                            static_cast<size_t>(kBI) * kDmStride * sizeof(float) + kBI * sizeof(uint32_t);
+        const size_t smem = static_cast<size_t>(D) * (kQueries + kCols) * sizeof(float) +
+                            static_cast<size_t>(kQueries) * kDmStride * sizeof(float) + kQueries * sizeof(uint32_t);
         auto kern = k_sample_knn<D>;
         allow_max_smem(c, kern);
         kern<<<qblocks * splits, kLeafThreads, smem, c.stream>>>(d_queries, nq, c.points, c.ld, c.n, splits, K, pd,
@@ -765,7 +804,7 @@ void enqueue_leaves(Context& c, uint32_t count, const uint32_t* d_starts, const 
     ++c.launches;
     KNNG_CUDA(cudaGetLastError());
     KNNG_DISPATCH_D(c.d, {
-        const size_t smem = static_cast<size_t>(D) * (rows + kBJ) * sizeof(float) +
+        const size_t smem = static_cast<size_t>(D) * (rows + kCols) * sizeof(float) +
                             static_cast<size_t>(rows) * kDmStride * sizeof(float) +
                             static_cast<size_t>(rows) * kMarkWords * sizeof(uint32_t) +
                             static_cast<size_t>(std::max<uint32_t>(max_bucket, 1)) * sizeof(uint32_t);
