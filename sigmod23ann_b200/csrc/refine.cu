@@ -247,8 +247,8 @@ __global__ void __launch_bounds__(kRefWarps * kWarp)
 //                 repeats, get the exact FP32 distance; survivors are sorted by
 //                 id and replayed through the sequential set update in ascending
 //                 id order -- the same offers, in the same order, as the
-//                 per-point pass (one warp up to 1,024 candidates, k_apply_big
-//                 up to 8,192).
+//                 per-point pass (one warp up to 800 candidates, k_apply_big up
+//                 to 8,192).
 //   Points with more candidates are redone by k_refine.  When the budget has no
 //   room for every edge's bits, the pass goes over ranges of points p (1 to 3
 //   for each range; the snapshot, and so the result, is the same).
@@ -658,32 +658,48 @@ __global__ void __launch_bounds__(kJoinThreads, kJoinPerSm)
 // ---------------------------------------------------------------- replay
 //
 // Per point p: the columns that the join left of each of p's K lists, minus
-// p's members and the repeats (a hash set in shared memory), get the exact
-// FP32 distance; the survivors (distance < bound(p)) are sorted by id and
-// replayed through the sequential set update -- the offers of the per-point
-// pass, in its order.  One warp per point up to kWarpCands candidates, then
+// p's members and the repeats (a hash set in shared memory), are sorted by id and
+// offered in that order with their exact FP32 distances -- the offers of the
+// per-point pass, in its order.  One warp per point up to kWarpCands candidates, then
 // one CTA up to kCtaCands, then the per-point pass.
 
 constexpr int kApplyWarps = 5;
-constexpr uint32_t kWarpCands = 1024;   // candidates of a point that one warp handles
-constexpr uint32_t kWarpTable = 2048;   // its hash slots (members, p and candidates)
+constexpr int kApplyPerSm = 4;
+constexpr uint32_t kWarpCands = 800;    // candidates of a point that one warp handles
+constexpr uint32_t kWarpTable = 1024;   // its hash slots (members, p, candidates and what a step adds past the cap)
 constexpr uint32_t kWarpList = 1024;    // mask bits expanded at a time
 constexpr int kBigThreads = 256;
 constexpr uint32_t kCtaCands = 8192;
 constexpr uint32_t kCtaTable = 16384;
 
-// Inserts id (below 2^31) into an open-addressing table of `slots` (a power of
-// two, never full) ids; `mark` (kMember or 0) goes in with it.  Returns the
-// mark it was found with, or kFresh.
+// Inserts id (below 2^31) into a table of `buckets` (a power of two) buckets of
+// four ids, never full; `mark` (kMember or 0) goes in with it.  Returns the mark
+// it was found with, or kFresh.  A bucket is one 16-byte load and fills from its
+// front, so nearly every id -- most are there already -- takes one step (with
+// single slots a warp waited for its longest probe chain).
 constexpr uint32_t kMember = 0x80000000u;
 constexpr uint32_t kFresh = 1u;
-__device__ __forceinline__ uint32_t table_insert(uint32_t* table, uint32_t slots, uint32_t id, uint32_t mark) {
-    uint32_t h = (id * 0x9E3779B1u) >> (__clz(slots) + 1);
-    for (uint32_t probe = 0; probe < slots; ++probe) {
-        const uint32_t prev = atomicCAS(&table[h], kNone, id | mark);
-        if (prev == kNone) return kFresh;
-        if ((prev & ~kMember) == id) return prev & kMember;
-        h = (h + 1) & (slots - 1);
+__device__ __forceinline__ uint32_t table_insert(uint32_t* table, uint32_t buckets, uint32_t id, uint32_t mark) {
+    uint32_t h = (id * 0x9E3779B1u) >> (__clz(buckets) + 1);
+    for (uint32_t probe = 0; probe < 8 * buckets; ++probe) {
+        uint4 v;
+        asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                     : "r"(tc::smem_u32(table + 4 * h))
+                     : "memory");
+        uint32_t hit = kFresh;  // the entry found, without its id's bits
+        hit = ((v.x ^ id) & ~kMember) == 0 ? v.x & kMember : hit;
+        hit = ((v.y ^ id) & ~kMember) == 0 ? v.y & kMember : hit;
+        hit = ((v.z ^ id) & ~kMember) == 0 ? v.z & kMember : hit;
+        hit = ((v.w ^ id) & ~kMember) == 0 ? v.w & kMember : hit;
+        if (hit != kFresh) return hit;
+        if (v.w == kNone) {
+            const uint32_t slot = v.x == kNone ? 0u : v.y == kNone ? 1u : v.z == kNone ? 2u : 3u;
+            if (atomicCAS(&table[4 * h + slot], kNone, id | mark) == kNone) return kFresh;
+            // Another lane took the slot: the bucket is read again.
+        } else {
+            h = (h + 1) & (buckets - 1);
+        }
     }
     return 0u;
 }
@@ -756,69 +772,172 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// Exact distances of candidates ids[first .. U) (step `step`, four at a time,
-// one per group of eight lanes) to the row `mine`; survivors' keys
-// (id << 32 | distance bits) are appended to keys through `put`, which returns
-// the position for the calling warp's `count` survivors.
-template <int D, class Put>
-__device__ __forceinline__ void survivor_keys(const ChainRow<D>& mine, const uint32_t* ids, uint32_t first, uint32_t step,
-                                              uint32_t U, float bound0, const float* __restrict__ pts, int ld,
-                                              unsigned long long* keys, int lane, Put put) {
-    const int l = lane & 7, g = lane >> 3, g0 = lane & ~7;
-    for (uint32_t t0 = first; t0 < U; t0 += step) {
-        constexpr int V = 2;  // candidates of a group in flight
-        ChainRow<D> row[V];
-        uint32_t id[V];
-#pragma unroll
-        for (int v = 0; v < V; ++v) {
-            const uint32_t t = t0 + 4 * v + g;
-            id[v] = ids[t < U ? t : t0];
-            load_chain_row<D>(row[v], pts + static_cast<size_t>(id[v]) * ld, l);
-        }
-#pragma unroll
-        for (int v = 0; v < V; ++v) {
-            const float d = group_distance<D>(row[v], mine, g0);
-            const bool in = t0 + 4 * v + g < U && d < bound0;
-            const unsigned b = __ballot_sync(kFull, in && l == 0);
-            if (b == 0) continue;
-            const uint32_t at = put(static_cast<uint32_t>(__popc(b)));
-            if (in && l == 0)
-                keys[at + __popc(b & ((1u << lane) - 1u))] =
-                    (static_cast<unsigned long long>(id[v]) << 32) | __float_as_uint(d);
-        }
-    }
+// A load that stays where it is written (the compiler otherwise puts a row's
+// loads next to their uses, and each row waits for its own latency).
+__device__ __forceinline__ float load_now(const float* p) {
+    float v;
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
 }
 
-// Replays a point's survivors buf[0..S), sorted by candidate id (each once, none
-// a member), through the sequential set update; returns the number of changes.
-// One warp.
-__device__ __forceinline__ uint32_t replay_keys(WarpSet& s, const unsigned long long* buf, uint32_t S, int K, int lane) {
+// canonical_distance of `mine` (p's row) and the rows of 32 points, lane t's
+// point id t; every lane returns its own.  A group of eight lanes reads its
+// eight rows one after the other, a lane a chain (32 bytes of each row a load);
+// the chains are then exchanged within the group, so that each lane sums the
+// eight of its own point and adds its tail.
+template <int D>
+__device__ __forceinline__ float warp_distances(const ChainRow<D>& mine, uint32_t id, const float* __restrict__ pts,
+                                                int ld, int lane) {
+    constexpr int M = ChainRow<D>::M;
+    static_assert(D - M == 0 || D - M == 4, "tail of 0 or 4 dims");
+    const int l = lane & 7, g0 = lane & ~7;
+    float4 tail = make_float4(0.f, 0.f, 0.f, 0.f);
+    if constexpr (D > M) tail = __ldg(reinterpret_cast<const float4*>(pts + static_cast<size_t>(id) * ld + M));
+    // Four rows' loads in flight, then their chains.
+    float x[8];
+    constexpr int V = 4;
+#pragma unroll
+    for (int v0 = 0; v0 < 8; v0 += V) {
+        float y[V][M / 8];
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            const float* row = pts + static_cast<size_t>(__shfl_sync(kFull, id, g0 + v0 + v)) * ld + l;
+#pragma unroll
+            for (int i = 0; i < M / 8; ++i) y[v][i] = load_now(row + 8 * i);
+        }
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            float chain = 0.0f;
+#pragma unroll
+            for (int i = 0; i < M / 8; ++i) {
+                const float d = __fsub_rn(y[v][i], mine.c[i]);
+                chain = __fmaf_rn(d, d, chain);
+            }
+            x[v0 + v] = chain;
+        }
+    }
+#pragma unroll
+    for (int s = 1; s < 8; s <<= 1) {
+        const bool high = (l & s) != 0;
+#pragma unroll
+        for (int a = 0; a < 8; ++a) {
+            if (a & s) continue;
+            const float got = __shfl_xor_sync(kFull, high ? x[a] : x[a | s], s);
+            if (high) x[a] = got; else x[a | s] = got;
+        }
+    }
+    float acc = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc = __fadd_rn(acc, x[j]);
+    if constexpr (D > M) {
+        float d = __fsub_rn(tail.x, mine.tail.x);
+        acc = __fadd_rn(acc, __fmul_rn(d, d));
+        d = __fsub_rn(tail.y, mine.tail.y);
+        acc = __fadd_rn(acc, __fmul_rn(d, d));
+        d = __fsub_rn(tail.z, mine.tail.z);
+        acc = __fadd_rn(acc, __fmul_rn(d, d));
+        d = __fsub_rn(tail.w, mine.tail.w);
+        acc = __fadd_rn(acc, __fmul_rn(d, d));
+    }
+    return acc;
+}
+
+// Ascending sort of ids[0 .. U), U <= 32 E, by one warp: a bitonic network over
+// E registers a lane (element lane * E + r).  Strides below E stay in a lane;
+// the lanes whose block a level sorts downwards hold its keys complemented, so
+// that every exchange in a lane is a minimum and a maximum.
+template <int E>
+__device__ __forceinline__ void warp_sort_ids(uint32_t* ids, uint32_t U, int lane) {
+    uint32_t x[E];
+#pragma unroll
+    for (int r = 0; r < E; ++r) x[r] = lane * E + r < static_cast<int>(U) ? ids[lane * E + r] : kNone;
+#pragma unroll
+    for (int k = 2; k <= E; k <<= 1) {
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+#pragma unroll
+            for (int r = 0; r < E; ++r) {
+                if (r & j) continue;
+                // Direction of element lane * E + r at level k: within the lane
+                // below E, the lane's own bit at E.
+                const bool up = k < E ? (r & k) == 0 : (lane & 1) == 0;
+                const uint32_t lo = min(x[r], x[r | j]), hi = max(x[r], x[r | j]);
+                x[r] = up ? lo : hi;
+                x[r | j] = up ? hi : lo;
+            }
+        }
+    }
+    uint32_t flip = 0;
+#pragma unroll
+    for (int k = 2; k <= kWarp; k <<= 1) {  // level k * E: blocks of k lanes
+        const uint32_t want = (lane & k) ? kNone : 0u;
+#pragma unroll
+        for (int r = 0; r < E; ++r) x[r] ^= flip ^ want;
+        flip = want;
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            const bool low = (lane & j) == 0;
+#pragma unroll
+            for (int r = 0; r < E; ++r) {
+                const uint32_t o = __shfl_xor_sync(kFull, x[r], j);
+                x[r] = low ? min(x[r], o) : max(x[r], o);
+            }
+        }
+#pragma unroll
+        for (int j = E >> 1; j > 0; j >>= 1) {
+#pragma unroll
+            for (int r = 0; r < E; ++r) {
+                if (r & j) continue;
+                const uint32_t lo = min(x[r], x[r | j]), hi = max(x[r], x[r | j]);
+                x[r] = lo;
+                x[r | j] = hi;
+            }
+        }
+    }
+    // The last level (k = 32) sorts upwards in every lane.
+#pragma unroll
+    for (int r = 0; r < E; ++r)
+        if (lane * E + r < static_cast<int>(U)) ids[lane * E + r] = x[r];
+    __syncwarp();
+}
+
+// Offers a point's candidates ids[0 .. U) (sorted, each once, none a member), 32
+// at a time, with their exact distances; returns the number of changes.  One
+// warp.  (A candidate is offered when its distance is below the bound it meets;
+// the bound p had when its pass started rules nothing else out.)
+template <int D>
+__device__ __forceinline__ uint32_t offer_sorted(WarpSet& s, const uint32_t* ids, uint32_t U, uint32_t p,
+                                                 const float* __restrict__ pts, int ld, int K, int lane) {
+    ChainRow<D> mine;
+    load_chain_row<D>(mine, pts + static_cast<size_t>(p) * ld, lane & 7);
     uint32_t changed = 0;
-    for (uint32_t t0 = 0; t0 < S; t0 += kWarp) {
-        const uint32_t t = t0 + lane;
-        const unsigned long long key = t < S ? buf[t] : ~0ull;
-        const uint32_t cid = static_cast<uint32_t>(key >> 32);
-        const float d = __uint_as_float(static_cast<uint32_t>(key & 0xFFFFFFFFu));
-        changed += set_offer_new_batch(s, cid, d, t < S, K, lane);
+    for (uint32_t t0 = 0; t0 < U; t0 += kWarp) {
+        const uint32_t id = ids[min(t0 + lane, U - 1)];
+        const float d = warp_distances<D>(mine, id, pts, ld, lane);
+        changed += set_offer_new_batch(s, id, d, t0 + lane < U, K, lane);
     }
     return changed;
 }
 
-// Shared memory of one warp of k_apply: the hash table (the survivors' keys
-// once every candidate is known), the candidates, the expanded mask bits, p's
-// own list.
+// Shared memory of one warp of k_apply: the hash table, the candidates, the
+// expanded mask bits, p's own list.
 struct ApplyWarpSmem {
     uint32_t table[kWarpTable];
-    uint32_t cands[kWarpCands];
+    uint32_t cands[kWarpTable];  // a power of two, for the sort
     uint16_t list[kWarpList];
     uint32_t mine[kMaxK];
 };
 
-// Points of [lo, hi), in `order` when given.  What bounds it is latency per
-// point (masks, list entries, rows are dependent gathers, mostly L2 hits): 15
-// warps an SM, each with many loads in flight.
+// Points of [lo, hi), in `order` when given.  What bounds it: per point some 200
+// candidate rows and 2,300 list entries gathered from L2 (5 TB/s at 2M points,
+// where gathers alone reach 9), behind chains of dependent steps that few warps
+// hide, so shared memory and registers are cut to 20 warps an SM: 15 warps with
+// tables twice the size took 113 ms for the two passes of a 2M build, 25 with a
+// cap of 512 candidates 144 (the points past it are slow), this 98; it was 111
+// with the distances first, 64-bit keys sorted in shared memory and single-slot
+// probes.
 template <int D>
-__global__ void __launch_bounds__(kApplyWarps * kWarp, 3)
+__global__ void __launch_bounds__(kApplyWarps * kWarp, kApplyPerSm)
     k_apply(const uint32_t* __restrict__ snap, const uint4* __restrict__ masks, const float* __restrict__ pts, int ld,
             uint32_t n, uint32_t lo, uint32_t hi, int K, uint32_t cap, const uint32_t* __restrict__ order,
             const uint32_t* __restrict__ error_flag, float* __restrict__ set_dist, uint32_t* __restrict__ set_id,
@@ -828,8 +947,6 @@ __global__ void __launch_bounds__(kApplyWarps * kWarp, 3)
     extern __shared__ __align__(1024) unsigned char smem[];
     const int lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
     ApplyWarpSmem& sm = reinterpret_cast<ApplyWarpSmem*>(smem)[warp];
-    unsigned long long* keys = reinterpret_cast<unsigned long long*>(sm.table);
-    static_assert(sizeof(sm.table) >= kWarpCands * sizeof(unsigned long long), "the keys take the table's space");
     const unsigned lt = (1u << lane) - 1u;
     unsigned long long n_member = 0, n_record = 0, n_exact = 0;
     uint32_t n_changed = 0;
@@ -837,7 +954,7 @@ __global__ void __launch_bounds__(kApplyWarps * kWarp, 3)
     for (uint32_t w = blockIdx.x * kApplyWarps + warp; w < n; w += gridDim.x * kApplyWarps) {
         const uint32_t p = order ? order[w] : w;
         if (p < lo || p >= hi) continue;
-        __syncwarp();  // the last point's keys are read
+        __syncwarp();  // the last point's candidates are read
         const uint32_t* list = snap + static_cast<size_t>(p) * K;
         const uint4* mask = masks + static_cast<size_t>(p - lo) * K;
         for (int a = lane; a < K; a += kWarp) sm.mine[a] = list[a];
@@ -847,10 +964,10 @@ __global__ void __launch_bounds__(kApplyWarps * kWarp, 3)
         set_load(s, set_dist, set_id, set_size, set_maxslot, set_bound, p, K, lane);
         __syncwarp();
         // p and its members first: they are never candidates.
-        if (lane == 0) table_insert(sm.table, kWarpTable, p, kMember);
+        if (lane == 0) table_insert(sm.table, kWarpTable / 4, p, kMember);
 #pragma unroll
         for (int r = 0; r < kSlotsPerLane; ++r)
-            if (lane + r * kWarp < static_cast<int>(s.size)) table_insert(sm.table, kWarpTable, s.id[r], kMember);
+            if (lane + r * kWarp < static_cast<int>(s.size)) table_insert(sm.table, kWarpTable / 4, s.id[r], kMember);
         __syncwarp();
         uint32_t U = 0, records = 0, members = 0;
         bool fits = true;
@@ -860,14 +977,19 @@ __global__ void __launch_bounds__(kApplyWarps * kWarp, 3)
             const int a = a0 + lane;
             uint4 m = make_uint4(0u, 0u, 0u, 0u);
             if (a < K && (a == 0 || sm.mine[a - 1] != sm.mine[a])) m = mask[a];
-            uint32_t part[4] = {m.x, m.y, m.z, m.w};
             const uint32_t bits = __popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w);
             const uint32_t all = __reduce_add_sync(kFull, bits);
             if (all == 0) continue;
-            // All four words at once when they fit the list, else one by one.
+            // All four words at once when they fit the list, else a word at a time
+            // (32 lanes' 32 bits fill it at most).
             const int steps = all <= kWarpList ? 1 : 4;
             for (int step = 0; step < steps && fits; ++step) {
-                uint32_t have = steps == 1 ? bits : static_cast<uint32_t>(__popc(step == 0 ? part[0] : step == 1 ? part[1] : step == 2 ? part[2] : part[3]));
+                uint32_t w[4] = {m.x, m.y, m.z, m.w};
+                if (steps > 1) {
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) w[x] = step == x ? w[x] : 0u;
+                }
+                const uint32_t have = __popc(w[0]) + __popc(w[1]) + __popc(w[2]) + __popc(w[3]);
                 uint32_t incl = have;
 #pragma unroll
                 for (int o = 1; o < kWarp; o <<= 1) {
@@ -877,36 +999,33 @@ __global__ void __launch_bounds__(kApplyWarps * kWarp, 3)
                 const uint32_t T = __shfl_sync(kFull, incl, kWarp - 1);
                 uint32_t at = incl - have;
 #pragma unroll
-                for (int x = 0; x < 4; ++x) {
-                    if (steps == 4 && x != step) continue;
-                    for (uint32_t b = part[x]; b; b &= b - 1)
+                for (int x = 0; x < 4; ++x)
+                    for (uint32_t b = w[x]; b; b &= b - 1)
                         sm.list[at++] = static_cast<uint16_t>(a << 7 | (x * kWarp + __ffs(b) - 1));
+                __syncwarp();
+                // Entry t of the list: its id, four steps ahead of its insertion.
+                auto entry = [&](uint32_t t) {
+                    if (t >= T) return kNone;
+                    const uint32_t x = sm.list[t];
+                    return __ldg(snap + static_cast<size_t>(sm.mine[x >> 7]) * K + (x & 127u));
+                };
+                uint32_t c0 = entry(lane), c1 = entry(kWarp + lane), c2 = entry(2 * kWarp + lane), c3 = entry(3 * kWarp + lane);
+                for (uint32_t t0 = 0; t0 < T && fits; t0 += kWarp) {
+                    const uint32_t c = c0;
+                    c0 = c1;
+                    c1 = c2;
+                    c2 = c3;
+                    c3 = entry(t0 + 4 * kWarp + lane);
+                    const uint32_t found = c != kNone ? table_insert(sm.table, kWarpTable / 4, c, 0u) : 0u;
+                    const bool fresh = found == kFresh;
+                    members += found == kMember ? 1u : 0u;
+                    const unsigned b = __ballot_sync(kFull, fresh);
+                    const uint32_t at2 = U + __popc(b & lt);
+                    if (fresh) sm.cands[at2] = c;  // at most a step past the cap
+                    U += __popc(b);
+                    fits = U <= cap;
                 }
                 __syncwarp();
-                for (uint32_t t0 = 0; t0 < T && fits; t0 += 4 * kWarp) {
-                    uint32_t c[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const uint32_t t = t0 + u * kWarp + lane;
-                        c[u] = kNone;
-                        if (t < T) {
-                            const uint32_t x = sm.list[t];
-                            c[u] = __ldg(snap + static_cast<size_t>(sm.mine[x >> 7]) * K + (x & 127u));
-                        }
-                    }
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const uint32_t found = c[u] != kNone ? table_insert(sm.table, kWarpTable, c[u], 0u) : 0u;
-                        const bool fresh = found == kFresh;
-                        members += found == kMember ? 1u : 0u;
-                        const unsigned b = __ballot_sync(kFull, fresh);
-                        const uint32_t at2 = U + __popc(b & lt);
-                        if (fresh && at2 < kWarpCands) sm.cands[at2] = c[u];
-                        U += __popc(b);
-                    }
-                    fits = U <= cap;
-                    __syncwarp();
-                }
                 records += T;
             }
         }
@@ -918,27 +1037,21 @@ __global__ void __launch_bounds__(kApplyWarps * kWarp, 3)
         n_record += lane == 0 ? records : 0u;
         n_exact += lane == 0 ? U : 0u;
         if (U == 0) continue;
-        ChainRow<D> row;
-        load_chain_row<D>(row, pts + static_cast<size_t>(p) * ld, lane & 7);
-        uint32_t S = 0;
-        survivor_keys<D>(row, sm.cands, 0, 8, U, s.bound, pts, ld, keys, lane, [&](uint32_t count) {
-            const uint32_t at = S;
-            S += count;
-            return at;
-        });
-        if (S == 0) {
+        if (U <= 4 * kWarp)
+            warp_sort_ids<4>(sm.cands, U, lane);
+        else if (U <= 8 * kWarp)
+            warp_sort_ids<8>(sm.cands, U, lane);
+        else if (U <= 16 * kWarp)
+            warp_sort_ids<16>(sm.cands, U, lane);
+        else {
+            for (uint32_t t = U + lane; t < kWarpTable; t += kWarp) sm.cands[t] = kNone;
             __syncwarp();
-            continue;
+            warp_bitonic_sort(sm.cands, kWarpTable, lane);
         }
-        const uint32_t P2 = pow2_at_least(S);
-        for (uint32_t t = S + lane; t < P2; t += kWarp) keys[t] = ~0ull;
-        __syncwarp();
-        warp_bitonic_sort(keys, P2, lane);
-        if (replay_keys(s, keys, S, K, lane)) {
+        if (offer_sorted<D>(s, sm.cands, U, p, pts, ld, K, lane)) {
             set_store(s, set_dist, set_id, set_size, set_maxslot, set_bound, p, K, lane);
             ++n_changed;
         }
-        __syncwarp();
     }
     if (n_member) atomicAdd(&counters[2], n_member);
     if (lane == 0) {
@@ -965,9 +1078,7 @@ __global__ void __launch_bounds__(kBigThreads)
                 uint32_t* __restrict__ lost, uint32_t* __restrict__ lost_n, unsigned long long* __restrict__ counters) {
     extern __shared__ __align__(1024) unsigned char smem[];
     ApplyBigSmem& sm = *reinterpret_cast<ApplyBigSmem*>(smem);
-    unsigned long long* keys = reinterpret_cast<unsigned long long*>(sm.table);
-    static_assert(sizeof(sm.table) >= kCtaCands * sizeof(unsigned long long), "the keys take the table's space");
-    __shared__ uint32_t found_s, keys_s;
+    __shared__ uint32_t found_s;
     constexpr int kWarps = kBigThreads / kWarp;
     const int tid = threadIdx.x, lane = tid % kWarp, warp = tid / kWarp;
     const uint32_t total = *big_n;
@@ -978,11 +1089,11 @@ __global__ void __launch_bounds__(kBigThreads)
         for (uint32_t t = tid; t < kCtaTable / 4; t += kBigThreads)
             reinterpret_cast<uint4*>(sm.table)[t] = make_uint4(kNone, kNone, kNone, kNone);
         for (int a = tid; a < K; a += kBigThreads) sm.mine[a] = list[a];
-        if (tid == 0) found_s = keys_s = 0;
+        if (tid == 0) found_s = 0;
         __syncthreads();
-        if (tid == 0) table_insert(sm.table, kCtaTable, p, kMember);
+        if (tid == 0) table_insert(sm.table, kCtaTable / 4, p, kMember);
         for (uint32_t t = tid; t < set_size[p]; t += kBigThreads)
-            table_insert(sm.table, kCtaTable, set_id[static_cast<size_t>(p) * K + t], kMember);
+            table_insert(sm.table, kCtaTable / 4, set_id[static_cast<size_t>(p) * K + t], kMember);
         __syncthreads();
         uint32_t members = 0, records = 0;
         for (int a = warp; a < K; a += kWarps) {
@@ -997,7 +1108,7 @@ __global__ void __launch_bounds__(kBigThreads)
                 uint32_t c = 0, found = 0;
                 if ((part[x] >> lane) & 1u) {
                     c = __ldg(snap + static_cast<size_t>(sm.mine[a]) * K + x * kWarp + lane);
-                    found = table_insert(sm.table, kCtaTable, c, 0u);
+                    found = table_insert(sm.table, kCtaTable / 4, c, 0u);
                 }
                 members += found == kMember ? 1u : 0u;
                 records += __popc(part[x]);
@@ -1019,16 +1130,8 @@ __global__ void __launch_bounds__(kBigThreads)
         if (members) atomicAdd(&counters[2], static_cast<unsigned long long>(members));
         if (lane == 0) atomicAdd(&counters[4], static_cast<unsigned long long>(records));
         if (tid == 0) atomicAdd(&counters[3], static_cast<unsigned long long>(U));
-        ChainRow<D> row;
-        load_chain_row<D>(row, pts + static_cast<size_t>(p) * ld, lane & 7);
-        survivor_keys<D>(row, sm.cands, warp * 8, kWarps * 8, U, set_bound[p], pts, ld, keys, lane, [&](uint32_t count) {
-            uint32_t at = 0;
-            if (lane == 0) at = atomicAdd(&keys_s, count);
-            return __shfl_sync(kFull, at, 0);
-        });
-        __syncthreads();
-        const uint32_t S = keys_s, P2 = pow2_at_least(S);
-        for (uint32_t t = S + tid; t < P2; t += kBigThreads) keys[t] = ~0ull;
+        const uint32_t P2 = pow2_at_least(U);
+        for (uint32_t t = U + tid; t < P2; t += kBigThreads) sm.cands[t] = kNone;
         __syncthreads();
         for (uint32_t k = 2; k <= P2; k <<= 1) {
             for (uint32_t j = k >> 1; j > 0; j >>= 1) {
@@ -1036,24 +1139,39 @@ __global__ void __launch_bounds__(kBigThreads)
                     const uint32_t i = 2 * t - (t & (j - 1));  // 2 j (t / j) + t % j, j a power of two
                     const uint32_t partner = i + j;
                     const bool up = (i & k) == 0;
-                    const unsigned long long a = keys[i], b = keys[partner];
+                    const uint32_t a = sm.cands[i], b = sm.cands[partner];
                     if ((a > b) == up) {
-                        keys[i] = b;
-                        keys[partner] = a;
+                        sm.cands[i] = b;
+                        sm.cands[partner] = a;
                     }
                 }
                 __syncthreads();
             }
         }
+        // Every warp its share of the distances (the table's space takes them),
+        // then the first one makes the offers.
+        float* dists = reinterpret_cast<float*>(sm.table);
+        ChainRow<D> row;
+        load_chain_row<D>(row, pts + static_cast<size_t>(p) * ld, lane & 7);
+        for (uint32_t t0 = warp * kWarp; t0 < U; t0 += kBigThreads) {
+            const float d = warp_distances<D>(row, sm.cands[min(t0 + lane, U - 1)], pts, ld, lane);
+            if (t0 + lane < U) dists[t0 + lane] = d;
+        }
+        __syncthreads();
         if (warp == 0) {
             WarpSet s;
             set_load(s, set_dist, set_id, set_size, set_maxslot, set_bound, p, K, lane);
-            if (replay_keys(s, keys, S, K, lane)) {
+            uint32_t changed = 0;
+            for (uint32_t t0 = 0; t0 < U; t0 += kWarp) {
+                const uint32_t t = min(t0 + lane, U - 1);
+                changed += set_offer_new_batch(s, sm.cands[t], dists[t], t0 + lane < U, K, lane);
+            }
+            if (changed) {
                 set_store(s, set_dist, set_id, set_size, set_maxslot, set_bound, p, K, lane);
                 if (lane == 0) atomicAdd(changed_count, 1u);
             }
         }
-        __syncthreads();  // the keys are read before the next point's table
+        __syncthreads();  // the distances are read before the next point's table
     }
 }
 
@@ -1319,7 +1437,7 @@ uint64_t run_refine(Context& c) {
         KNNG_CUDA(cudaGetLastError());
         KNNG_CUDA(cudaEventRecord(ev[2], c.stream));
         KNNG_DISPATCH_D(c.d, {
-            k_apply<D><<<std::min<uint32_t>((n + kApplyWarps - 1) / kApplyWarps, 3 * sms), kApplyWarps * kWarp,
+            k_apply<D><<<std::min<uint32_t>((n + kApplyWarps - 1) / kApplyWarps, kApplyPerSm * sms), kApplyWarps * kWarp,
                          kApplyWarps * sizeof(ApplyWarpSmem), c.stream>>>(
                 snap, masks, c.points, c.ld, n, lo, hi, K, warp_cap, order, &counts->error, c.set_dist, c.set_id,
                 c.set_size, c.set_maxslot, c.set_bound, big, &counts->big, &counts->changed, counts->join);
