@@ -54,7 +54,7 @@ enum {
     KNNG_PRECISION_FP32 = 0,       /* exact FP32 distances everywhere (bit-exact form) */
     KNNG_PRECISION_BF16_RERANK = 1 /* bucket distances estimated in BF16 on the tensor cores (FP32
                                       accumulation, FP32 norms), each point's 128 best candidates
-                                      re-ranked with exact FP32 distances; buckets <= 512 points */
+                                      re-ranked with exact FP32 distances; buckets <= 1024 points */
 };
 
 /* Build parameters.  knng_default_params() fills the reference's values. */

@@ -175,6 +175,95 @@ __device__ __forceinline__ float canonical_distance4_lean(const float4* __restri
     return acc;
 }
 
+// ------------------------------------------------- distances by warp groups
+
+// A row as lane l of a group of eight holds it for the reference's distance
+// order: FMA chain l's dimensions l, l + 8, ..., and the tail.
+template <int D>
+struct ChainRow {
+    static constexpr int M = D / 8 * 8;
+    float c[M / 8];
+    float4 tail;
+};
+
+template <int D>
+__device__ __forceinline__ void load_chain_row(ChainRow<D>& r, const float* __restrict__ row, int l) {
+    constexpr int M = ChainRow<D>::M;
+#pragma unroll
+    for (int i = 0; i < M / 8; ++i) r.c[i] = __ldg(row + 8 * i + l);
+    r.tail = make_float4(0.f, 0.f, 0.f, 0.f);
+    if constexpr (D > M) r.tail = __ldg(reinterpret_cast<const float4*>(row + M));
+}
+
+// A load that stays where it is written (the compiler otherwise puts a row's
+// loads next to their uses, and each row waits for its own latency).
+__device__ __forceinline__ float load_now(const float* p) {
+    float v;
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+
+// canonical_distance of `mine` (p's row) and the rows of 32 points, lane t's
+// point id t; every lane returns its own.  A group of eight lanes reads its
+// eight rows one after the other, a lane a chain (32 bytes of each row a load);
+// the chains are then exchanged within the group, so that each lane sums the
+// eight of its own point and adds its tail.
+template <int D, int V>
+__device__ __forceinline__ float warp_distances(const ChainRow<D>& mine, uint32_t id, const float* __restrict__ pts,
+                                                int ld, int lane) {
+    constexpr int M = ChainRow<D>::M;
+    static_assert(D - M == 0 || D - M == 4, "tail of 0 or 4 dims");
+    const int l = lane & 7, g0 = lane & ~7;
+    float4 tail = make_float4(0.f, 0.f, 0.f, 0.f);
+    if constexpr (D > M) tail = __ldg(reinterpret_cast<const float4*>(pts + static_cast<size_t>(id) * ld + M));
+    // V rows' loads in flight, then their chains.
+    float x[8];
+#pragma unroll
+    for (int v0 = 0; v0 < 8; v0 += V) {
+        float y[V][M / 8];
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            const float* row = pts + static_cast<size_t>(__shfl_sync(kFull, id, g0 + v0 + v)) * ld + l;
+#pragma unroll
+            for (int i = 0; i < M / 8; ++i) y[v][i] = load_now(row + 8 * i);
+        }
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            float chain = 0.0f;
+#pragma unroll
+            for (int i = 0; i < M / 8; ++i) {
+                const float d = __fsub_rn(y[v][i], mine.c[i]);
+                chain = __fmaf_rn(d, d, chain);
+            }
+            x[v0 + v] = chain;
+        }
+    }
+#pragma unroll
+    for (int s = 1; s < 8; s <<= 1) {
+        const bool high = (l & s) != 0;
+#pragma unroll
+        for (int a = 0; a < 8; ++a) {
+            if (a & s) continue;
+            const float got = __shfl_xor_sync(kFull, high ? x[a] : x[a | s], s);
+            if (high) x[a] = got; else x[a | s] = got;
+        }
+    }
+    float acc = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc = __fadd_rn(acc, x[j]);
+    if constexpr (D > M) {
+        float d = __fsub_rn(tail.x, mine.tail.x);
+        acc = __fadd_rn(acc, __fmul_rn(d, d));
+        d = __fsub_rn(tail.y, mine.tail.y);
+        acc = __fadd_rn(acc, __fmul_rn(d, d));
+        d = __fsub_rn(tail.z, mine.tail.z);
+        acc = __fadd_rn(acc, __fmul_rn(d, d));
+        d = __fsub_rn(tail.w, mine.tail.w);
+        acc = __fadd_rn(acc, __fmul_rn(d, d));
+    }
+    return acc;
+}
+
 // ---------------------------------------------------------- neighbour sets
 //
 // Tie order of getMaxIdx: among slots holding the maximum distance, the one

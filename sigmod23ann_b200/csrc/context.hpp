@@ -252,8 +252,14 @@ void launch_leaves(Context& c, uint32_t count, const uint32_t* d_starts, const u
 size_t leaf_items_bytes(uint32_t n);
 void launch_leaves_list(Context& c, const uint32_t* d_starts, const uint32_t* d_ends, const uint32_t* d_count,
                         void* d_items, uint32_t* d_n_items, uint32_t* d_work, uint32_t max_bucket, uint32_t* d_error);
+// The work items of a bucket pass over [0, count) or [0, *dcount) buckets: row
+// blocks of `rows` rows in items[0 .. *n_items) (zeroed beforehand); returns the
+// inverse of the index permutation.
+uint32_t* launch_leaf_items(Context& c, uint32_t count, const uint32_t* d_starts, const uint32_t* d_ends,
+                            const uint32_t* dcount, uint32_t rows, uint2* items, uint32_t* n_items);
+// The precision form over a device list, with n floats for the rows' norms.
 void launch_leaves_bf16_list(Context& c, const uint32_t* d_starts, const uint32_t* d_ends, const uint32_t* d_count,
-                             uint32_t* d_work, uint32_t* d_error);
+                             void* d_items, uint32_t* d_n_items, uint32_t* d_work, float* d_norms, uint32_t* d_error);
 // Exact k nearest points (FP32 distances in the reference's order) of the
 // nq points d_queries, ids into d_truth (nq x k, kNone past the end).
 void sample_knn(Context& c, const uint32_t* d_queries, uint32_t nq, uint32_t* d_truth);

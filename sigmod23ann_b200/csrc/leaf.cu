@@ -785,6 +785,16 @@ double sample_recall(Context& c, const uint32_t* d_queries, uint32_t nq, const u
     return static_cast<double>(h) / (static_cast<double>(nq) * c.k);
 }
 
+uint32_t* launch_leaf_items(Context& c, uint32_t count, const uint32_t* d_starts, const uint32_t* d_ends,
+                            const uint32_t* dcount, uint32_t rows, uint2* items, uint32_t* n_items) {
+    uint32_t* pos = c.indices_tmp;  // the partition's second buffer is free during a bucket pass
+    k_leaf_items<<<std::min<uint32_t>((c.n + 255) / 256, 148 * 8), 256, 0, c.stream>>>(
+        d_starts, d_ends, count, dcount, rows, c.indices, c.n, pos, items, n_items);
+    ++c.launches;
+    KNNG_CUDA(cudaGetLastError());
+    return pos;
+}
+
 namespace {
 
 // Rows of a block of the FP32 pass: 32 (two a warp) once the points make a block
@@ -798,11 +808,7 @@ uint32_t leaf_rows(const Context& c) { return c.n >= 2u * c.sms * 2u * kLeafWarp
 void enqueue_leaves(Context& c, uint32_t count, const uint32_t* d_starts, const uint32_t* d_ends, const uint32_t* dcount,
                     uint2* items, uint32_t* n_items, uint32_t* work, uint32_t max_bucket) {
     const uint32_t rows = leaf_rows(c);
-    uint32_t* pos = c.indices_tmp;  // the partition's second buffer is free during the pass
-    k_leaf_items<<<std::min<uint32_t>((c.n + 255) / 256, 148 * 8), 256, 0, c.stream>>>(
-        d_starts, d_ends, count, dcount, rows, c.indices, c.n, pos, items, n_items);
-    ++c.launches;
-    KNNG_CUDA(cudaGetLastError());
+    uint32_t* pos = launch_leaf_items(c, count, d_starts, d_ends, dcount, rows, items, n_items);
     KNNG_DISPATCH_D(c.d, {
         const size_t smem = static_cast<size_t>(D) * (rows + kCols) * sizeof(float) +
                             static_cast<size_t>(rows) * kDmStride * sizeof(float) +

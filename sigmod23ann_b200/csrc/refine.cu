@@ -41,6 +41,7 @@
 #include "context.hpp"
 #include "dispatch.hpp"
 #include "tc.cuh"
+#include "tile16.cuh"
 
 namespace knng {
 namespace {
@@ -383,64 +384,12 @@ constexpr int kTile = 128;                        // MMA M: rows of R(q) per chu
 constexpr int kGroupCols = 64;                    // columns one thread filters (2 groups of 64)
 constexpr uint32_t kJoinBatch = 4;                // points a CTA takes from the work counter at a time
 
-// FP16 operand tiles, chunk-major: K padded to the MMA step of 16, a row held
-// as KP / 8 chunks of 16 bytes (8 halves), chunk c of row r at c * stride +
-// r * 16.  The stride is one row more than the tile has, so that the lanes of
-// a warp that hold consecutive pieces of one row write to different banks.
-template <int D>
-struct JoinTile {
-    static constexpr int KP = (D + 15) / 16 * 16;
-    static constexpr int CH = KP / 8;
-    static constexpr int Q = D / 4;       // 16-byte pieces of an FP32 row
-    static constexpr int R = kWarp / Q;   // rows a warp reads at once, a piece a lane
-    static constexpr uint32_t stride(uint32_t rows) { return rows * 16 + 16; }
-    static constexpr uint32_t bytes(uint32_t rows) { return CH * stride(rows); }
-};
-
 // Columns of the B tile: the MMA takes N in steps of 16.
 __host__ __device__ constexpr uint32_t join_cols(uint32_t K) { return K <= 16 ? 16u : (K + 15) / 16 * 16; }
 
 __host__ __device__ inline uint32_t join_smem(int D, uint32_t K) {
     const uint32_t chunks = (static_cast<uint32_t>(D) + 15) / 16 * 2;
     return chunks * (kTile * 16 + 16) + chunks * (join_cols(K) * 16 + 16);
-}
-
-// Rows i * kJoinWarps + warp (i < kTile / kJoinWarps, below `count`) of a tile:
-// the FP32 row of point id_i (held by lane i) minus `centre` (this lane's four
-// dimensions of it), rounded to FP16.  Consecutive lanes read consecutive
-// pieces of a row, eight loads in flight each.
-template <int D>
-__device__ __forceinline__ void tile_rows(const float* __restrict__ pts, int ld, uint32_t ids, uint32_t count,
-                                          unsigned char* __restrict__ tile, uint32_t stride, float4 centre, int lane,
-                                          int warp) {
-    using T = JoinTile<D>;
-    constexpr int N = kTile / kJoinWarps, U = 8;
-    const int piece = lane % T::Q, sub = lane / T::Q;
-    unsigned char* at = tile + (piece >> 1) * stride + (piece & 1) * 8;
-    const float* from = pts + 4 * piece;
-#pragma unroll
-    for (int j = 0; j < N / T::R; j += U) {
-        if (static_cast<uint32_t>(j * T::R * kJoinWarps + warp) >= count) break;  // warp-uniform
-        float4 x[U];
-        bool in[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int i = (j + u) * T::R + sub;
-            const uint32_t id = __shfl_sync(kFull, ids, i % kWarp);
-            in[u] = sub < T::R && static_cast<uint32_t>(i * kJoinWarps + warp) < count;
-            x[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (in[u]) x[u] = __ldg(reinterpret_cast<const float4*>(from + static_cast<size_t>(id) * ld));
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int i = (j + u) * T::R + sub;
-            const __half2 a = __floats2half2_rn(__fsub_rn(x[u].x, centre.x), __fsub_rn(x[u].y, centre.y));
-            const __half2 b = __floats2half2_rn(__fsub_rn(x[u].z, centre.z), __fsub_rn(x[u].w, centre.w));
-            if (in[u])
-                *reinterpret_cast<uint2*>(at + (i * kJoinWarps + warp) * 16) =
-                    make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
-        }
-    }
 }
 
 // The filter's error terms.  A pair is left out only when
@@ -493,7 +442,7 @@ __global__ void __launch_bounds__(kJoinThreads, kJoinPerSm)
            const float* __restrict__ pts, int ld, const float* __restrict__ bound, uint32_t K, uint32_t n, uint32_t lo,
            uint2* __restrict__ masks, uint32_t* __restrict__ error_flag, unsigned long long* __restrict__ counters,
            const uint32_t* __restrict__ order, uint32_t* __restrict__ work, const uint32_t* __restrict__ old_marks) {
-    using T = JoinTile<D>;
+    using T = Tile16<D>;
     extern __shared__ __align__(1024) unsigned char smem[];
     const uint32_t NB = join_cols(K);
     unsigned char* tile_a = smem;
@@ -557,10 +506,10 @@ __global__ void __launch_bounds__(kJoinThreads, kJoinPerSm)
                     na = snap_d[static_cast<size_t>(lo) * K + e];
                     bp = bound[lo + e / K];
                 }
-                tile_rows<D>(pts, ld, a_id, m, tile_a, T::stride(kTile), centre, lane, warp);
+                tile_rows<D, kTile, kJoinWarps, __half>(pts, ld, a_id, m, tile_a, T::stride(kTile), centre, lane, warp);
                 if (cb == rb) {  // uniform over the CTA
                     const uint32_t b_id = lane < kTile / kJoinWarps && mine < K ? snap[sq + mine] : 0u;
-                    tile_rows<D>(pts, ld, b_id, K, tile_b, T::stride(NB), centre, lane, warp);
+                    tile_rows<D, kTile, kJoinWarps, __half>(pts, ld, b_id, K, tile_b, T::stride(NB), centre, lane, warp);
                     if (warp < kOldWords) {
                         const uint32_t c = tid;  // column
                         const bool in = c < K;
@@ -704,24 +653,6 @@ __device__ __forceinline__ uint32_t table_insert(uint32_t* table, uint32_t bucke
     return 0u;
 }
 
-// A row as lane l of a group of eight holds it for the reference's distance
-// order: FMA chain l's dimensions l, l + 8, ..., and the tail.
-template <int D>
-struct ChainRow {
-    static constexpr int M = D / 8 * 8;
-    float c[M / 8];
-    float4 tail;
-};
-
-template <int D>
-__device__ __forceinline__ void load_chain_row(ChainRow<D>& r, const float* __restrict__ row, int l) {
-    constexpr int M = ChainRow<D>::M;
-#pragma unroll
-    for (int i = 0; i < M / 8; ++i) r.c[i] = __ldg(row + 8 * i + l);
-    r.tail = make_float4(0.f, 0.f, 0.f, 0.f);
-    if constexpr (D > M) r.tail = __ldg(reinterpret_cast<const float4*>(row + M));
-}
-
 // canonical_distance of two rows held by the eight lanes of the group whose
 // first lane is g0; every lane of the group returns it.  All 32 lanes call it.
 template <int D>
@@ -770,76 +701,6 @@ __global__ void __launch_bounds__(256)
             if (i < K && l == 0) snap_d[base + i] = d;
         }
     }
-}
-
-// A load that stays where it is written (the compiler otherwise puts a row's
-// loads next to their uses, and each row waits for its own latency).
-__device__ __forceinline__ float load_now(const float* p) {
-    float v;
-    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
-    return v;
-}
-
-// canonical_distance of `mine` (p's row) and the rows of 32 points, lane t's
-// point id t; every lane returns its own.  A group of eight lanes reads its
-// eight rows one after the other, a lane a chain (32 bytes of each row a load);
-// the chains are then exchanged within the group, so that each lane sums the
-// eight of its own point and adds its tail.
-template <int D>
-__device__ __forceinline__ float warp_distances(const ChainRow<D>& mine, uint32_t id, const float* __restrict__ pts,
-                                                int ld, int lane) {
-    constexpr int M = ChainRow<D>::M;
-    static_assert(D - M == 0 || D - M == 4, "tail of 0 or 4 dims");
-    const int l = lane & 7, g0 = lane & ~7;
-    float4 tail = make_float4(0.f, 0.f, 0.f, 0.f);
-    if constexpr (D > M) tail = __ldg(reinterpret_cast<const float4*>(pts + static_cast<size_t>(id) * ld + M));
-    // Four rows' loads in flight, then their chains.
-    float x[8];
-    constexpr int V = 4;
-#pragma unroll
-    for (int v0 = 0; v0 < 8; v0 += V) {
-        float y[V][M / 8];
-#pragma unroll
-        for (int v = 0; v < V; ++v) {
-            const float* row = pts + static_cast<size_t>(__shfl_sync(kFull, id, g0 + v0 + v)) * ld + l;
-#pragma unroll
-            for (int i = 0; i < M / 8; ++i) y[v][i] = load_now(row + 8 * i);
-        }
-#pragma unroll
-        for (int v = 0; v < V; ++v) {
-            float chain = 0.0f;
-#pragma unroll
-            for (int i = 0; i < M / 8; ++i) {
-                const float d = __fsub_rn(y[v][i], mine.c[i]);
-                chain = __fmaf_rn(d, d, chain);
-            }
-            x[v0 + v] = chain;
-        }
-    }
-#pragma unroll
-    for (int s = 1; s < 8; s <<= 1) {
-        const bool high = (l & s) != 0;
-#pragma unroll
-        for (int a = 0; a < 8; ++a) {
-            if (a & s) continue;
-            const float got = __shfl_xor_sync(kFull, high ? x[a] : x[a | s], s);
-            if (high) x[a] = got; else x[a | s] = got;
-        }
-    }
-    float acc = 0.0f;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc = __fadd_rn(acc, x[j]);
-    if constexpr (D > M) {
-        float d = __fsub_rn(tail.x, mine.tail.x);
-        acc = __fadd_rn(acc, __fmul_rn(d, d));
-        d = __fsub_rn(tail.y, mine.tail.y);
-        acc = __fadd_rn(acc, __fmul_rn(d, d));
-        d = __fsub_rn(tail.z, mine.tail.z);
-        acc = __fadd_rn(acc, __fmul_rn(d, d));
-        d = __fsub_rn(tail.w, mine.tail.w);
-        acc = __fadd_rn(acc, __fmul_rn(d, d));
-    }
-    return acc;
 }
 
 // Ascending sort of ids[0 .. U), U <= 32 E, by one warp: a bitonic network over
@@ -913,7 +774,7 @@ __device__ __forceinline__ uint32_t offer_sorted(WarpSet& s, const uint32_t* ids
     uint32_t changed = 0;
     for (uint32_t t0 = 0; t0 < U; t0 += kWarp) {
         const uint32_t id = ids[min(t0 + lane, U - 1)];
-        const float d = warp_distances<D>(mine, id, pts, ld, lane);
+        const float d = warp_distances<D, 4>(mine, id, pts, ld, lane);
         changed += set_offer_new_batch(s, id, d, t0 + lane < U, K, lane);
     }
     return changed;
@@ -1154,7 +1015,7 @@ __global__ void __launch_bounds__(kBigThreads)
         ChainRow<D> row;
         load_chain_row<D>(row, pts + static_cast<size_t>(p) * ld, lane & 7);
         for (uint32_t t0 = warp * kWarp; t0 < U; t0 += kBigThreads) {
-            const float d = warp_distances<D>(row, sm.cands[min(t0 + lane, U - 1)], pts, ld, lane);
+            const float d = warp_distances<D, 4>(row, sm.cands[min(t0 + lane, U - 1)], pts, ld, lane);
             if (t0 + lane < U) dists[t0 + lane] = d;
         }
         __syncthreads();
@@ -1182,7 +1043,7 @@ template <int D>
 __global__ void __launch_bounds__(kJoinThreads, 1)
     k_tile_gram(const float* __restrict__ a, uint32_t m, const float* __restrict__ b, uint32_t n,
                 float* __restrict__ out, uint32_t* __restrict__ error_flag) {
-    using T = JoinTile<D>;
+    using T = Tile16<D>;
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char* tile_a = smem;
     unsigned char* tile_b = smem + T::bytes(kTile);
@@ -1202,8 +1063,8 @@ __global__ void __launch_bounds__(kJoinThreads, 1)
     const uint32_t tmem = tmem_slot;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     const uint32_t id = lane < kTile / kJoinWarps ? lane * kJoinWarps + warp : 0u;
-    tile_rows<D>(a, D, id, m, tile_a, T::stride(kTile), zero, lane, warp);
-    tile_rows<D>(b, D, id, n, tile_b, T::stride(kTile), zero, lane, warp);
+    tile_rows<D, kTile, kJoinWarps, __half>(a, D, id, m, tile_a, T::stride(kTile), zero, lane, warp);
+    tile_rows<D, kTile, kJoinWarps, __half>(b, D, id, n, tile_b, T::stride(kTile), zero, lane, warp);
     tc::fence_proxy_async();
     tc::fence_before_sync();
     __syncthreads();

@@ -1357,7 +1357,9 @@ void enqueue_level(Context& c, DevRep& r, uint32_t lloyd_iters, cudaGraphConditi
 
 void enqueue_buckets(Context& c, DevRep& r, uint32_t max_leaf, uint32_t precision) {
     if (precision == KNNG_PRECISION_BF16_RERANK)
-        launch_leaves_bf16_list(c, r.leaf_start, r.leaf_end, &r.cnt->leaves, &r.cnt->leaf_work,
+        launch_leaves_bf16_list(c, r.leaf_start, r.leaf_end, &r.cnt->leaves, r.leaf_items, &r.cnt->leaf_items,
+                                &r.cnt->leaf_work,
+                                reinterpret_cast<float*>(r.lids),  // at least n entries, free once the tree is built
                                 reinterpret_cast<uint32_t*>(r.error + 1));
     else
         launch_leaves_list(c, r.leaf_start, r.leaf_end, &r.cnt->leaves, r.leaf_items, &r.cnt->leaf_items,
@@ -1497,10 +1499,10 @@ void run_rep_device(Context& c, uint32_t max_leaf, uint32_t lloyd_iters, uint32_
     }
     LevelCounts h{};
     download(c, &h, r.cnt, 1);
-    // Kernels the graph ran: prologue (2), every level, the bucket pass (with
-    // its items in the plain FP32 form).
-    const bool with_items = precision != KNNG_PRECISION_BF16_RERANK && !c.leaf_tc;
-    if (graph) c.launches += (with_items ? 4 : 3) + static_cast<uint64_t>(h.iterations) * (14 + 3 * lloyd_iters);
+    // Kernels the graph ran: prologue (2), every level, the bucket pass (items,
+    // and in the precision form norms, before the pass itself).
+    const uint32_t bucket_kernels = precision == KNNG_PRECISION_BF16_RERANK ? 3 : c.leaf_tc ? 1 : 2;
+    if (graph) c.launches += 2 + bucket_kernels + static_cast<uint64_t>(h.iterations) * (14 + 3 * lloyd_iters);
     int32_t err[4] = {0, 0, 0, 0};
     download(c, err, r.error, 4);
     if (err[0]) fail(KNNG_ERR_CUDA, "Lloyd sums: a bulk-copy wait gave up");

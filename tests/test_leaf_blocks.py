@@ -66,3 +66,25 @@ def test_many_buckets_in_blocks_of_32_rows(knng_lib, oracle_lib):
         assert np.array_equal(got["dist"][ids].view(np.uint32), o["dist"].view(np.uint32)), (s, e)
         filled = np.arange(k)[None] < size[:, None]
         assert np.array_equal(got["id"][ids][filled], ids[o["id"]][filled])
+
+
+@pytest.mark.parametrize("n", [2, 33, 129, 130, 131, 160, 256, 257, 300, 1000])
+@pytest.mark.parametrize("d", [64, 100, 128])
+def test_precision_form_keeps_the_128_best(knng_lib, n, d):
+    """Points with small integer coordinates: the BF16 estimates are the exact
+    distances, with many ties, so the kept candidates of a bucket are the 128
+    smallest by (distance, position) and lists of 128 hold just them."""
+    from sigmod23ann_b200 import default_params
+
+    rng = np.random.default_rng(n + d)
+    pts = np.zeros((n, d), np.float32)
+    pts[:, :6] = rng.integers(-2, 3, (n, 6))
+    dist = ((pts[:, None].astype(np.int64) - pts[None].astype(np.int64)) ** 2).sum(-1)
+    key = dist * n + np.arange(n)[None]
+    np.fill_diagonal(key, np.iinfo(np.int64).max)
+    best = np.sort(key, axis=1)[:, :min(128, n - 1)]
+    want = np.ones((n, 128), np.uint32)
+    want[:, :best.shape[1]] = best % n  # ascending by (distance, id)
+    with KnngContext(0) as c:
+        got = c.build(pts, default_params(k=128, reps=1, refine=0, max_leaf=1025, max_leaf_odd=0, precision=1))
+    assert np.array_equal(got, want)
