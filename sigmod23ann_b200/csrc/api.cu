@@ -15,12 +15,15 @@
 #include <chrono>
 #include <cfloat>
 #include <cmath>
+#include <condition_variable>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <numeric>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "common.cuh"
@@ -97,14 +100,68 @@ uint32_t sample_count(uint32_t n) {
 // kmeansStartVecs' seed count: (uint32)(log10 n)^2.5 (src/SolutionKmeans.hpp:70, :105).
 uint32_t start_count(uint32_t n) { return static_cast<uint32_t>(std::pow(std::log10(static_cast<double>(n)), 2.5)); }
 
+// Pinned blocks between contexts: pinning a megabyte takes about 0.4 ms, which
+// every context (every served job) would pay anew.  Blocks a context gives back
+// are kept for the next one, at most kPinnedKept of them, while some context or
+// server is alive; the last one to go frees them.
+namespace {
+constexpr size_t kPinnedKept = 24;
+std::mutex g_pinned_mutex;
+size_t g_pinned_holders = 0;
+std::vector<std::pair<size_t, void*>> g_pinned_free;
+}  // namespace
+
+void pinned_hold() {
+    std::lock_guard<std::mutex> lk(g_pinned_mutex);
+    ++g_pinned_holders;
+}
+
+void pinned_drop() {
+    std::lock_guard<std::mutex> lk(g_pinned_mutex);
+    if (--g_pinned_holders > 0) return;
+    for (auto& b : g_pinned_free) cudaFreeHost(b.second);
+    g_pinned_free.clear();
+}
+
+void* pinned_take(size_t bytes) {
+    {
+        std::lock_guard<std::mutex> lk(g_pinned_mutex);
+        for (size_t i = 0; i < g_pinned_free.size(); ++i) {
+            if (g_pinned_free[i].first != bytes) continue;
+            void* p = g_pinned_free[i].second;
+            g_pinned_free[i] = g_pinned_free.back();
+            g_pinned_free.pop_back();
+            return p;
+        }
+    }
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, bytes, cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return p;
+}
+
+void pinned_give(void* p, size_t bytes) {
+    if (!p) return;
+    {
+        std::lock_guard<std::mutex> lk(g_pinned_mutex);
+        if (g_pinned_holders > 0 && g_pinned_free.size() < kPinnedKept) {
+            g_pinned_free.emplace_back(bytes, p);
+            return;
+        }
+    }
+    cudaFreeHost(p);
+}
+
 void* staging_take(Context& c, size_t bytes) {
     bytes = (bytes + 15) / 16 * 16;
     if (bytes > c.staging_cap) {
         KNNG_CUDA(cudaStreamSynchronize(c.stream));
         staging_free(c);
-        const size_t cap = std::max<size_t>(bytes, 4u << 20);
-        void* p = nullptr;
-        check_cuda(cudaMallocHost(&p, cap), "cudaMallocHost");
+        const size_t cap = std::max<size_t>(bytes, 2u << 20);
+        void* p = pinned_take(cap);
+        if (!p) fail(KNNG_ERR_OUT_OF_MEMORY, "no pinned host memory");
         c.staging = static_cast<unsigned char*>(p);
         c.staging_cap = cap;
         c.staging_used = 0;
@@ -119,8 +176,111 @@ void* staging_take(Context& c, size_t bytes) {
     return p;
 }
 
+// Results go to whatever memory the caller has.  Pageable memory of a fresh
+// array is the slow kind: the driver copies it through its own buffers on one
+// thread, which also takes the page faults (240 MB in 50 ms).  Here the pieces
+// land in pinned blocks and several threads carry them on, faults included (240
+// MB in 11 ms); the threads end with the call.
+constexpr size_t kLandingBlock = 1u << 20;
+constexpr size_t kLandingBlocks = 16;
+constexpr size_t kLandingMin = 2u << 20;  // below, the threads cost more than they save
+
+void download_large(Context& c, void* host, const void* dev, size_t bytes) {
+    cudaPointerAttributes attr{};
+    const bool pageable = cudaPointerGetAttributes(&attr, host) == cudaSuccess && attr.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    const unsigned cores = std::thread::hardware_concurrency();
+    const size_t pieces = (bytes + kLandingBlock - 1) / kLandingBlock;
+    const unsigned workers = static_cast<unsigned>(std::min<size_t>({8u, cores / 2, pieces}));
+    if (!pageable || bytes < kLandingMin || workers < 2) {
+        KNNG_CUDA(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, c.stream));
+        return;
+    }
+    if (!c.landing) {
+        void* p = pinned_take(kLandingBlock * kLandingBlocks);
+        if (!p) {
+            KNNG_CUDA(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, c.stream));
+            return;
+        }
+        c.landing = static_cast<unsigned char*>(p);
+    }
+    while (c.landing_ev.size() < kLandingBlocks) {
+        cudaEvent_t e = nullptr;
+        KNNG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        c.landing_ev.push_back(e);
+    }
+    // Piece i passes through block i % kLandingBlocks.  `issued` pieces are on
+    // the stream; a block is free again once its piece has been carried on.
+    std::mutex mu;
+    std::condition_variable cv;
+    size_t issued = 0, taken = 0;
+    std::vector<bool> carried(pieces, false);
+    bool stop = false;
+    cudaError_t error = cudaSuccess;
+    auto work = [&] {
+        cudaSetDevice(c.device);
+        std::unique_lock<std::mutex> lk(mu);
+        for (;;) {
+            cv.wait(lk, [&] { return stop || taken < issued || taken == pieces; });
+            if (stop || taken == pieces) return;
+            const size_t i = taken++;
+            lk.unlock();
+            const size_t block = i % kLandingBlocks, at = i * kLandingBlock;
+            const cudaError_t e = cudaEventSynchronize(c.landing_ev[block]);
+            if (e == cudaSuccess)
+                std::memcpy(static_cast<unsigned char*>(host) + at, c.landing + block * kLandingBlock,
+                            std::min(kLandingBlock, bytes - at));
+            lk.lock();
+            if (e != cudaSuccess) {
+                error = e;
+                stop = true;
+            }
+            carried[i] = true;
+            cv.notify_all();
+        }
+    };
+    std::vector<std::thread> pool;
+    try {
+        for (unsigned t = 0; t < workers; ++t) pool.emplace_back(work);
+    } catch (...) {  // fewer threads than asked for; none: the plain copy
+    }
+    if (pool.empty()) {
+        KNNG_CUDA(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, c.stream));
+        return;
+    }
+    for (size_t i = 0; i < pieces; ++i) {
+        const size_t block = i % kLandingBlocks, at = i * kLandingBlock;
+        {
+            std::unique_lock<std::mutex> lk(mu);
+            cv.wait(lk, [&] { return stop || i < kLandingBlocks || carried[i - kLandingBlocks]; });
+            if (stop) break;
+        }
+        cudaError_t e = cudaMemcpyAsync(c.landing + block * kLandingBlock, static_cast<const unsigned char*>(dev) + at,
+                                        std::min(kLandingBlock, bytes - at), cudaMemcpyDeviceToHost, c.stream);
+        if (e == cudaSuccess) e = cudaEventRecord(c.landing_ev[block], c.stream);
+        std::lock_guard<std::mutex> lk(mu);
+        if (e != cudaSuccess) {
+            error = e;
+            stop = true;
+        } else {
+            issued = i + 1;
+        }
+        cv.notify_all();
+        if (stop) break;
+    }
+    for (auto& t : pool) t.join();
+    check_cuda(error, "copy of results to the host");
+}
+
+void landing_free(Context& c) {
+    pinned_give(c.landing, kLandingBlock * kLandingBlocks);
+    c.landing = nullptr;
+    for (auto& e : c.landing_ev) cudaEventDestroy(e);
+    c.landing_ev.clear();
+}
+
 void staging_free(Context& c) {
-    if (c.staging) cudaFreeHost(c.staging);
+    pinned_give(c.staging, c.staging_cap);
     c.staging = nullptr;
     c.staging_cap = c.staging_used = 0;
 }
@@ -690,9 +850,12 @@ knng_status knng_create(int device, uint64_t hbm_budget_bytes, knng_context** ou
         return KNNG_ERR_NO_DEVICE;
     }
     if (device < 0 || device >= count) return KNNG_ERR_INVALID_ARGUMENT;
-    cudaDeviceProp prop;
-    if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) return KNNG_ERR_CUDA;
-    if (prop.major != 10) return KNNG_ERR_NO_DEVICE;
+    // The two properties needed, not all of them: that query takes 2.5 ms, which
+    // every served job would pay.
+    int major = 0, sms = 0;
+    if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device) != cudaSuccess) return KNNG_ERR_CUDA;
+    if (major != 10) return KNNG_ERR_NO_DEVICE;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return KNNG_ERR_CUDA;
     if (cudaSetDevice(device) != cudaSuccess) return KNNG_ERR_CUDA;
     auto* c = new (std::nothrow) Context();
     if (!c) return KNNG_ERR_OUT_OF_MEMORY;
@@ -704,31 +867,32 @@ knng_status knng_create(int device, uint64_t hbm_budget_bytes, knng_context** ou
     if (const char* r = std::getenv("KNNG_REFINE_SKIP")) c->refine_skip_old = std::strcmp(r, "0") != 0;
     if (const char* r = std::getenv("KNNG_REP_LOOP"))
         c->rep_loop = std::strcmp(r, "host") == 0 ? 2 : (std::strcmp(r, "device") == 0 ? 1 : 0);
-    c->sms = prop.multiProcessorCount;
+    c->sms = sms;
     if (const char* r = std::getenv("KNNG_REFINE_POOL")) c->refine_pool = std::max<long long>(0, std::atoll(r));
     if (hbm_budget_bytes) {
         c->budget = hbm_budget_bytes;
     } else {
-        // 90% of the device, but no more than what is free now (less 1 GiB):
-        // memory other users of the device hold is not this context's.
-        c->budget = static_cast<uint64_t>(prop.totalGlobalMem * 0.9);
         // Memory freed to the device's stream-ordered pool (by contexts
         // destroyed earlier) counts as free: return what the pool keeps unused.
         cudaMemPool_t pool = nullptr;
         if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
         cudaGetLastError();
+        // 90% of the device, but no more than what is free now (less 1 GiB):
+        // memory other users of the device hold is not this context's.
         size_t free_b = 0, total_b = 0;
-        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
-            const uint64_t room = free_b > (1ull << 30) ? free_b - (1ull << 30) : 0;
-            c->budget = std::min<uint64_t>(c->budget, room);
-        } else {
+        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
             cudaGetLastError();
+            delete c;
+            return KNNG_ERR_CUDA;
         }
+        const uint64_t room = free_b > (1ull << 30) ? free_b - (1ull << 30) : 0;
+        c->budget = std::min<uint64_t>(static_cast<uint64_t>(total_b * 0.9), room);
     }
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) {
         delete c;
         return KNNG_ERR_CUDA;
     }
+    knng::pinned_hold();
     *out = reinterpret_cast<knng_context*>(c);
     return KNNG_OK;
 }
@@ -739,6 +903,8 @@ knng_status knng_destroy(knng_context* ctx) {
     cudaSetDevice(c->device);
     knng::release_all(*c);
     knng::staging_free(*c);
+    knng::landing_free(*c);
+    knng::pinned_drop();
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
     return KNNG_OK;

@@ -88,6 +88,10 @@ struct Context {
     // after the next synchronisation of the stream.
     unsigned char* staging = nullptr;
     size_t staging_cap = 0, staging_used = 0;
+    // Pinned blocks that large results pass through on their way to pageable
+    // memory, and an event each (download_large).
+    unsigned char* landing = nullptr;
+    std::vector<cudaEvent_t> landing_ev;
 
     // Neighbour-of-neighbour pass: 0 = local join on the tensor cores,
     // 1 = one warp per point (environment KNNG_REFINE=pointwise at creation).
@@ -135,12 +139,20 @@ void* scratch(Context& c, const char* name, size_t bytes);
 size_t scratch_bytes(const Context& c, const char* name);
 void release_all(Context& c);
 
+// Pinned host blocks kept between contexts: taken and given back by size (null:
+// none to be had); whoever may use them holds the store from creation to end.
+void pinned_hold();
+void pinned_drop();
+void* pinned_take(size_t bytes);
+void pinned_give(void* p, size_t bytes);
+
 // Transfers up to this size go through the pinned staging space.
 constexpr size_t kStagedMax = 1u << 20;
 // `bytes` of pinned staging space (synchronises the stream and starts over
 // when the space is used up; grows it when one transfer needs more).
 void* staging_take(Context& c, size_t bytes);
 void staging_free(Context& c);
+void landing_free(Context& c);
 
 // Uploads `count` elements into named scratch and returns the device pointer.
 template <class T>
@@ -158,6 +170,9 @@ T* upload(Context& c, const char* name, const T* host, size_t count) {
     return d;
 }
 
+// A copy to host memory of any kind and size, complete on return.
+void download_large(Context& c, void* host, const void* dev, size_t bytes);
+
 template <class T>
 void download(Context& c, T* host, const T* dev, size_t count) {
     const size_t bytes = count * sizeof(T);
@@ -167,7 +182,7 @@ void download(Context& c, T* host, const T* dev, size_t count) {
         KNNG_CUDA(cudaStreamSynchronize(c.stream));
         std::memcpy(host, p, bytes);
     } else {
-        if (bytes) KNNG_CUDA(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, c.stream));
+        if (bytes) download_large(c, host, dev, bytes);
         KNNG_CUDA(cudaStreamSynchronize(c.stream));
     }
     c.staging_used = 0;  // every earlier copy through the staging space has completed

@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "admission.hpp"
+#include "context.hpp"
 #include "knng.h"
 
 namespace {
@@ -166,14 +167,19 @@ knng_status knng_server_create(int device, uint64_t hbm_budget_bytes, uint32_t m
         return KNNG_ERR_NO_DEVICE;
     }
     if (device < 0 || device >= count) return KNNG_ERR_INVALID_ARGUMENT;
-    cudaDeviceProp prop;
-    if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) return KNNG_ERR_CUDA;
-    if (prop.major != 10) return KNNG_ERR_NO_DEVICE;
+    int major = 0;
+    if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device) != cudaSuccess) return KNNG_ERR_CUDA;
+    if (major != 10) return KNNG_ERR_NO_DEVICE;
     if (cudaSetDevice(device) != cudaSuccess) return KNNG_ERR_CUDA;
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+        cudaGetLastError();
+        return KNNG_ERR_CUDA;
+    }
     auto* s = new (std::nothrow) knng_server();
     if (!s) return KNNG_ERR_OUT_OF_MEMORY;
     s->device = device;
-    s->budget = hbm_budget_bytes ? hbm_budget_bytes : static_cast<uint64_t>(prop.totalGlobalMem * 0.8);
+    s->budget = hbm_budget_bytes ? hbm_budget_bytes : static_cast<uint64_t>(total_b * 0.8);
     s->max_running = max_running;
     // Jobs allocate and free stream-ordered memory from the device's default
     // pool: keep up to the budget cached there between jobs instead of
@@ -183,6 +189,7 @@ knng_status knng_server_create(int device, uint64_t hbm_budget_bytes, uint32_t m
         uint64_t keep = s->budget;
         cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
     }
+    knng::pinned_hold();  // the jobs' pinned blocks stay for the next jobs
     try {
         for (uint32_t i = 0; i < max_running; ++i) s->workers.emplace_back(worker_loop, s);
     } catch (...) {
@@ -192,6 +199,7 @@ knng_status knng_server_create(int device, uint64_t hbm_budget_bytes, uint32_t m
         }
         s->cv_work.notify_all();
         for (auto& t : s->workers) t.join();
+        knng::pinned_drop();
         delete s;
         return KNNG_ERR_OUT_OF_MEMORY;
     }
@@ -294,6 +302,7 @@ knng_status knng_server_destroy(knng_server* s) {
         cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
         cudaMemPoolTrimTo(pool, 0);
     }
+    knng::pinned_drop();
     delete s;
     return KNNG_OK;
 }

@@ -1222,9 +1222,8 @@ DevRep& ensure_devrep(Context& c, uint32_t max_leaf, uint32_t small_threshold) {
     if (!c.devrep) {
         c.devrep = new DevRep();
         for (auto& e : c.devrep->ev) KNNG_CUDA(cudaEventCreate(&e));
-        void* p = nullptr;
-        KNNG_CUDA(cudaMallocHost(&p, 4 * sizeof(uint64_t)));
-        c.devrep->h_params = static_cast<uint64_t*>(p);
+        c.devrep->h_params = static_cast<uint64_t*>(pinned_take(4 * sizeof(uint64_t)));
+        if (!c.devrep->h_params) fail(KNNG_ERR_OUT_OF_MEMORY, "no pinned host memory");
     }
     DevRep& r = *c.devrep;
     const bool same = r.n == c.n && r.h_set_offsets == c.set_offsets && r.min_leaf <= max_leaf &&
@@ -1467,7 +1466,7 @@ void devrep_release(Context& c) {
     release_buffers(c, *c.devrep);
     for (auto& e : c.devrep->ev)
         if (e) cudaEventDestroy(e);
-    if (c.devrep->h_params) cudaFreeHost(c.devrep->h_params);
+    pinned_give(c.devrep->h_params, 4 * sizeof(uint64_t));
     delete c.devrep;
     c.devrep = nullptr;
 }
