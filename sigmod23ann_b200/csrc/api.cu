@@ -694,8 +694,8 @@ void validate_params(const knng_params* p) {
 // has passed since the call began (at least one, at most p->reps when it is
 // non-zero), then whole refinement passes start while less than
 // build_ms + refine_ms has passed (at most p->refine).
-void build_all(Context& c, const knng_params* p, knng_stats* stats, uint64_t build_ms = 0, uint64_t refine_ms = 0) {
-    const auto t0 = std::chrono::steady_clock::now();
+void build_all(Context& c, const knng_params* p, knng_stats* stats, uint64_t build_ms = 0, uint64_t refine_ms = 0,
+               std::chrono::steady_clock::time_point t0 = {}) {
     auto elapsed_ms = [&] {
         KNNG_CUDA(cudaStreamSynchronize(c.stream));
         return static_cast<uint64_t>(
@@ -1407,9 +1407,10 @@ knng_status knng_build_timed(knng_context* ctx, const float* points, uint32_t n,
         knng::validate_params(params);
         if (!out_ids) knng::fail(KNNG_ERR_INVALID_ARGUMENT, "null output");
         if (build_ms == 0) knng::fail(KNNG_ERR_INVALID_ARGUMENT, "build_ms must be positive");
+        const auto t0 = std::chrono::steady_clock::now();  // the points' upload counts too
         if (stats) std::memset(stats, 0, sizeof(*stats));
         knng::load_points(c, points, n, d, ld_bytes, false, false);
-        knng::build_all(c, params, stats, build_ms, refine_ms);
+        knng::build_all(c, params, stats, build_ms, refine_ms, t0);
         const size_t nk = static_cast<size_t>(c.n) * c.k;
         knng::EventPair ft(c);
         uint32_t* d_ids = static_cast<uint32_t*>(knng::scratch(c, "fin_ids", nk * sizeof(uint32_t)));
