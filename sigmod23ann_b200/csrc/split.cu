@@ -134,15 +134,22 @@ __global__ void k_farthest_pair(const uint64_t* __restrict__ offsets, const uint
     __syncthreads();
     float best = FLT_MIN;
     uint32_t bi = kNone, bj = kNone;
-    for (uint32_t i = 0; i + 1 < m; ++i) {
-        for (uint32_t j = i + 1 + threadIdx.x; j < m; j += blockDim.x) {
-            const float dd = canonical_distance<D>(rows + i * Q * 4, rows + j * Q * 4);
-            // Within one thread pairs arrive in increasing (i, j) order.
-            if (dd > best) {
-                best = dd;
-                bi = i;
-                bj = j;
-            }
+    // The pairs in (i, j) order, a CTA's threads taking consecutive ones: with a
+    // row i at a time each of the m - 1 rows was one step's latency, most
+    // threads idle (21 us a launch at 100k points, now 6).
+    for (uint32_t i = 0, j = 1 + threadIdx.x;; j += blockDim.x) {
+        while (i + 1 < m && j >= m) {
+            ++i;
+            j = j - m + i + 1;
+        }
+        if (i + 1 >= m) break;
+        const float dd = canonical_distance4<D>(reinterpret_cast<const float4*>(rows) + i * Q,
+                                                reinterpret_cast<const float4*>(rows) + j * Q);
+        // Within one thread pairs arrive in increasing (i, j) order.
+        if (dd > best) {
+            best = dd;
+            bi = i;
+            bj = j;
         }
     }
     // Block arg-max: larger distance wins; equal distances -> smaller (i, j).
@@ -197,8 +204,7 @@ __global__ void k_farthest_pair(const uint64_t* __restrict__ offsets, const uint
 // between = 0.5f * (c1 + c2); coefs = c1 - between; offset = dot(between, coefs).
 template <int D>
 __global__ void k_plane(const float* __restrict__ c1, const float* __restrict__ c2, int ld, uint32_t count,
-                        float* __restrict__ coefs, float* __restrict__ offsets, const uint32_t* __restrict__ dcount) {
-    if (dcount) count = *dcount;
+                        float* __restrict__ coefs, float* __restrict__ offsets) {
     const int lane = threadIdx.x % kWarp;
     __shared__ float between_s[8][(D + 3) / 4 * 4];
     float* between = between_s[threadIdx.x / kWarp];
@@ -246,6 +252,43 @@ __device__ __forceinline__ void load_chain_plane(ChainPlane<D>& p, const float* 
     if constexpr (D > M) p.tail = *reinterpret_cast<const float4*>(coefs_row + M);
 }
 
+// The same from a node's two centres (between = 0.5 (c1 + c2), coefs = c1 -
+// between, offset = dot(between, coefs), src/SolutionKmeans.hpp:162-164, as
+// k_plane rounds them); returns the offset.  All 32 lanes call it.
+template <int D>
+__device__ __forceinline__ float load_centre_plane(ChainPlane<D>& p, const float* __restrict__ c1_row,
+                                                   const float* __restrict__ c2_row, int l, int g0) {
+    constexpr int M = ChainPlane<D>::M;
+    float chain = 0.0f;
+#pragma unroll
+    for (int i = 0; i < M / 8; ++i) {
+        const float a = c1_row[8 * i + l];
+        const float between = __fmul_rn(0.5f, __fadd_rn(a, c2_row[8 * i + l]));
+        p.c[i] = __fsub_rn(a, between);
+        chain = __fmaf_rn(p.c[i], between, chain);
+    }
+    float acc = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc = __fadd_rn(acc, __shfl_sync(kFull, chain, g0 + j));
+    p.tail = make_float4(0.f, 0.f, 0.f, 0.f);
+    if constexpr (D > M) {
+        const float4 a = *reinterpret_cast<const float4*>(c1_row + M), b = *reinterpret_cast<const float4*>(c2_row + M);
+        float between = __fmul_rn(0.5f, __fadd_rn(a.x, b.x));
+        p.tail.x = __fsub_rn(a.x, between);
+        acc = __fadd_rn(acc, __fmul_rn(between, p.tail.x));
+        between = __fmul_rn(0.5f, __fadd_rn(a.y, b.y));
+        p.tail.y = __fsub_rn(a.y, between);
+        acc = __fadd_rn(acc, __fmul_rn(between, p.tail.y));
+        between = __fmul_rn(0.5f, __fadd_rn(a.z, b.z));
+        p.tail.z = __fsub_rn(a.z, between);
+        acc = __fadd_rn(acc, __fmul_rn(between, p.tail.z));
+        between = __fmul_rn(0.5f, __fadd_rn(a.w, b.w));
+        p.tail.w = __fsub_rn(a.w, between);
+        acc = __fadd_rn(acc, __fmul_rn(between, p.tail.w));
+    }
+    return acc;
+}
+
 // dot(coefs, row) in the reference's order, by the eight lanes of the group
 // whose first lane is `g0`; every lane of the group returns the result.  All
 // 32 lanes must call it together.
@@ -282,11 +325,15 @@ __device__ __forceinline__ float group_dot(const ChainPlane<D>& p, const float* 
 // a CTA per 2,048-entry item left a 100k x 100 level to 49 CTAs that walked
 // 64 units' latency each in turn (42 us a launch, now 9).  Units go to warps
 // unit-major, so that the empty ones of short items fall together at the end.
-template <int D>
+//
+// The hyperplanes are `plane_of` (rows of coefficients) and `plane2` (offsets), or
+// with kCentres the nodes' two centres, each warp making its node's plane: some
+// 60 instructions a unit in place of a launch.
+template <int D, bool kCentres>
 __global__ void __launch_bounds__(kSideThreads) k_side(const Item* __restrict__ items, const uint32_t* __restrict__ list,
                                                        const uint32_t* __restrict__ idx, const float* __restrict__ pts,
-                                                       int ld, const float* __restrict__ coefs,
-                                                       const float* __restrict__ offsets, uint8_t* __restrict__ flags,
+                                                       int ld, const float* __restrict__ plane_of,
+                                                       const float* __restrict__ plane2, uint8_t* __restrict__ flags,
                                                        uint32_t* __restrict__ ids_out,
                                                        uint32_t* __restrict__ item_true, uint32_t n_items,
                                                        const uint32_t* __restrict__ dcount) {
@@ -309,8 +356,14 @@ __global__ void __launch_bounds__(kSideThreads) k_side(const Item* __restrict__ 
             id = idx[from_list ? list[e] : static_cast<uint32_t>(e)];
         }
         ChainPlane<D> plane;
-        load_chain_plane<D>(plane, coefs + static_cast<size_t>(node) * ld, l);
-        const float off = offsets[node];
+        float off;
+        if constexpr (kCentres) {
+            off = load_centre_plane<D>(plane, plane_of + static_cast<size_t>(node) * ld,
+                                       plane2 + static_cast<size_t>(node) * ld, l, g0);
+        } else {
+            load_chain_plane<D>(plane, plane_of + static_cast<size_t>(node) * ld, l);
+            off = plane2[node];
+        }
         uint32_t mask = 0;  // bit j: entry r0 + j is side-true
 #pragma unroll 4
         for (int b = 0; b < 8; ++b) {
@@ -568,28 +621,50 @@ __global__ void __launch_bounds__(kSeqThreads)
     }
 }
 
+constexpr uint32_t kPlanThreads = 1024;
+
+// Exclusive prefix sum of one value per thread over a CTA of kPlanThreads;
+// *total receives the sum.  Every thread calls it.
+__device__ __forceinline__ unsigned long long plan_scan(unsigned long long v, unsigned long long* __restrict__ wt,
+                                                        unsigned long long* total) {
+    const int lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
+    unsigned long long incl = v;
+#pragma unroll
+    for (int o = 1; o < kWarp; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == kWarp - 1) wt[warp] = incl;
+    __syncthreads();
+    if (warp == 0) {
+        unsigned long long t = wt[lane];
+#pragma unroll
+        for (int o = 1; o < kWarp; o <<= 1) {
+            const unsigned long long y = __shfl_up_sync(kFull, t, o);
+            if (lane >= o) t += y;
+        }
+        wt[lane] = t;
+    }
+    __syncthreads();
+    const unsigned long long base = warp > 0 ? wt[warp - 1] : 0ull;
+    *total = wt[kWarp - 1];
+    __syncthreads();
+    return base + incl - v;
+}
+
 // Exclusive scan of n values into out[0..n] (out[n] = total); one CTA.
-__global__ void k_scan_items(const uint32_t* __restrict__ in, uint32_t n, uint32_t* __restrict__ out,
-                             const uint32_t* __restrict__ dn) {
-    __shared__ uint32_t part[1024];
+__global__ void __launch_bounds__(kPlanThreads) k_scan_items(const uint32_t* __restrict__ in, uint32_t n,
+                                                             uint32_t* __restrict__ out,
+                                                             const uint32_t* __restrict__ dn) {
+    __shared__ unsigned long long wt[kWarp];
     if (dn) n = *dn;
     const uint32_t per = (n + blockDim.x - 1) / blockDim.x;
     const uint32_t b = threadIdx.x * per, e = min(n, b + per);
     uint32_t s = 0;
     for (uint32_t i = b; i < e; ++i) s += in[i];
-    part[threadIdx.x] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t run = 0;
-        for (uint32_t w = 0; w < blockDim.x; ++w) {
-            const uint32_t v = part[w];
-            part[w] = run;
-            run += v;
-        }
-        out[n] = run;
-    }
-    __syncthreads();
-    uint32_t run = part[threadIdx.x];
+    unsigned long long total;
+    uint32_t run = static_cast<uint32_t>(plan_scan(s, wt, &total));
+    if (threadIdx.x == 0) out[n] = static_cast<uint32_t>(total);
     for (uint32_t i = b; i < e; ++i) {
         out[i] = run;
         run += in[i];
@@ -597,9 +672,7 @@ __global__ void k_scan_items(const uint32_t* __restrict__ in, uint32_t n, uint32
 }
 
 __global__ void k_node_true(const uint32_t* __restrict__ item_begin, const uint32_t* __restrict__ item_end,
-                            const uint32_t* __restrict__ prefix, uint32_t count, uint32_t* __restrict__ out_true,
-                            const uint32_t* __restrict__ dcount) {
-    if (dcount) count = *dcount;
+                            const uint32_t* __restrict__ prefix, uint32_t count, uint32_t* __restrict__ out_true) {
     for (uint32_t node = blockIdx.x * blockDim.x + threadIdx.x; node < count; node += gridDim.x * blockDim.x)
         out_true[node] = prefix[item_end[node]] - prefix[item_begin[node]];
 }
@@ -609,7 +682,7 @@ __global__ void k_node_true(const uint32_t* __restrict__ item_begin, const uint3
 __global__ void __launch_bounds__(kSideThreads) k_scatter(const Item* __restrict__ items,
                                                           const uint32_t* __restrict__ node_start,
                                                           const uint32_t* __restrict__ node_item_begin,
-                                                          const uint32_t* __restrict__ node_true,
+                                                          const uint32_t* __restrict__ node_item_end,
                                                           const uint32_t* __restrict__ prefix,
                                                           const uint8_t* __restrict__ flags,
                                                           const uint32_t* __restrict__ idx,
@@ -620,8 +693,9 @@ __global__ void __launch_bounds__(kSideThreads) k_scatter(const Item* __restrict
     for (uint32_t item = blockIdx.x; item < n_items; item += gridDim.x) {
     const Item it = items[item];
     const uint32_t s = node_start[it.node];
-    const uint32_t T = node_true[it.node];
-    const uint32_t before_item = prefix[item] - prefix[node_item_begin[it.node]];
+    const uint32_t first_item = prefix[node_item_begin[it.node]];
+    const uint32_t T = prefix[node_item_end[it.node]] - first_item;  // the node's side-true positions
+    const uint32_t before_item = prefix[item] - first_item;
     // Thread t owns positions [t*kSidePer, (t+1)*kSidePer) of the chunk.
     const uint32_t first = threadIdx.x * kSidePer;
     uint8_t f[kSidePer];
@@ -686,7 +760,6 @@ __global__ void k_copy_back(const Item* __restrict__ items, const uint32_t* __re
 // an empty cluster or side) is retried with the next attempt index in the
 // next level instead of at once, which changes nothing but the order.
 
-constexpr uint32_t kPlanThreads = 1024;
 constexpr uint32_t kMaxSplitAttempts = 64;
 // Level iterations a repetition may take: far above any real tree (depth
 // <= 32, each node retried at most kMaxSplitAttempts times); past it the
@@ -698,35 +771,6 @@ struct LevelCounts {
     unsigned long long pairs;  // sum of b (b - 1) / 2 over the leaves
 };
 
-// Exclusive prefix sum of one value per thread over a CTA of kPlanThreads;
-// *total receives the sum.  Every thread calls it.
-__device__ __forceinline__ unsigned long long plan_scan(unsigned long long v, unsigned long long* __restrict__ wt,
-                                                        unsigned long long* total) {
-    const int lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
-    unsigned long long incl = v;
-#pragma unroll
-    for (int o = 1; o < kWarp; o <<= 1) {
-        const unsigned long long y = __shfl_up_sync(kFull, incl, o);
-        if (lane >= o) incl += y;
-    }
-    if (lane == kWarp - 1) wt[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        unsigned long long t = wt[lane];
-#pragma unroll
-        for (int o = 1; o < kWarp; o <<= 1) {
-            const unsigned long long y = __shfl_up_sync(kFull, t, o);
-            if (lane >= o) t += y;
-        }
-        wt[lane] = t;
-    }
-    __syncthreads();
-    const unsigned long long base = warp > 0 ? wt[warp - 1] : 0ull;
-    *total = wt[kWarp - 1];
-    __syncthreads();
-    return base + incl - v;
-}
-
 // The level's sampling plan (rules of getSampleFromPercent / kmeansStartVecs,
 // as the host-sequenced level applies them; `table[n]` = sample count << 8 |
 // seed count): per node the CSR offsets of its draws, seeds and Lloyd list,
@@ -736,7 +780,7 @@ __global__ void __launch_bounds__(kPlanThreads)
     k_level_plan(const uint32_t* __restrict__ start, const uint32_t* __restrict__ end, LevelCounts* __restrict__ cnt,
                  const uint32_t* __restrict__ table, uint32_t small_threshold, uint64_t* __restrict__ draw_off,
                  uint64_t* __restrict__ seed_off, uint64_t* __restrict__ lloyd_off, SeqNode* __restrict__ seq,
-                 uint64_t* __restrict__ lbegin, uint32_t* __restrict__ lfrom, uint32_t* __restrict__ item_off) {
+                 Item* __restrict__ items) {
     __shared__ unsigned long long wt[kWarp];
     const uint32_t count = cnt->cur;
     const uint32_t per = (count + kPlanThreads - 1) / kPlanThreads;
@@ -771,20 +815,20 @@ __global__ void __launch_bounds__(kPlanThreads)
         seed_off[i] = os;
         lloyd_off[i] = ol;
         seq[i] = {of, entries, 0u};
-        lbegin[i] = list > 0 ? ol : start[i];
-        lfrom[i] = list > 0 ? 1u : 0u;
-        item_off[i] = static_cast<uint32_t>(oi);
+        // Its Lloyd items: a sample or a small node's range, a few chunks at most.
+        const uint32_t tag = i | (list > 0 ? kListItem : 0u);
+        const uint64_t begin = list > 0 ? ol : start[i];
+        for (uint32_t o = 0; o < entries; o += kChunk)
+            items[oi++] = {tag, min(static_cast<uint32_t>(kChunk), entries - o), begin + o, of + o};
         od += draws;
         os += seeds;
         ol += list;
         of += (entries + 15u) / 16u * 16u;
-        oi += (entries + kChunk - 1) / kChunk;
     }
     if (threadIdx.x == 0) {
         draw_off[count] = td;
         seed_off[count] = ts;
         lloyd_off[count] = tl;
-        item_off[count] = static_cast<uint32_t>(ti);
         cnt->lloyd_items = static_cast<uint32_t>(ti);
         cnt->nodes += count;
     }
@@ -798,20 +842,6 @@ __device__ __forceinline__ uint32_t owner_of(const uint32_t* __restrict__ off, u
         if (off[mid] <= t) lo = mid; else hi = mid - 1;
     }
     return lo;
-}
-
-// Lloyd work items of the level (chunks of kChunk entries of a node's set).
-__global__ void k_lloyd_items(const LevelCounts* __restrict__ cnt, const uint32_t* __restrict__ item_off,
-                              const SeqNode* __restrict__ seq, const uint64_t* __restrict__ lbegin,
-                              const uint32_t* __restrict__ lfrom, Item* __restrict__ items) {
-    const uint32_t count = cnt->cur, total = cnt->lloyd_items;
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-        const uint32_t i = owner_of(item_off, count, t);
-        const uint64_t o = static_cast<uint64_t>(t - item_off[i]) * kChunk;
-        const uint64_t left = seq[i].len - o;
-        items[t] = {i | (lfrom[i] ? kListItem : 0u), static_cast<uint32_t>(left < kChunk ? left : kChunk),
-                    lbegin[i] + o, seq[i].fbase + o};
-    }
 }
 
 // Partition plan: the nodes that seeded and converged (ok) are cut into
@@ -852,45 +882,56 @@ __global__ void k_part_items(const LevelCounts* __restrict__ cnt, const uint32_t
 // retried with the next attempt (no seed pair, an empty cluster or side), or
 // after kMaxSplitAttempts failures split at its index midpoint; children below
 // max_leaf points become leaves, the others the next level's nodes.
-__global__ void k_level_next(const uint32_t* __restrict__ start, const uint32_t* __restrict__ end,
-                             const uint32_t* __restrict__ base, const uint32_t* __restrict__ attempt,
-                             LevelCounts* __restrict__ cnt, const int32_t* __restrict__ ok,
-                             const uint32_t* __restrict__ node_true, const uint64_t* __restrict__ rep_params,
-                             uint32_t* __restrict__ nstart, uint32_t* __restrict__ nend, uint32_t* __restrict__ nbase,
-                             uint32_t* __restrict__ nattempt, uint32_t* __restrict__ leaf_start,
-                             uint32_t* __restrict__ leaf_end) {
+// Then the next level becomes the current one, and with `set_cond` the graph's
+// WHILE condition becomes (nodes left to split).  One CTA: counters in shared
+// memory, and no launch between the two steps.
+__global__ void __launch_bounds__(kPlanThreads)
+    k_level_next(uint32_t* __restrict__ start, uint32_t* __restrict__ end, uint32_t* __restrict__ base,
+                 uint32_t* __restrict__ attempt, LevelCounts* __restrict__ cnt, const int32_t* __restrict__ ok,
+                 const uint32_t* __restrict__ ib, const uint32_t* __restrict__ ie, const uint32_t* __restrict__ prefix,
+                 const uint64_t* __restrict__ rep_params, uint32_t* __restrict__ nstart, uint32_t* __restrict__ nend,
+                 uint32_t* __restrict__ nbase, uint32_t* __restrict__ nattempt, uint32_t* __restrict__ leaf_start,
+                 uint32_t* __restrict__ leaf_end, int32_t* __restrict__ error_flag, cudaGraphConditionalHandle cond,
+                 int set_cond) {
+    __shared__ uint32_t next_s, leaves_s, restarts_s, fallbacks_s;
+    __shared__ unsigned long long pairs_s;
     const uint32_t count = cnt->cur;
     const uint32_t max_leaf = static_cast<uint32_t>(rep_params[2]);
+    if (threadIdx.x == 0) {
+        next_s = restarts_s = fallbacks_s = 0;
+        leaves_s = cnt->leaves;
+        pairs_s = cnt->pairs;
+    }
+    __syncthreads();
+    auto node = [&](uint32_t lo, uint32_t hi, uint32_t b, uint32_t a) {
+        const uint32_t ni = atomicAdd(&next_s, 1u);
+        nstart[ni] = lo;
+        nend[ni] = hi;
+        nbase[ni] = b;
+        nattempt[ni] = a;
+    };
     auto child = [&](uint32_t lo, uint32_t hi, uint32_t b) {
         if (hi - lo < max_leaf) {
-            const uint32_t li = atomicAdd(&cnt->leaves, 1u);
+            const uint32_t li = atomicAdd(&leaves_s, 1u);
             leaf_start[li] = lo;
             leaf_end[li] = hi;
             const unsigned long long m = hi - lo;
-            atomicAdd(&cnt->pairs, m * (m - 1) / 2);
+            atomicAdd(&pairs_s, m * (m - 1) / 2);
         } else {
-            const uint32_t ni = atomicAdd(&cnt->next, 1u);
-            nstart[ni] = lo;
-            nend[ni] = hi;
-            nbase[ni] = b;
-            nattempt[ni] = 0;
+            node(lo, hi, b, 0);
         }
     };
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+    for (uint32_t i = threadIdx.x; i < count; i += kPlanThreads) {
         const uint32_t s = start[i], e = end[i], b = base[i], a = attempt[i];
-        const uint32_t n = e - s, t = node_true[i];
+        const uint32_t n = e - s, t = prefix[ie[i]] - prefix[ib[i]];
         uint32_t mid;
         if (!ok[i] || t == 0 || t == n) {
-            atomicAdd(&cnt->restarts, 1u);
+            atomicAdd(&restarts_s, 1u);
             if (a + 1 < kMaxSplitAttempts) {
-                const uint32_t ni = atomicAdd(&cnt->next, 1u);
-                nstart[ni] = s;
-                nend[ni] = e;
-                nbase[ni] = b;
-                nattempt[ni] = a + 1;
+                node(s, e, b, a + 1);
                 continue;
             }
-            atomicAdd(&cnt->fallbacks, 1u);
+            atomicAdd(&fallbacks_s, 1u);
             mid = s + n / 2;
         } else {
             mid = s + t;
@@ -898,19 +939,10 @@ __global__ void k_level_next(const uint32_t* __restrict__ start, const uint32_t*
         child(s, mid, b);
         child(mid, e, b);
     }
-}
-
-// The next level becomes the current one; with `set_cond` the graph's WHILE
-// condition becomes (nodes left to split).
-__global__ void __launch_bounds__(kPlanThreads)
-    k_level_swap(LevelCounts* __restrict__ cnt, const uint32_t* __restrict__ nstart,
-                 const uint32_t* __restrict__ nend, const uint32_t* __restrict__ nbase,
-                 const uint32_t* __restrict__ nattempt, uint32_t* __restrict__ start, uint32_t* __restrict__ end,
-                 uint32_t* __restrict__ base, uint32_t* __restrict__ attempt, int32_t* __restrict__ error_flag,
-                 cudaGraphConditionalHandle cond, int set_cond) {
+    __syncthreads();
     const bool runaway = cnt->iterations + 1 >= kMaxLevelIterations;
-    const uint32_t n = runaway ? 0u : cnt->next;
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+    const uint32_t n = runaway ? 0u : next_s;
+    for (uint32_t i = threadIdx.x; i < n; i += kPlanThreads) {
         start[i] = nstart[i];
         end[i] = nend[i];
         base[i] = nbase[i];
@@ -920,7 +952,10 @@ __global__ void __launch_bounds__(kPlanThreads)
     if (threadIdx.x == 0) {
         if (runaway) *error_flag = 1;
         cnt->cur = n;
-        cnt->next = 0;
+        cnt->leaves = leaves_s;
+        cnt->pairs = pairs_s;
+        cnt->restarts += restarts_s;
+        cnt->fallbacks += fallbacks_s;
         cnt->iterations += 1;
         if (set_cond) cudaGraphSetConditional(cond, n > 0 ? 1u : 0u);
     }
@@ -1024,7 +1059,7 @@ void launch_plane(Context& c, uint32_t count, const float* d_c1, const float* d_
                   float* d_offsets) {
     if (count == 0) return;
     KNNG_DISPATCH_D(c.d, {
-        k_plane<D><<<(count + 7) / 8, 256, 0, c.stream>>>(d_c1, d_c2, c.ld, count, d_coefs, d_offsets, nullptr);
+        k_plane<D><<<(count + 7) / 8, 256, 0, c.stream>>>(d_c1, d_c2, c.ld, count, d_coefs, d_offsets);
     });
     ++c.launches;
     KNNG_CUDA(cudaGetLastError());
@@ -1061,10 +1096,8 @@ void launch_lloyd(Context& c, uint32_t count, const uint32_t* h_starts, const ui
     KNNG_CUDA(cudaMemsetAsync(err, 0, sizeof(int32_t), c.stream));
     KNNG_DISPATCH_D(c.d, {
         for (uint32_t iter = 0; iter < iters; ++iter) {
-            launch_plane(c, count, d_c1, d_c2, d_coefs, d_offsets);
-            k_side<D><<<side_grid(ni), kSideThreads, 0, c.stream>>>(d_items, d_lloyd_positions, c.indices, c.points, c.ld,
-                                                                    d_coefs, d_offsets, flags, ids, nullptr, ni,
-                                                                    nullptr);
+            k_side<D, true><<<side_grid(ni), kSideThreads, 0, c.stream>>>(d_items, d_lloyd_positions, c.indices, c.points, c.ld,
+                                                                    d_c1, d_c2, flags, ids, nullptr, ni, nullptr);
             k_lloyd_seq<D><<<std::min(count * seq_groups(D), kSeqGrid), kSeqThreads, 0, c.stream>>>(
                 d_nodes, flags, ids, c.points, c.ld, d_c1, d_c2, d_ok, err, count, nullptr);
             c.launches += 2;
@@ -1094,12 +1127,12 @@ void launch_partition(Context& c, uint32_t count, const uint32_t* h_starts, cons
     uint32_t* prefix = static_cast<uint32_t*>(scratch(c, "item_prefix", (ni + 1) * sizeof(uint32_t)));
     KNNG_CUDA(cudaMemsetAsync(item_true, 0, ni * sizeof(uint32_t), c.stream));
     KNNG_DISPATCH_D(c.d, {
-        k_side<D><<<side_grid(ni), kSideThreads, 0, c.stream>>>(d_items, nullptr, c.indices, c.points, c.ld, d_coefs,
-                                                                d_offsets, flags, nullptr, item_true, ni, nullptr);
+        k_side<D, false><<<side_grid(ni), kSideThreads, 0, c.stream>>>(d_items, nullptr, c.indices, c.points, c.ld, d_coefs,
+                                                                       d_offsets, flags, nullptr, item_true, ni, nullptr);
     });
     k_scan_items<<<1, 1024, 0, c.stream>>>(item_true, ni, prefix, nullptr);
-    k_node_true<<<(count + 255) / 256, 256, 0, c.stream>>>(d_ib, d_ie, prefix, count, d_true, nullptr);
-    k_scatter<<<ni, kSideThreads, 0, c.stream>>>(d_items, d_starts, d_ib, d_true, prefix, flags, c.indices,
+    k_node_true<<<(count + 255) / 256, 256, 0, c.stream>>>(d_ib, d_ie, prefix, count, d_true);
+    k_scatter<<<ni, kSideThreads, 0, c.stream>>>(d_items, d_starts, d_ib, d_ie, prefix, flags, c.indices,
                                                  c.indices_tmp, nullptr);
     k_copy_back<<<ni, 256, 0, c.stream>>>(d_items, c.indices_tmp, c.indices, nullptr);
     c.launches += 5;
@@ -1126,14 +1159,13 @@ struct DevRep {
     uint64_t *draw_off, *seed_off, *lloyd_off;
     uint32_t *seeds, *lloyd;
     SeqNode* seq;
-    uint64_t* lbegin;
-    uint32_t *lfrom, *item_off, *lids;
+    uint32_t* lids;
     Item* litems;
     uint8_t* lflags;
     uint32_t *first, *second;
     int32_t* ok;
-    float *c1, *c2, *coefs, *offs;
-    uint32_t *ib, *ie, *item_true, *prefix, *node_true;
+    float *c1, *c2;
+    uint32_t *ib, *ie, *item_true, *prefix;
     Item* pitems;
     uint8_t* side_flags;
     uint64_t* h_params = nullptr;  // pinned
@@ -1275,9 +1307,6 @@ DevRep& ensure_devrep(Context& c, uint32_t max_leaf, uint32_t small_threshold) {
     r.seeds = rep_alloc<uint32_t>(c, r, static_cast<size_t>(nc) * r.max_seed + 1);
     r.lloyd = rep_alloc<uint32_t>(c, r, r.draw_cap);
     r.seq = rep_alloc<SeqNode>(c, r, nc);
-    r.lbegin = rep_alloc<uint64_t>(c, r, nc);
-    r.lfrom = rep_alloc<uint32_t>(c, r, nc);
-    r.item_off = rep_alloc<uint32_t>(c, r, nc + 1);
     r.litems = rep_alloc<Item>(c, r, r.lloyd_item_cap);
     r.lflags = rep_alloc<uint8_t>(c, r, r.entry_cap);
     r.lids = rep_alloc<uint32_t>(c, r, r.entry_cap);
@@ -1286,15 +1315,12 @@ DevRep& ensure_devrep(Context& c, uint32_t max_leaf, uint32_t small_threshold) {
     r.ok = rep_alloc<int32_t>(c, r, nc);
     r.c1 = rep_alloc<float>(c, r, static_cast<size_t>(nc) * ld);
     r.c2 = rep_alloc<float>(c, r, static_cast<size_t>(nc) * ld);
-    r.coefs = rep_alloc<float>(c, r, static_cast<size_t>(nc) * ld);
-    r.offs = rep_alloc<float>(c, r, nc);
     r.ib = rep_alloc<uint32_t>(c, r, nc);
     r.ie = rep_alloc<uint32_t>(c, r, nc);
     r.pitems = rep_alloc<Item>(c, r, r.part_item_cap);
     r.side_flags = rep_alloc<uint8_t>(c, r, static_cast<size_t>(r.n) + 16);
     r.item_true = rep_alloc<uint32_t>(c, r, r.part_item_cap + 1);
     r.prefix = rep_alloc<uint32_t>(c, r, r.part_item_cap + 1);
-    r.node_true = rep_alloc<uint32_t>(c, r, nc);
     KNNG_CUDA(cudaStreamSynchronize(c.stream));
     return r;
 }
@@ -1310,15 +1336,17 @@ void enqueue_prologue(Context& c, DevRep& r, cudaGraphConditionalHandle cond, in
     KNNG_CUDA(cudaGetLastError());
 }
 
+// Launches of a level beside the two of each Lloyd iteration.
+constexpr uint32_t kLevelLaunches = 10;
+
 // One tree level: plan, draws, seeding, Lloyd iterations, partition, outcome.
 // Launch sizes do not depend on the level; no allocation, no host sync.
 void enqueue_level(Context& c, DevRep& r, uint32_t lloyd_iters, cudaGraphConditionalHandle cond, int set_cond) {
     uint32_t* cur = &r.cnt->cur;
     k_level_plan<<<1, kPlanThreads, 0, c.stream>>>(r.start, r.end, r.cnt, r.table, r.small_threshold, r.draw_off,
-                                                   r.seed_off, r.lloyd_off, r.seq, r.lbegin, r.lfrom, r.item_off);
+                                                   r.seed_off, r.lloyd_off, r.seq, r.litems);
     k_draw_positions<<<kNodeGrid, 256, 0, c.stream>>>(r.start, r.end, r.base, r.attempt, r.draw_off, r.seed_off,
                                                       r.lloyd_off, 0, 0, r.seeds, r.lloyd, cur, r.params);
-    k_lloyd_items<<<kThreadGrid, 256, 0, c.stream>>>(r.cnt, r.item_off, r.seq, r.lbegin, r.lfrom, r.litems);
     KNNG_DISPATCH_D(c.d, {
         const size_t fp_smem = static_cast<size_t>(r.max_seed) * c.ld * sizeof(float);
         auto fp = k_farthest_pair<D>;
@@ -1326,31 +1354,26 @@ void enqueue_level(Context& c, DevRep& r, uint32_t lloyd_iters, cudaGraphConditi
         fp<<<kNodeGrid, kPairThreads, fp_smem, c.stream>>>(r.seed_off, r.seeds, c.indices, c.points, c.ld, r.first,
                                                            r.second, r.ok, r.c1, r.c2, cur);
         for (uint32_t iter = 0; iter < lloyd_iters; ++iter) {
-            k_plane<D><<<kNodeGrid, 256, 0, c.stream>>>(r.c1, r.c2, c.ld, 0, r.coefs, r.offs, cur);
-            k_side<D><<<kItemGrid, kSideThreads, 0, c.stream>>>(r.litems, r.lloyd, c.indices, c.points, c.ld, r.coefs,
-                                                                r.offs, r.lflags, r.lids, nullptr, 0,
-                                                                &r.cnt->lloyd_items);
+            k_side<D, true><<<kItemGrid, kSideThreads, 0, c.stream>>>(r.litems, r.lloyd, c.indices, c.points, c.ld, r.c1,
+                                                                      r.c2, r.lflags, r.lids, nullptr, 0,
+                                                                      &r.cnt->lloyd_items);
             k_lloyd_seq<D><<<kSeqGrid, kSeqThreads, 0, c.stream>>>(r.seq, r.lflags, r.lids, c.points, c.ld, r.c1, r.c2,
                                                                    r.ok, r.error, 0, cur);
         }
-        k_plane<D><<<kNodeGrid, 256, 0, c.stream>>>(r.c1, r.c2, c.ld, 0, r.coefs, r.offs, cur);
         k_part_plan<<<1, kPlanThreads, 0, c.stream>>>(r.start, r.end, r.cnt, r.ok, r.ib, r.ie);
         k_part_items<<<kThreadGrid, 256, 0, c.stream>>>(r.cnt, r.start, r.end, r.ib, r.pitems, r.item_true);
-        k_side<D><<<kItemGrid, kSideThreads, 0, c.stream>>>(r.pitems, nullptr, c.indices, c.points, c.ld, r.coefs,
-                                                            r.offs, r.side_flags, nullptr, r.item_true, 0,
-                                                            &r.cnt->part_items);
+        k_side<D, true><<<kItemGrid, kSideThreads, 0, c.stream>>>(r.pitems, nullptr, c.indices, c.points, c.ld, r.c1,
+                                                                  r.c2, r.side_flags, nullptr, r.item_true, 0,
+                                                                  &r.cnt->part_items);
     });
     k_scan_items<<<1, 1024, 0, c.stream>>>(r.item_true, 0, r.prefix, &r.cnt->part_items);
-    k_node_true<<<kThreadGrid, 256, 0, c.stream>>>(r.ib, r.ie, r.prefix, 0, r.node_true, cur);
-    k_scatter<<<kItemGrid, kSideThreads, 0, c.stream>>>(r.pitems, r.start, r.ib, r.node_true, r.prefix, r.side_flags,
+    k_scatter<<<kItemGrid, kSideThreads, 0, c.stream>>>(r.pitems, r.start, r.ib, r.ie, r.prefix, r.side_flags,
                                                         c.indices, c.indices_tmp, &r.cnt->part_items);
     k_copy_back<<<kItemGrid, 256, 0, c.stream>>>(r.pitems, c.indices_tmp, c.indices, &r.cnt->part_items);
-    k_level_next<<<kThreadGrid, 256, 0, c.stream>>>(r.start, r.end, r.base, r.attempt, r.cnt, r.ok, r.node_true,
-                                                    r.params, r.nstart, r.nend, r.nbase, r.nattempt, r.leaf_start,
-                                                    r.leaf_end);
-    k_level_swap<<<1, kPlanThreads, 0, c.stream>>>(r.cnt, r.nstart, r.nend, r.nbase, r.nattempt, r.start, r.end,
-                                                   r.base, r.attempt, r.error + 2, cond, set_cond);
-    c.launches += 14 + 3 * lloyd_iters;
+    k_level_next<<<1, kPlanThreads, 0, c.stream>>>(r.start, r.end, r.base, r.attempt, r.cnt, r.ok, r.ib, r.ie, r.prefix,
+                                                   r.params, r.nstart, r.nend, r.nbase, r.nattempt, r.leaf_start,
+                                                   r.leaf_end, r.error + 2, cond, set_cond);
+    c.launches += kLevelLaunches + 2 * lloyd_iters;
     KNNG_CUDA(cudaGetLastError());
 }
 
@@ -1501,7 +1524,7 @@ void run_rep_device(Context& c, uint32_t max_leaf, uint32_t lloyd_iters, uint32_
     // Kernels the graph ran: prologue (2), every level, the bucket pass (items,
     // and in the precision form norms, before the pass itself).
     const uint32_t bucket_kernels = precision == KNNG_PRECISION_BF16_RERANK ? 3 : c.leaf_tc ? 1 : 2;
-    if (graph) c.launches += 2 + bucket_kernels + static_cast<uint64_t>(h.iterations) * (14 + 3 * lloyd_iters);
+    if (graph) c.launches += 2 + bucket_kernels + static_cast<uint64_t>(h.iterations) * (kLevelLaunches + 2 * lloyd_iters);
     int32_t err[4] = {0, 0, 0, 0};
     download(c, err, r.error, 4);
     if (err[0]) fail(KNNG_ERR_CUDA, "Lloyd sums: a bulk-copy wait gave up");
