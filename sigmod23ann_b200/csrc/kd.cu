@@ -194,46 +194,81 @@ __global__ void __launch_bounds__(256) k_kd_rotate(const float* __restrict__ pts
 
 // Node statistics in a fixed order that does not depend on the launch: a
 // node's positions in chunks of kKdChunk; each chunk's values added one at a
-// time in index order to a double starting at 0 (k_kd_chunk_sums, one warp per
-// chunk, lane c one rotated dimension), then the chunk sums one at a time in
+// time in index order to a double starting at 0 (k_kd_chunk_sums, lane c one
+// rotated dimension), then the chunk sums one at a time in
 // chunk order (k_kd_node_stats, one warp per node).  With `mean` null the
 // values are rot; otherwise (rot - mean)^2 in double.
 constexpr uint32_t kKdChunk = 1024;
 constexpr int kKdWarps = 8;
 
-struct KdChunk {
-    uint32_t node, begin, end;
-};
-
-__global__ void __launch_bounds__(kKdWarps * kWarp) k_kd_chunk_sums(const KdChunk* __restrict__ chunks, uint32_t count,
-                                                                    const uint32_t* __restrict__ idx,
-                                                                    const float* __restrict__ rot, uint32_t nd,
-                                                                    const double* __restrict__ mean,
-                                                                    double* __restrict__ partial) {
-    const uint32_t item = blockIdx.x * kKdWarps + threadIdx.x / kWarp;
-    const uint32_t c = threadIdx.x % kWarp;
-    if (item >= count || c >= nd) return;
-    const KdChunk ch = chunks[item];
-    double s = 0.0;
-    if (mean == nullptr) {
-#pragma unroll 8
-        for (uint32_t i = ch.begin; i < ch.end; ++i)
-            s = __dadd_rn(s, static_cast<double>(rot[static_cast<size_t>(idx[i]) * nd + c]));
-    } else {
-        const double m = mean[static_cast<size_t>(ch.node) * nd + c];
-#pragma unroll 8
-        for (uint32_t i = ch.begin; i < ch.end; ++i) {
-            const double diff = __dsub_rn(static_cast<double>(rot[static_cast<size_t>(idx[i]) * nd + c]), m);
-            s = __dadd_rn(s, __dmul_rn(diff, diff));
-        }
+// A CTA is one warp and one chunk, so that the 150 chunks of a 150,000-point
+// level sit on as many SMs.  A chunk is a chain of 1,024 additions, each value
+// converted to double (16 cycles a warp on one sub-core: 9 us), and the values
+// are rows gathered through the index: 32 rows are in flight in registers
+// while the 32 before them are added, and their positions' indices are read a
+// batch ahead of that.  Eight chunks a CTA with eight rows in flight took 63
+// us a launch at 150,000 points, this takes 25.
+// A warp finds its node by bisection in `first_chunk` (m + 1 entries).
+__global__ void __launch_bounds__(kWarp) k_kd_chunk_sums(const uint32_t* __restrict__ first_chunk,
+                                                         const uint32_t* __restrict__ starts,
+                                                         const uint32_t* __restrict__ ends, uint32_t m,
+                                                         const uint32_t* __restrict__ idx,
+                                                         const float* __restrict__ rot, uint32_t nd,
+                                                         const double* __restrict__ mean,
+                                                         double* __restrict__ partial) {
+    const uint32_t item = blockIdx.x, lane = threadIdx.x;
+    uint32_t node = 0;
+    for (uint32_t hi = m; hi - node > 1;) {
+        const uint32_t mid = (node + hi) / 2;
+        if (first_chunk[mid] <= item)
+            node = mid;
+        else
+            hi = mid;
     }
-    partial[static_cast<size_t>(item) * nd + c] = s;
+    const uint32_t begin = starts[node] + (item - first_chunk[node]) * kKdChunk;
+    const uint32_t end = min(ends[node], begin + kKdChunk);
+    const uint32_t c = min(lane, nd - 1);  // idle lanes repeat the last dimension
+    const double mu = mean != nullptr ? mean[static_cast<size_t>(node) * nd + c] : 0.0;
+    auto id_at = [&](uint32_t i) { return idx[min(i + lane, end - 1)]; };
+    float v[2][kWarp];
+    auto gather = [&](float* row, uint32_t id) {
+#pragma unroll
+        for (int r = 0; r < kWarp; ++r)
+            row[r] = rot[static_cast<size_t>(__shfl_sync(kFull, id, r)) * nd + c];
+    };
+    double s = 0.0;
+    auto add = [&](const float* row, uint32_t rows) {
+        if (mean == nullptr) {
+#pragma unroll
+            for (int r = 0; r < kWarp; ++r)
+                if (r < static_cast<int>(rows)) s = __dadd_rn(s, static_cast<double>(row[r]));
+        } else {
+#pragma unroll
+            for (int r = 0; r < kWarp; ++r) {
+                const double diff = __dsub_rn(static_cast<double>(row[r]), mu);
+                if (r < static_cast<int>(rows)) s = __dadd_rn(s, __dmul_rn(diff, diff));
+            }
+        }
+    };
+    uint32_t id = id_at(begin + kWarp);
+    gather(v[0], id_at(begin));
+    for (uint32_t i = begin; i < end; i += 2 * kWarp) {
+        gather(v[1], id);
+        id = id_at(i + 2 * kWarp);
+        add(v[0], min(end - i, static_cast<uint32_t>(kWarp)));
+        if (end - i <= kWarp) break;
+        gather(v[0], id);
+        id = id_at(i + 3 * kWarp);
+        add(v[1], min(end - i - kWarp, static_cast<uint32_t>(kWarp)));
+    }
+    if (lane < nd) partial[static_cast<size_t>(item) * nd + lane] = s;
 }
 
 // out[node][c] = (sum of the node's chunk sums in chunk order) / divisor,
 // divisor = size (means) or size - 1 (variances).
 __global__ void __launch_bounds__(kKdWarps * kWarp) k_kd_node_stats(const uint32_t* __restrict__ first_chunk,
-                                                                    const uint32_t* __restrict__ sizes, uint32_t m,
+                                                                    const uint32_t* __restrict__ starts,
+                                                                    const uint32_t* __restrict__ ends, uint32_t m,
                                                                     const double* __restrict__ partial, uint32_t nd,
                                                                     uint32_t minus, double* __restrict__ out) {
     const uint32_t node = blockIdx.x * kKdWarps + threadIdx.x / kWarp;
@@ -243,7 +278,7 @@ __global__ void __launch_bounds__(kKdWarps * kWarp) k_kd_node_stats(const uint32
 #pragma unroll 8
     for (uint32_t j = first_chunk[node]; j < first_chunk[node + 1]; ++j)
         s = __dadd_rn(s, partial[static_cast<size_t>(j) * nd + c]);
-    out[static_cast<size_t>(node) * nd + c] = __ddiv_rn(s, static_cast<double>(sizes[node] - minus));
+    out[static_cast<size_t>(node) * nd + c] = __ddiv_rn(s, static_cast<double>(ends[node] - starts[node] - minus));
 }
 
 }  // namespace
@@ -360,36 +395,30 @@ void run_rep_kd(Context& c, uint32_t max_leaf, uint32_t new_dims, uint64_t seed,
             hs[i] = level[i].start;
             he[i] = level[i].end;
         }
-        uint32_t* d_s = upload(c, "kd_starts", hs.data(), m);
-        // Chunks of every node of the level, in node order.
-        std::vector<KdChunk> chunks;
-        std::vector<uint32_t> first(m + 1), sizes(m);
+        // Starts, ends, attempts and first chunks (in node order) in one copy.
+        std::vector<uint32_t> table(4 * static_cast<size_t>(m) + 1);
+        uint32_t nc = 0;
         for (uint32_t i = 0; i < m; ++i) {
-            first[i] = static_cast<uint32_t>(chunks.size());
-            sizes[i] = he[i] - hs[i];
-            for (uint32_t b = hs[i]; b < he[i]; b += std::min(kKdChunk, he[i] - b))
-                chunks.push_back({i, b, b + std::min(kKdChunk, he[i] - b)});
+            table[i] = hs[i];
+            table[m + i] = he[i];
+            table[2 * m + i] = level[i].attempt;
+            table[3 * m + i] = nc;
+            nc += (he[i] - hs[i] + kKdChunk - 1) / kKdChunk;
         }
-        first[m] = static_cast<uint32_t>(chunks.size());
-        const uint32_t nc = first[m];
-        const KdChunk* d_chunks = upload(c, "kd_chunks", chunks.data(), nc);
-        const uint32_t* d_first = upload(c, "kd_first_chunk", first.data(), m + 1);
-        const uint32_t* d_sizes = upload(c, "kd_sizes", sizes.data(), m);
+        table[4 * m] = nc;
+        uint32_t* d_s = upload(c, "kd_level", table.data(), table.size());
+        const uint32_t *d_e = d_s + m, *d_att = d_s + 2 * m, *d_first = d_s + 3 * m;
         auto* d_partial = static_cast<double*>(scratch(c, "kd_partial", static_cast<size_t>(nc) * nd * sizeof(double)));
         auto* d_mean = static_cast<double*>(scratch(c, "kd_mean", static_cast<size_t>(m) * nd * sizeof(double)));
         auto* d_var = static_cast<double*>(scratch(c, "kd_var", static_cast<size_t>(m) * nd * sizeof(double)));
-        const uint32_t cb = (nc + kKdWarps - 1) / kKdWarps, nb = (m + kKdWarps - 1) / kKdWarps;
-        k_kd_chunk_sums<<<cb, kKdWarps * kWarp, 0, c.stream>>>(d_chunks, nc, c.indices, rot, nd, nullptr, d_partial);
-        k_kd_node_stats<<<nb, kKdWarps * kWarp, 0, c.stream>>>(d_first, d_sizes, m, d_partial, nd, 0, d_mean);
-        k_kd_chunk_sums<<<cb, kKdWarps * kWarp, 0, c.stream>>>(d_chunks, nc, c.indices, rot, nd, d_mean, d_partial);
-        k_kd_node_stats<<<nb, kKdWarps * kWarp, 0, c.stream>>>(d_first, d_sizes, m, d_partial, nd, 1, d_var);
+        const uint32_t nb = (m + kKdWarps - 1) / kKdWarps;
+        k_kd_chunk_sums<<<nc, kWarp, 0, c.stream>>>(d_first, d_s, d_e, m, c.indices, rot, nd, nullptr, d_partial);
+        k_kd_node_stats<<<nb, kKdWarps * kWarp, 0, c.stream>>>(d_first, d_s, d_e, m, d_partial, nd, 0, d_mean);
+        k_kd_chunk_sums<<<nc, kWarp, 0, c.stream>>>(d_first, d_s, d_e, m, c.indices, rot, nd, d_mean, d_partial);
+        k_kd_node_stats<<<nb, kKdWarps * kWarp, 0, c.stream>>>(d_first, d_s, d_e, m, d_partial, nd, 1, d_var);
         c.launches += 4;
         KNNG_CUDA(cudaGetLastError());
         // Dimension picks and hyperplanes on the device.
-        std::vector<uint32_t> att(m);
-        for (uint32_t i = 0; i < m; ++i) att[i] = level[i].attempt;
-        const uint32_t* d_e = upload(c, "kd_ends", he.data(), m);
-        const uint32_t* d_att = upload(c, "kd_attempts", att.data(), m);
         auto* d_c = static_cast<float*>(scratch(c, "kd_coefs", static_cast<size_t>(m) * ld * sizeof(float)));
         auto* d_o = static_cast<float*>(scratch(c, "kd_offsets", m * sizeof(float)));
         k_kd_pick<<<nb, kKdWarps * kWarp, 0, c.stream>>>(d_s, d_e, d_att, m, d_mean, d_var, nd, d_rotation, d, ld, seed,

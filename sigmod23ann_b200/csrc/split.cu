@@ -136,7 +136,7 @@ __global__ void k_farthest_pair(const uint64_t* __restrict__ offsets, const uint
     uint32_t bi = kNone, bj = kNone;
     // The pairs in (i, j) order, a CTA's threads taking consecutive ones: with a
     // row i at a time each of the m - 1 rows was one step's latency, most
-    // threads idle (21 us a launch at 100k points, now 6).
+    // threads idle (21 us a launch at 100k points, now 7).
     for (uint32_t i = 0, j = 1 + threadIdx.x;; j += blockDim.x) {
         while (i + 1 < m && j >= m) {
             ++i;
@@ -1111,17 +1111,16 @@ void launch_partition(Context& c, uint32_t count, const uint32_t* h_starts, cons
                       const uint32_t* d_starts, const float* d_coefs, const float* d_offsets, uint32_t* d_true) {
     if (count == 0) return;
     std::vector<Item> items;
-    std::vector<uint32_t> ib(count), ie(count);
+    std::vector<uint32_t> first(count + 1, 0);
     for (uint32_t i = 0; i < count; ++i) {
-        ib[i] = static_cast<uint32_t>(items.size());
         for (uint64_t o = h_starts[i]; o < h_ends[i]; o += kChunk)
             items.push_back({i, static_cast<uint32_t>(std::min<uint64_t>(kChunk, h_ends[i] - o)), o, o});
-        ie[i] = static_cast<uint32_t>(items.size());
+        first[i + 1] = static_cast<uint32_t>(items.size());
     }
     const uint32_t ni = static_cast<uint32_t>(items.size());
     const Item* d_items = upload(c, "part_items", items.data(), ni);
-    const uint32_t* d_ib = upload(c, "part_ib", ib.data(), count);
-    const uint32_t* d_ie = upload(c, "part_ie", ie.data(), count);
+    const uint32_t* d_ib = upload(c, "part_first", first.data(), first.size());
+    const uint32_t* d_ie = d_ib + 1;
     uint8_t* flags = static_cast<uint8_t*>(scratch(c, "side_flags", c.n + 16));
     uint32_t* item_true = static_cast<uint32_t*>(scratch(c, "item_true", (ni + 1) * sizeof(uint32_t)));
     uint32_t* prefix = static_cast<uint32_t*>(scratch(c, "item_prefix", (ni + 1) * sizeof(uint32_t)));

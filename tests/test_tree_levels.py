@@ -93,3 +93,17 @@ def test_repetition_in_other_dimensions(oracle_lib, knng_lib, d):
         order = np.argsort(t["leaf_start"])
         np.testing.assert_array_equal(s, t["leaf_start"][order])
         np.testing.assert_array_equal(e, t["leaf_end"][order])
+
+
+@pytest.mark.parametrize("n,nd,leaf", [(65, 1, 33), (1024, 7, 31), (1057, 32, 64), (2081, 30, 1025), (3300, 3, 2)])
+def test_kd_sums_at_batch_and_chunk_edges(oracle_lib, knng_lib, n, nd, leaf):
+    """Nodes of every size from the bucket bound up: batches of 32 rows and
+    chunks of 1,024 that end early, one rotated dimension and all 32."""
+    pts = workloads.gaussian_mixture(n=n, d=100, clusters=8, sigma=0.3, seed=n)
+    o = oracle_lib.Oracle(pts, k=10)
+    o.kd_rep(leaf, nd, 99, 0)
+    with KnngContext(0) as ctx:
+        ctx.load_points(pts)
+        ctx.reset_sets(10)
+        ctx.run_rep_kd(leaf, nd, 99, 0)
+        np.testing.assert_array_equal(ctx.indices(), o.indices())
