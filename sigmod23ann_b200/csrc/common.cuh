@@ -14,6 +14,7 @@
 
 #include <cfloat>
 #include <cstdint>
+#include <cstring>
 
 namespace knng {
 
@@ -479,6 +480,75 @@ __device__ __forceinline__ uint32_t set_offer_new_batch(WarpSet& s, uint32_t can
     } while (pending);
     s.maxslot = __shfl_sync(kFull, mine * kWarp + lane, owner);
     return changed;
+}
+
+// Ascending sort of a warp's 32 E unsigned keys, E (a power of two) registers a
+// lane, element lane * E + r of the result in x[r]: a bitonic network.  Strides
+// below E stay in a lane; the lanes whose block a level sorts downwards hold its
+// keys complemented, so that every exchange is a minimum and a maximum.
+template <int E, class Key>
+__device__ __forceinline__ void warp_sort_lanes(Key (&x)[E], int lane) {
+#pragma unroll
+    for (int k = 2; k <= E; k <<= 1) {
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+#pragma unroll
+            for (int r = 0; r < E; ++r) {
+                if (r & j) continue;
+                // Direction of element lane * E + r at level k: within the lane
+                // below E, the lane's own bit at E.
+                const bool up = k < E ? (r & k) == 0 : (lane & 1) == 0;
+                const Key lo = min(x[r], x[r | j]), hi = max(x[r], x[r | j]);
+                x[r] = up ? lo : hi;
+                x[r | j] = up ? hi : lo;
+            }
+        }
+    }
+    Key flip = 0;
+#pragma unroll
+    for (int k = 2; k <= kWarp; k <<= 1) {  // level k * E: blocks of k lanes; the last sorts upwards everywhere
+        const Key want = (lane & k) ? ~Key(0) : Key(0);
+#pragma unroll
+        for (int r = 0; r < E; ++r) x[r] ^= flip ^ want;
+        flip = want;
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            const bool low = (lane & j) == 0;
+#pragma unroll
+            for (int r = 0; r < E; ++r) {
+                const Key o = __shfl_xor_sync(kFull, x[r], j);
+                x[r] = low ? min(x[r], o) : max(x[r], o);
+            }
+        }
+#pragma unroll
+        for (int j = E >> 1; j > 0; j >>= 1) {
+#pragma unroll
+            for (int r = 0; r < E; ++r) {
+                if (r & j) continue;
+                const Key lo = min(x[r], x[r | j]), hi = max(x[r], x[r | j]);
+                x[r] = lo;
+                x[r | j] = hi;
+            }
+        }
+    }
+}
+
+// A warp writes out[0 .. K): entries 4 lane .. 4 lane + 3 from each lane, as one
+// 16-byte store where the row's address allows it (k not a multiple of 4, or a
+// caller's array, may leave it anywhere).
+template <class T>
+__device__ __forceinline__ void store_lane_run(T* out, int K, int lane, const T (&x)[4]) {
+    static_assert(sizeof(T) == 4, "four entries are one 16-byte store");
+    const int i = 4 * lane;
+    if (i + 3 < K && (reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
+        uint4 v;
+        memcpy(&v, x, sizeof(v));
+        *reinterpret_cast<uint4*>(out + i) = v;
+    } else {
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+            if (i + r < K) out[i + r] = x[r];
+    }
 }
 
 // Ascending bitonic sort of n (power of two, n >= 2) unsigned keys by one
