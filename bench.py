@@ -47,9 +47,9 @@ REPS = 4
 REFINE = 2
 SEED = 1
 QUERIES = 10_000
-# DRAM read + write bytes of one k_join launch at 500k points (ncu capture,
-# profiles/k_join_500k.md); the bench scales it by the points processed.
-JOIN_DRAM_BYTES_500K = 55.56e9
+# DRAM read + write bytes of one k_join launch at 400k points (ncu capture,
+# profiles/k_join_400k.md); the bench scales it by the points processed.
+JOIN_DRAM_BYTES_400K = 3.15e9
 
 
 def parse_args(argv=None):
@@ -511,7 +511,7 @@ def run_precision(device: int = 0, steps: int = 3, cpu_reference: bool = True) -
 
 def refine_breakdown(st) -> dict:
     """One neighbour-of-neighbour pass's device time by stage (ms) and its
-    survivor records that went past the pool to the per-point pass."""
+    points whose candidates went past a warp's tables."""
     return {"ms": sig(st.ms_refine), "prep": sig(st.ms_refine_prep), "join": sig(st.ms_refine_join),
             "replay": sig(st.ms_refine_apply), "per_point": sig(st.ms_refine_fallback),
             "overflow": int(st.refine_overflow), "changed": int(st.refine_changed),
@@ -824,16 +824,17 @@ def run_ours(args):
         hbm_peak = float(peaks.get("hbm_gbs", 6650.0))
         # Dominant kernel: the tensor-core join of the neighbour-of-neighbour
         # pass.  Algorithmic bytes per launch: for every point q, the rows of
-        # R(q) and S(q) (4d bytes each) and the lists S(p) of R(q) (4k bytes
-        # each); sum_q |R(q)| = sum_q |S(q)| = n*k.
+        # R(q) and S(q) (4d bytes each), S(q)'s ids, R(q)'s edges with their
+        # distances and bounds (16 bytes a pair of entries) and an edge's mask
+        # (16 bytes); sum_q |R(q)| = sum_q |S(q)| = n*k.
         join_ms = sum(st["ms_refine_join"] for st in stats_list)
         join_launches = sum(st["refine_join_launches"] for st in stats_list)
         per_launch_ms = join_ms / max(1, join_launches)
-        bytes_per_launch = (2.0 * n * K * DIM * 4) + (1.0 * n * K * K * 4)
+        bytes_per_launch = (2.0 * n * K * DIM * 4) + (1.0 * n * K * 32)
         achieved = bytes_per_launch / (per_launch_ms / 1000.0) / 1e9
-        # DRAM bytes of one launch from the committed ncu capture at 500k
+        # DRAM bytes of one launch from the committed ncu capture at 400k
         # points, scaled by the points processed.
-        traffic = JOIN_DRAM_BYTES_500K * n / 500_000
+        traffic = JOIN_DRAM_BYTES_400K * n / 400_000
         roofline = {"bound": "hbm", "achieved": sig(achieved), "peak": hbm_peak, "unit": "GB/s",
                     "frac": sig(achieved / hbm_peak), "traffic": sig(traffic),
                     "kernel": "k_join", "peak_source": "measured" if peaks else "fallback",
@@ -852,7 +853,7 @@ def run_ours(args):
             "stages_ms_last_step": stages,
             # The joins' pair funnel in the last step (both passes): pairs
             # evaluated, pairs the tensor-core bound kept, of those already in
-            # the point's list, exact distances, survivor records.
+            # the point's list, exact distances, candidate records.
             "join_pairs_last_step": {k: int(last[v]) for k, v in (
                 ("pairs", "refine_pairs"), ("filter_kept", "refine_filter_pass"),
                 ("members", "refine_member_skip"), ("exact", "refine_exact"), ("survivors", "refine_emits"))},
