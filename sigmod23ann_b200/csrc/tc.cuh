@@ -1,14 +1,14 @@
 // Blackwell (sm_100a) tensor-core helpers: one CTA computes a 128 x N tile of
-// dot products G[i][j] = sum_k A[i][k] * B[j][k] with tcgen05.mma kind::tf32,
+// dot products G[i][j] = sum_k A[i][k] * B[j][k] with tcgen05.mma kind::f16,
 // operands in shared memory, accumulator in tensor memory (TMEM).
 //
 // Shared-memory operand layout (K-major, no swizzle): the tile is stored as
-// K/4 "column chunks" of 16 bytes (4 tf32 values) per row.  Chunk c of row r
+// K/8 "column chunks" of 16 bytes (8 values) per row.  Chunk c of row r
 // lives at   base + c * (ROWS * 16) + r * 16,
 // so each 8-row x 16-byte core matrix is 128 contiguous bytes.  In the
 // descriptor terms: stride-dimension byte offset (between 8-row groups) = 128,
 // leading-dimension byte offset (between the two K chunks one MMA consumes)
-// = ROWS * 16.  One MMA consumes K = 8 (two chunks); step s starts at chunk 2s.
+// = ROWS * 16.  One MMA consumes K = 16 (two chunks); step s starts at chunk 2s.
 //
 // Accumulator: M = 128 rows map to TMEM lanes 0..127, column j of the tile to
 // TMEM column (tmem_base + j).  Warp w of the CTA's first warpgroup reads
@@ -33,10 +33,6 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void mbar_inval(uint64_t* bar) {
-    asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 __device__ __forceinline__ void fence_barrier_init() {
@@ -174,44 +170,10 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo_bytes
     return d;
 }
 
-// Instruction descriptor: kind::tf32, F32 accumulate, A and B K-major, M x N.
-__host__ __device__ constexpr uint32_t idesc_tf32(uint32_t M, uint32_t N) {
-    return (1u << 4)                // D format: F32
-           | (2u << 7)              // A format: TF32
-           | (2u << 10)             // B format: TF32
-           | ((N >> 3) << 17)       // N / 8
-           | ((M >> 4) << 24);      // M / 16
-}
-
-__device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                         bool accumulate) {
-    const uint32_t acc = accumulate ? 1u : 0u;
-    const uint32_t z = 0;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-        :
-        : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(acc), "r"(z), "r"(z), "r"(z), "r"(z)
-        : "memory");
-}
-
 // Arrives on the mbarrier once every MMA this thread issued has completed.
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
-}
-
-// Issues the K/8 MMAs of one 128 x N tile (call from a single thread).
-// a_base / b_base: shared addresses of the chunk-major operand tiles with
-// a_rows (= 128) and b_rows (= N) rows; kpad: K rounded up to 8.
-__device__ __forceinline__ void issue_tile_tf32(uint32_t tmem_d, uint32_t a_base, uint32_t b_base, uint32_t a_rows,
-                                                uint32_t b_rows, uint32_t kpad, uint32_t idesc) {
-    for (uint32_t s = 0; s < kpad / 8; ++s) {
-        const uint64_t da = smem_desc(a_base + 2 * s * a_rows * 16, a_rows * 16, 128);
-        const uint64_t db = smem_desc(b_base + 2 * s * b_rows * 16, b_rows * 16, 128);
-        mma_tf32(tmem_d, da, db, idesc, s > 0);
-    }
 }
 
 // Instruction descriptor: kind::f16 with BF16 A and B, F32 accumulate, both
@@ -248,10 +210,8 @@ __host__ __device__ constexpr uint32_t idesc_f16(uint32_t M, uint32_t N) {
 }
 
 // Issues the K/16 MMAs of one 128 x N 16-bit tile (call from a single thread).
-// The operand tiles (FP16 or BF16, as idesc says) use the same chunk-major
-// layout as the TF32 ones, a 16-byte chunk holding 8 values, chunks a_stride /
-// b_stride bytes apart (at least rows * 16); one MMA consumes K = 16 (two
-// chunks).
+// The operand tiles are FP16 or BF16, as idesc says, their chunks a_stride /
+// b_stride bytes apart (at least rows * 16).
 __device__ __forceinline__ void issue_tile_strided(uint32_t tmem_d, uint32_t a_base, uint32_t b_base, uint32_t a_stride,
                                                    uint32_t b_stride, uint32_t kpad, uint32_t idesc) {
     for (uint32_t s = 0; s < kpad / 16; ++s) {
@@ -265,11 +225,6 @@ __device__ __forceinline__ void issue_tile_strided(uint32_t tmem_d, uint32_t a_b
 __device__ __forceinline__ void issue_tile_16bit(uint32_t tmem_d, uint32_t a_base, uint32_t b_base, uint32_t a_rows,
                                                  uint32_t b_rows, uint32_t kpad, uint32_t idesc) {
     issue_tile_strided(tmem_d, a_base, b_base, a_rows * 16, b_rows * 16, kpad, idesc);
-}
-
-// Byte offset of element (row r, k) in a chunk-major tile with `rows` rows.
-__host__ __device__ constexpr uint32_t chunk_offset(uint32_t r, uint32_t k, uint32_t rows) {
-    return (k >> 2) * rows * 16 + r * 16 + (k & 3) * 4;
 }
 
 }  // namespace tc
