@@ -940,8 +940,12 @@ __global__ void __launch_bounds__(kBigThreads)
 #pragma unroll
             for (int x = 0; x < 4; ++x) {
                 if (part[x] == 0) continue;
-                // The table has room for what the warps can add past the cap.
-                if (*static_cast<volatile uint32_t*>(&found_s) > cap) continue;
+                // The table has room for what the warps can add past the cap.  One
+                // lane reads the count and the others take its word: other warps
+                // add to it meanwhile, and the votes below need the whole warp.
+                uint32_t so_far = 0;
+                if (lane == 0) so_far = *static_cast<volatile uint32_t*>(&found_s);
+                if (__shfl_sync(kFull, so_far, 0) > cap) continue;
                 uint32_t c = 0, found = 0;
                 if ((part[x] >> lane) & 1u) {
                     c = __ldg(snap + static_cast<size_t>(sm.mine[a]) * K + x * kWarp + lane);

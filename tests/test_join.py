@@ -89,3 +89,23 @@ def test_distances_of_given_sets_do_not_steer_the_filter(knng_lib):
     got, changed, _ = _pass_from(pts, 100, before)
     assert_sets_equal(got, want, "scaled distances")
     assert changed == want_changed
+
+
+@pytest.mark.parametrize("cap", [1, 31, 64, 257, 700, 1500, 4000, None])
+def test_candidates_around_the_cta_cap(knng_lib, monkeypatch, cap):
+    """Part-filled lists (buckets under 43 points), so that every point has
+    thousands of candidates: the caps of the CTA's replay are passed while its
+    eight warps add candidates side by side, at counts below, amid and (None)
+    near what the points have."""
+    pts = workloads.gaussian_mixture(n=2600, d=64, clusters=8, sigma=0.2, seed=12)
+    before = _sets_after_reps(pts, 128, 43, reps=3)
+    want, want_changed, _ = _pass_from(pts, 128, before, pointwise=True)
+    monkeypatch.setenv("KNNG_REFINE_SLOTS", "0")
+    if cap is not None:
+        monkeypatch.setenv("KNNG_REFINE_POOL", str(cap))
+    got, changed, st = _pass_from(pts, 128, before)
+    assert_sets_equal(got, want, f"cap {cap}")
+    assert changed == want_changed
+    assert st.refine_overflow > 0
+    if cap is not None and cap <= 64:
+        assert st.refine_lost > 0
