@@ -509,7 +509,9 @@ __global__ void __launch_bounds__(kSeqThreads)
                         mask |= static_cast<unsigned long long>(__ballot_sync(kFull, f[a][u] == 1)) << (u * kWarp);
                     load_flags(t + kSeqAhead, f[a]);
                     const uint32_t s = g % S;
-                    if (g >= S && !tc::mbar_wait_limited(&empty[s], ((g / S) - 1) & 1u)) {
+                    // Each lane polls up to the limit by itself: the warp goes on, or
+                    // gives up, as one (the shuffles and votes need all of it).
+                    if (g >= S && !__all_sync(kFull, tc::mbar_wait_limited(&empty[s], ((g / S) - 1) & 1u))) {
                         if (lane == 0) atomicExch(error_flag, 1);
                         failed = true;
                         break;
@@ -555,7 +557,7 @@ __global__ void __launch_bounds__(kSeqThreads)
         uint32_t cnt = 0;
         for (uint32_t t = 0; t < ntiles; ++t, ++g) {
             const uint32_t s = g % S;
-            if (!tc::mbar_wait_limited(&full[s], (g / S) & 1u)) {
+            if (!__all_sync(kFull, tc::mbar_wait_limited(&full[s], (g / S) & 1u))) {  // as one, like the copiers
                 if (lane == 0) atomicExch(error_flag, 1);
                 return;
             }

@@ -64,3 +64,24 @@ def test_join_wait_runs_out_and_context_recovers(knng_lib):
         assert _same_sets(before, ctx.sets())
         ctx.refine()
         assert _same_sets(want, ctx.sets())
+
+
+@pytest.mark.parametrize("limit", [1, 2, 3, 5, 8, 20, 100])
+def test_short_limits_fail_or_give_the_result(knng_lib, limit):
+    """Limits that some waits of a warp's lanes meet and others may not: the
+    build reports the failure or returns the right lists, never anything
+    between, and the context runs on."""
+    pts = workloads.gaussian_mixture(n=9000, d=128, clusters=8, sigma=0.2, seed=33)
+    params = default_params(reps=2, refine=0, max_leaf=129, max_leaf_odd=0, lloyd_iters=2, seed=3)
+    with KnngContext(0) as ref:
+        want = ref.build(pts, params)
+    with KnngContext(0) as ctx:
+        try:
+            debug_set_wait_limit(ctx, limit)
+            try:
+                assert np.array_equal(ctx.build(pts, params), want)
+            except KnngError as e:
+                assert e.status == 2 and "gave up" in str(e)
+        finally:
+            debug_set_wait_limit(ctx, DEFAULT_LIMIT)
+        assert np.array_equal(ctx.build(pts, params), want)
