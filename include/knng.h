@@ -256,7 +256,12 @@ knng_status knng_get_leaves(knng_context* ctx, uint32_t capacity, uint32_t* star
 
 /* Neighbour-of-neighbour pass (topUpSingle, src/SolutionKmeans.hpp:480-555),
  * candidates offered in ascending id order.  out_changed and stats (its
- * refinement fields are added to) may be NULL. */
+ * refinement fields are added to) may be NULL.
+ * A pass is whole or not started.  When a wait of the join gives up, the sets
+ * are left as they were and the call reports KNNG_ERR_CUDA; only where a small
+ * budget takes the points in ranges and an earlier range has been done already
+ * do the remaining points go to the per-point pass instead (refine_lost counts
+ * them), and the call succeeds with the same sets. */
 knng_status knng_refine(knng_context* ctx, uint64_t* out_changed, knng_stats* stats);
 
 knng_status knng_get_indices(knng_context* ctx, uint32_t* out);

@@ -868,6 +868,7 @@ knng_status knng_create(int device, uint64_t hbm_budget_bytes, knng_context** ou
     if (const char* r = std::getenv("KNNG_REP_LOOP"))
         c->rep_loop = std::strcmp(r, "host") == 0 ? 2 : (std::strcmp(r, "device") == 0 ? 1 : 0);
     c->sms = sms;
+    if (const char* r = std::getenv("KNNG_JOIN_FAILS_IN")) c->join_fails_in = std::atoi(r);
     if (const char* r = std::getenv("KNNG_REFINE_POOL")) c->refine_pool = std::max<long long>(0, std::atoll(r));
     if (hbm_budget_bytes) {
         c->budget = hbm_budget_bytes;

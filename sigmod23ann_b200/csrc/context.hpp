@@ -123,6 +123,9 @@ struct Context {
     // points; false once sets were handed over or read from a file.
     bool dists_own = true;
     int64_t refine_pool = -1;
+    // Range of points (environment KNNG_JOIN_FAILS_IN at creation; -1: none) whose
+    // join is taken to have given up, for tests of what a pass then does.
+    int join_fails_in = -1;
     // Breakdown of the last refinement pass.
     struct RefineRecord {
         double ms_join = 0, ms_apply = 0, ms_fallback = 0, ms_prep = 0;

@@ -152,7 +152,7 @@ template <int D>
 __global__ void __launch_bounds__(kRefWarps * kWarp)
     k_refine(const uint32_t* __restrict__ snap, const float* __restrict__ pts, int ld, float* __restrict__ set_dist,
              uint32_t* __restrict__ set_id, uint32_t* __restrict__ set_size, uint32_t* __restrict__ set_maxslot,
-             float* __restrict__ set_bound, int K, uint32_t n, const uint32_t* __restrict__ plist,
+             float* __restrict__ set_bound, int K, uint32_t n, const uint32_t* __restrict__ plist, uint32_t first,
              unsigned long long* __restrict__ scratch_keys, uint32_t warp_capacity,
              uint32_t* __restrict__ changed_count) {
     constexpr int Q = D / 4;
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(kRefWarps * kWarp)
     unsigned long long* gbuf = scratch_keys + static_cast<size_t>(gw) * warp_capacity;
     const unsigned lt_mask = (1u << lane) - 1u;
     for (uint32_t w = gw; w < n; w += nw) {
-        const uint32_t p = plist ? plist[w] : w;
+        const uint32_t p = plist ? plist[w] : first + w;
         for (int q = lane; q < Q; q += kWarp)
             rowp_s[warp][q] = __ldg(reinterpret_cast<const float4*>(pts + static_cast<size_t>(p) * ld) + q);
         WarpSet s;
@@ -1110,24 +1110,42 @@ void run_tile_gram(Context& c, uint32_t d, const float* d_a, uint32_t m, const f
     if (h) fail(KNNG_ERR_CUDA, "tensor-core tile: the MMA completion wait gave up");
 }
 
-uint64_t run_refine_pointwise(Context& c, const uint32_t* snap, const uint32_t* d_list, uint32_t count) {
+namespace {
+
+// Survivor keys of one block's warps in the per-point pass (k * k candidates a
+// warp, as a power of two for the sort), and that pass's scratch for `blocks`.
+uint64_t pointwise_block_bytes(const Context& c) {
+    return static_cast<uint64_t>(kRefWarps) * pow2_at_least(c.k * c.k) * sizeof(unsigned long long);
+}
+struct PointwiseScratch {
+    unsigned long long* keys;
+    uint32_t* changed;
+};
+PointwiseScratch pointwise_scratch(Context& c, uint32_t blocks) {
+    return {static_cast<unsigned long long*>(scratch(c, "refine_keys", blocks * pointwise_block_bytes(c))),
+            static_cast<uint32_t*>(scratch(c, "refine_changed", sizeof(uint32_t)))};
+}
+
+}  // namespace
+
+// The per-point pass over the points of d_list, or first .. first + count - 1.
+uint64_t run_refine_pointwise(Context& c, const uint32_t* snap, const uint32_t* d_list, uint32_t count,
+                              uint32_t first = 0) {
     const int K = static_cast<int>(c.k);
     const uint32_t cap = pow2_at_least(static_cast<uint32_t>(K * K));
     uint32_t blocks = std::max<uint32_t>(1, std::min<uint32_t>((count + kRefWarps - 1) / kRefWarps, 148 * 5));
     // Each block's warps need cap survivor keys; fewer blocks (a longer grid
     // stride) when the budget leaves less room.
-    const uint64_t per_block = static_cast<uint64_t>(kRefWarps) * cap * sizeof(unsigned long long);
+    const uint64_t per_block = pointwise_block_bytes(c);
     const uint64_t held_other = c.held - scratch_bytes(c, "refine_keys");
     const uint64_t room = c.budget > held_other + (16ull << 20) ? c.budget - held_other - (16ull << 20) : 0;
     blocks = static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>(blocks, room / per_block)));
-    auto* keys = static_cast<unsigned long long*>(
-        scratch(c, "refine_keys", static_cast<size_t>(blocks) * kRefWarps * cap * sizeof(unsigned long long)));
-    auto* changed = static_cast<uint32_t*>(scratch(c, "refine_changed", sizeof(uint32_t)));
+    const auto [keys, changed] = pointwise_scratch(c, blocks);
     KNNG_CUDA(cudaMemsetAsync(changed, 0, sizeof(uint32_t), c.stream));
     KNNG_DISPATCH_D(c.d, {
         k_refine<D><<<blocks, kRefWarps * kWarp, 0, c.stream>>>(snap, c.points, c.ld, c.set_dist, c.set_id,
                                                                c.set_size, c.set_maxslot, c.set_bound, K, count,
-                                                               d_list, keys, cap, changed);
+                                                               d_list, first, keys, cap, changed);
     });
     ++c.launches;
     KNNG_CUDA(cudaGetLastError());
@@ -1184,13 +1202,19 @@ uint64_t run_refine(Context& c) {
     for (const char* name : {"refine_snap_d", "rev_count", "rev_cursor", "rev_offsets", "rev_ids", "join_masks", "apply_big",
                              "apply_lost"})
         held_mine += scratch_bytes(c, name);
-    const uint64_t reserve = std::min<uint64_t>(256ull << 20, c.budget / 8);
+    // The reserve holds the other scratch, the per-point pass's least among it.
+    const uint64_t reserve =
+        std::max<uint64_t>(std::min<uint64_t>(256ull << 20, c.budget / 8), pointwise_block_bytes(c) + (64u << 10));
     const uint64_t used = c.held - held_mine + fixed + reserve;
     const uint64_t room = c.budget > used ? c.budget - used : 0;
     const uint64_t fit = std::min<uint64_t>({n, room / (20ull * K), ((1ull << 31) - 1) / K});
     if (fit < (n + 63) / 64) return pointwise();
     const uint32_t rounds = static_cast<uint32_t>((n + fit - 1) / fit);
     const uint32_t step = (n + rounds - 1) / rounds;
+
+    // With several ranges a later one may have to go to the per-point pass after
+    // the sets have begun to change: what that needs is taken now.
+    if (rounds > 1) pointwise_scratch(c, 1);
 
     const uint32_t wblocks = std::min<uint32_t>((n + 7) / 8, 148 * 16);
     Context::RefineRecord rec;
@@ -1276,6 +1300,8 @@ uint64_t run_refine(Context& c) {
                 reinterpret_cast<uint2*>(masks), &counts->error, counts->join, order, &counts->work, old);
         });
         KNNG_CUDA(cudaGetLastError());
+        if (c.join_fails_in == static_cast<int>(r))  // as a wait that gives up leaves it
+            KNNG_CUDA(cudaMemsetAsync(&counts->error, 1, sizeof(uint32_t), c.stream));
         KNNG_CUDA(cudaEventRecord(ev[2], c.stream));
         KNNG_DISPATCH_D(c.d, {
             k_apply<D><<<std::min<uint32_t>((n + kApplyWarps - 1) / kApplyWarps, kApplyPerSm * sms), kApplyWarps * kWarp,
@@ -1292,19 +1318,23 @@ uint64_t run_refine(Context& c) {
         KNNG_CUDA(cudaEventRecord(ev[3], c.stream));
         Counts h{};
         download(c, &h, counts, 1);
-        if (h.error) {
+        // A pass is whole or not started.  The first range's join gave up: no set
+        // has changed, and the pass fails.  A later one's: the points from here on
+        // take the per-point pass, which waits for nothing, to the same sets.
+        if (h.error && r == 0) {
             for (auto& e : ev) cudaEventDestroy(e);
             fail(KNNG_ERR_CUDA, "tensor-core join: an MMA completion wait gave up");
         }
+        const uint32_t redo = h.error ? n - lo : h.lost;
         const float ms_all = elapsed(ev[0], ev[3]), ms_join = elapsed(ev[1], ev[2]), ms_apply = elapsed(ev[2], ev[3]);
         rec.ms_join += ms_join;
         rec.ms_apply += ms_apply;
         rec.ms_prep += std::max(0.f, ms_all - ms_join - ms_apply);
         // Points with too many candidates: the one-warp-per-point pass over
         // their list.
-        if (h.lost > 0) {
+        if (redo > 0) {
             KNNG_CUDA(cudaEventRecord(ev[0], c.stream));
-            changed += run_refine_pointwise(c, snap, lost, h.lost);
+            changed += run_refine_pointwise(c, snap, h.error ? nullptr : lost, redo, lo);
             KNNG_CUDA(cudaEventRecord(ev[1], c.stream));
             KNNG_CUDA(cudaEventSynchronize(ev[1]));
             rec.ms_fallback += elapsed(ev[0], ev[1]);
@@ -1316,7 +1346,8 @@ uint64_t run_refine(Context& c) {
         rec.exact += h.join[3];
         rec.emits += h.join[4] - h.join[2];
         rec.overflow += h.big;
-        rec.lost += h.lost;
+        rec.lost += redo;
+        if (h.error) break;
     }
     for (auto& e : ev) cudaEventDestroy(e);
     c.last_refine = rec;
@@ -1453,7 +1484,7 @@ extern "C" knng_status knng_refine_pointwise_noalloc(const float* d_points, uint
     try {
         KNNG_DISPATCH_D(d, {
             k_refine<D><<<blocks, kRefWarps * kWarp, 0, s>>>(d_snapshot, d_points, static_cast<int>(d), d_dist,
-                                                             d_ids, d_size, d_maxslot, d_bound, K, n, nullptr,
+                                                             d_ids, d_size, d_maxslot, d_bound, K, n, nullptr, 0,
                                                              scratch_keys, region, d_changed);
         });
     } catch (const Error& e) {

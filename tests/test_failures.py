@@ -8,7 +8,7 @@ from __future__ import annotations
 import numpy as np
 import pytest
 
-from sigmod23ann_b200 import KnngContext, KnngError, default_params, workloads
+from sigmod23ann_b200 import KnngContext, KnngError, Stats, default_params, workloads
 from sigmod23ann_b200.api import debug_set_wait_limit
 
 pytestmark = pytest.mark.gpu
@@ -85,3 +85,50 @@ def test_short_limits_fail_or_give_the_result(knng_lib, limit):
         finally:
             debug_set_wait_limit(ctx, DEFAULT_LIMIT)
         assert np.array_equal(ctx.build(pts, params), want)
+
+
+@pytest.mark.parametrize("fails_in", [0, 1, 2, 4])
+def test_a_pass_in_ranges_is_whole_or_not_started(knng_lib, monkeypatch, fails_in):
+    """A budget with room for part of the points' join: the pass goes in ranges.
+    The first range's join gives up: the call fails and no set has changed.  A
+    later one's: the pass ends with the sets it ends with otherwise."""
+    n, d, k = 12_000, 64, 50
+    pts = workloads.gaussian_mixture(n=n, d=d, clusters=16, sigma=0.2, seed=34)
+
+    def context():
+        # Points, order, sets; snapshot and its distances; counts and offsets; room
+        # for the edges (20 bytes each) of some of the points beside the reserve.
+        base = n * (4 * d + 8 + 8 * k + 12) + n * k * 8 + n * 24 + n * k * 20 // 6
+        return KnngContext(0, base * 8 // 7 + (1 << 20))
+
+    with KnngContext(0) as a:
+        a.load_points(pts)
+        a.reset_sets(k)
+        for r in range(2):
+            a.run_rep(129, 1, 3000, seed=5, rep_index=r)
+        before = a.sets()
+    wants = []
+    with context() as a:
+        a.load_points(pts)
+        a.reset_sets(k)
+        a.set_sets(before)
+        for _ in range(2):
+            st = Stats()
+            wants.append((a.refine(st), a.sets()))
+            assert st.refine_join_launches >= 5 and st.refine_lost == 0
+    monkeypatch.setenv("KNNG_JOIN_FAILS_IN", str(fails_in))
+    with context() as a:
+        a.load_points(pts)
+        a.reset_sets(k)
+        a.set_sets(before)
+        if fails_in == 0:
+            with pytest.raises(KnngError) as e:
+                a.refine()
+            assert e.value.status == 2 and "gave up" in str(e.value)
+            assert _same_sets(before, a.sets())
+        else:
+            for changed, want in wants:
+                st = Stats()
+                assert a.refine(st) == changed
+                assert _same_sets(want, a.sets())
+                assert st.refine_join_launches == fails_in + 1 and st.refine_lost > 0
