@@ -53,6 +53,14 @@ bool dim_supported(uint32_t d) { return d == 64 || d == 100 || d == 128; }
 // the device under other contexts' work.
 void* dev_alloc(Context& c, size_t bytes) {
     if (bytes == 0) bytes = 16;
+    if (c.held + bytes > c.budget) {  // the spare scratch gives way
+        for (auto& e : c.scratch) {
+            if (!e.second.spare) continue;
+            dev_free(c, e.second.ptr, e.second.bytes);
+            e.second.ptr = nullptr;
+            e.second.bytes = 0;
+        }
+    }
     if (c.held + bytes > c.budget) fail(KNNG_ERR_BUDGET, "device memory budget exceeded");
     void* p = nullptr;
     check_cuda(cudaMallocAsync(&p, bytes, c.stream), "cudaMallocAsync");
@@ -86,6 +94,14 @@ void* scratch(Context& c, const char* name, size_t bytes) {
     b.bytes = bytes == 0 ? 16 : bytes;
     c.scratch.emplace_back(name, b);
     return b.ptr;
+}
+
+void* spare_scratch(Context& c, const char* name, size_t bytes) {
+    if (scratch_bytes(c, name) < bytes && c.held - scratch_bytes(c, name) + bytes > c.budget) return nullptr;
+    void* p = scratch(c, name, bytes);
+    for (auto& e : c.scratch)
+        if (e.first == name) e.second.spare = true;
+    return p;
 }
 
 // --------------------------------------------------------------- sizing rules

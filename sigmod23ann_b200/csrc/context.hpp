@@ -27,6 +27,7 @@ void check_cuda(cudaError_t e, const char* what);
 struct DeviceBuffer {
     void* ptr = nullptr;
     size_t bytes = 0;
+    bool spare = false;  // given back when another allocation needs the room
 };
 
 struct Timer {
@@ -138,6 +139,9 @@ struct Context {
 void* dev_alloc(Context& c, size_t bytes);
 void dev_free(Context& c, void* p, size_t bytes);
 void* scratch(Context& c, const char* name, size_t bytes);
+// Scratch that a call can do without: null when the budget has no room for it.
+// It holds until the next allocation at most, which may take its room.
+void* spare_scratch(Context& c, const char* name, size_t bytes);
 // Bytes currently held by the named scratch allocation (0 if none).
 size_t scratch_bytes(const Context& c, const char* name);
 void release_all(Context& c);
@@ -264,20 +268,29 @@ uint32_t start_count(uint32_t n);
 // leaf.cu
 void launch_leaves(Context& c, uint32_t count, const uint32_t* d_starts, const uint32_t* d_ends,
                    uint32_t max_bucket, uint64_t* evals);
-// Persistent bucket pass over a device list of *d_count buckets; d_items
-// (leaf_items_bytes of it) receives its work items, *d_n_items and *d_work are
-// zeroed beforehand; *d_error is set when a tensor-core wait gives up.
-size_t leaf_items_bytes(uint32_t n);
-void launch_leaves_list(Context& c, const uint32_t* d_starts, const uint32_t* d_ends, const uint32_t* d_count,
-                        void* d_items, uint32_t* d_n_items, uint32_t* d_work, uint32_t max_bucket, uint32_t* d_error);
-// The work items of a bucket pass over [0, count) or [0, *dcount) buckets: row
-// blocks of `rows` rows in items[0 .. *n_items) (zeroed beforehand); returns the
-// inverse of the index permutation.
+// Work items of a bucket pass, row blocks: item i is rows from row[-i] on of
+// bucket leaf[-i], both arrays written from their last entry downwards.  So
+// they fit behind the bucket list itself, in arrays of one entry per point and
+// one per point set: a bucket of b >= 2 points has at most b - 1 blocks (of 16
+// rows or more), one of a single point none.
+struct LeafItems {
+    uint32_t* leaf = nullptr;
+    uint32_t* row = nullptr;
+};
+// Persistent bucket pass over a device list of *d_count buckets at the front of
+// d_starts / d_ends, arrays of `cap` = points + point sets entries whose rest
+// takes the work items; *d_n_items and *d_work are zeroed beforehand; *d_error is
+// set when a tensor-core wait gives up.
+void launch_leaves_list(Context& c, uint32_t* d_starts, uint32_t* d_ends, uint32_t cap, const uint32_t* d_count,
+                        uint32_t* d_n_items, uint32_t* d_work, uint32_t max_bucket, uint32_t* d_error);
+// The inverse of the index permutation (returned), and with `items` the work
+// items of a bucket pass over [0, count) or [0, *dcount) buckets: row blocks of
+// `rows` rows, *n_items of them (zeroed beforehand).
 uint32_t* launch_leaf_items(Context& c, uint32_t count, const uint32_t* d_starts, const uint32_t* d_ends,
-                            const uint32_t* dcount, uint32_t rows, uint2* items, uint32_t* n_items);
+                            const uint32_t* dcount, uint32_t rows, LeafItems items, uint32_t* n_items);
 // The precision form over a device list, with n floats for the rows' norms.
-void launch_leaves_bf16_list(Context& c, const uint32_t* d_starts, const uint32_t* d_ends, const uint32_t* d_count,
-                             void* d_items, uint32_t* d_n_items, uint32_t* d_work, float* d_norms, uint32_t* d_error);
+void launch_leaves_bf16_list(Context& c, uint32_t* d_starts, uint32_t* d_ends, uint32_t cap, const uint32_t* d_count,
+                             uint32_t* d_n_items, uint32_t* d_work, float* d_norms, uint32_t* d_error);
 // Exact k nearest points (FP32 distances in the reference's order) of the
 // nq points d_queries, ids into d_truth (nq x k, kNone past the end).
 void sample_knn(Context& c, const uint32_t* d_queries, uint32_t nq, uint32_t* d_truth);

@@ -193,25 +193,32 @@ __device__ __forceinline__ void distance_block(const float* __restrict__ I, cons
 
 // Work of a bucket pass: pos[id] = bucket position array's index of point id
 // (the inverse of idx), and the row blocks of the buckets of at least two
-// points, items[0 .. *n_items) = (bucket, first row), in no particular order.
-__global__ void k_leaf_items(const uint32_t* __restrict__ starts, const uint32_t* __restrict__ ends, uint32_t count,
+// points, *n_items of them, in no particular order.  The items may lie in the
+// arrays of the starts and ends, behind the last bucket.
+__global__ void k_leaf_items(const uint32_t* starts, const uint32_t* ends, uint32_t count,
                              const uint32_t* __restrict__ dcount, uint32_t rows, const uint32_t* __restrict__ idx,
-                             uint32_t n, uint32_t* __restrict__ pos, uint2* __restrict__ items,
+                             uint32_t n, uint32_t* __restrict__ pos, LeafItems items,
                              uint32_t* __restrict__ n_items) {
     if (dcount) count = *dcount;
     const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
     for (uint32_t i = first; i < n; i += stride) pos[idx[i]] = i;
+    if (!items.leaf) return;
     for (uint32_t l = first; l < count; l += stride) {
         const uint32_t b = ends[l] - starts[l];
         if (b < 2) continue;
         const uint32_t blocks = (b + rows - 1) / rows;
-        uint32_t at = atomicAdd(n_items, blocks);
-        for (uint32_t k = 0; k < blocks; ++k) items[at++] = make_uint2(l, k * rows);
+        const int64_t at = atomicAdd(n_items, blocks);
+        for (uint32_t k = 0; k < blocks; ++k) {
+            items.leaf[-(at + k)] = l;
+            items.row[-(at + k)] = k * rows;
+        }
     }
 }
 
 // A persistent grid takes row blocks of P * 16 rows (P rows a warp) from the
-// work counter.
+// work counter.  Without a list of them (items.leaf null: a budget too small for
+// one) the grid has a CTA for every (bucket of `count`, block of the largest
+// bucket), and those past their bucket's end return at once.
 //
 // kOwn: the sets hold distances of these points.  A set's members are then
 // left out of its offers, marked beforehand by their bucket positions (`pos`):
@@ -233,8 +240,8 @@ __global__ void __launch_bounds__(kLeafThreads, 2)
     k_leaf(const uint32_t* __restrict__ starts, const uint32_t* __restrict__ ends, const uint32_t* __restrict__ idx,
            const uint32_t* __restrict__ pos, const float* __restrict__ pts, int ld, float* __restrict__ set_dist,
            uint32_t* __restrict__ set_id, uint32_t* __restrict__ set_size, uint32_t* __restrict__ set_maxslot,
-           float* __restrict__ set_bound, int K, const uint2* __restrict__ items, const uint32_t* __restrict__ n_items,
-           uint32_t* __restrict__ work) {
+           float* __restrict__ set_bound, int K, LeafItems items, const uint32_t* __restrict__ n_items,
+           uint32_t* __restrict__ work, uint32_t count) {
     constexpr int R = P * kLeafWarps;
     extern __shared__ float4 smem4[];
     float* I = reinterpret_cast<float*>(smem4);
@@ -245,14 +252,22 @@ __global__ void __launch_bounds__(kLeafThreads, 2)
     __shared__ uint32_t next_s;
     __shared__ uint8_t place_s[kLeafWarps][kWarp];
     const int lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
-    const uint32_t total = *n_items;
+    const uint32_t total = items.leaf ? *n_items : 0u;
     for (;;) {
-        if (threadIdx.x == 0) next_s = atomicAdd(work, 1u);
-        __syncthreads();
-        const uint32_t w = next_s;
-        if (w >= total) break;
-        const uint2 item = items[w];
-        const uint32_t s = starts[item.x], b = ends[item.x] - s, ib = item.y;
+        uint32_t leaf, ib;
+        if (items.leaf) {
+            if (threadIdx.x == 0) next_s = atomicAdd(work, 1u);
+            __syncthreads();
+            const int64_t w = next_s;
+            if (w >= total) break;
+            leaf = items.leaf[-w];
+            ib = items.row[-w];
+        } else {
+            leaf = blockIdx.x % count;
+            ib = blockIdx.x / count * R;
+        }
+        const uint32_t s = starts[leaf], b = ends[leaf] - s;
+        if (ib >= b || b < 2) break;  // only without a list
         for (uint32_t t = threadIdx.x; t < b; t += kLeafThreads) ids[t] = idx[s + t];
         __syncthreads();
         fill_tile<D, R, true>(I, pts, ld, b - ib, [&](uint32_t r) { return ids[ib + r]; });
@@ -314,6 +329,7 @@ __global__ void __launch_bounds__(kLeafThreads, 2)
             const uint32_t p = ib + warp * P + u;
             if (p < b) set_store(sets[u], set_dist, set_id, set_size, set_maxslot, set_bound, ids[p], K, lane);
         }
+        if (!items.leaf) break;
         __syncthreads();  // everyone is done with ids, I and the work word
     }
 }
@@ -786,7 +802,7 @@ double sample_recall(Context& c, const uint32_t* d_queries, uint32_t nq, const u
 }
 
 uint32_t* launch_leaf_items(Context& c, uint32_t count, const uint32_t* d_starts, const uint32_t* d_ends,
-                            const uint32_t* dcount, uint32_t rows, uint2* items, uint32_t* n_items) {
+                            const uint32_t* dcount, uint32_t rows, LeafItems items, uint32_t* n_items) {
     uint32_t* pos = c.indices_tmp;  // the partition's second buffer is free during a bucket pass
     k_leaf_items<<<std::min<uint32_t>((c.n + 255) / 256, 148 * 8), 256, 0, c.stream>>>(
         d_starts, d_ends, count, dcount, rows, c.indices, c.n, pos, items, n_items);
@@ -805,8 +821,9 @@ uint32_t leaf_rows(const Context& c) { return c.n >= 2u * c.sms * 2u * kLeafWarp
 
 // The bucket pass over the buckets [0, count) or [0, *dcount): its items, then
 // a persistent grid of leaf_ctas CTAs per SM.  *n_items and *work start at 0.
+// Without a list (and then with a host count) a CTA per possible row block.
 void enqueue_leaves(Context& c, uint32_t count, const uint32_t* d_starts, const uint32_t* d_ends, const uint32_t* dcount,
-                    uint2* items, uint32_t* n_items, uint32_t* work, uint32_t max_bucket) {
+                    LeafItems items, uint32_t* n_items, uint32_t* work, uint32_t max_bucket) {
     const uint32_t rows = leaf_rows(c);
     uint32_t* pos = launch_leaf_items(c, count, d_starts, d_ends, dcount, rows, items, n_items);
     KNNG_DISPATCH_D(c.d, {
@@ -818,11 +835,21 @@ void enqueue_leaves(Context& c, uint32_t count, const uint32_t* d_starts, const 
         auto kern = rows == kLeafWarps ? (c.dists_own ? k_leaf<D, 1, true> : k_leaf<D, 1, false>)
                                        : (c.dists_own ? k_leaf<D, 2, true> : k_leaf<D, 2, false>);
         allow_max_smem(c, kern);
-        kern<<<c.leaf_ctas * c.sms, kLeafThreads, smem, c.stream>>>(
-            d_starts, d_ends, c.indices, pos, c.points, c.ld, c.set_dist, c.set_id, c.set_size, c.set_maxslot,
-            c.set_bound, static_cast<int>(c.k), items, n_items, work);
+        auto run = [&](uint32_t grid, uint32_t first, uint32_t buckets) {
+            kern<<<grid, kLeafThreads, smem, c.stream>>>(
+                d_starts + first, d_ends + first, c.indices, pos, c.points, c.ld, c.set_dist, c.set_id, c.set_size,
+                c.set_maxslot, c.set_bound, static_cast<int>(c.k), items, n_items, work, buckets);
+            ++c.launches;
+        };
+        if (items.leaf) {
+            run(c.leaf_ctas * c.sms, 0, 0);
+        } else {
+            const uint32_t blocks = (max_bucket + rows - 1) / rows;
+            const uint32_t most = (1u << 30) / blocks;  // buckets whose blocks a grid has room for
+            for (uint32_t first = 0; first < count; first += std::min(most, count - first))
+                run(std::min(most, count - first) * blocks, first, std::min(most, count - first));
+        }
     });
-    ++c.launches;
     KNNG_CUDA(cudaGetLastError());
 }
 
@@ -851,12 +878,17 @@ void launch_leaves(Context& c, uint32_t count, const uint32_t* d_starts, const u
         if (h) fail(KNNG_ERR_CUDA, "bucket pass: the MMA completion wait gave up");
         return;
     }
-    // Row blocks: at most one more than n / rows of each bucket.
-    const uint32_t rows = leaf_rows(c);
-    auto* items = static_cast<uint2*>(scratch(c, "leaf_items", (c.n / rows + static_cast<size_t>(count) + 1) * sizeof(uint2)));
-    auto* counters = static_cast<uint32_t*>(scratch(c, "leaf_counters", 2 * sizeof(uint32_t)));
-    KNNG_CUDA(cudaMemsetAsync(counters, 0, 2 * sizeof(uint32_t), c.stream));
-    enqueue_leaves(c, count, d_starts, d_ends, nullptr, items, counters, counters + 1, max_bucket);
+    // Two counters and the row blocks, at most one more than n / rows of each
+    // bucket.  A budget without room for them runs the pass without a list.
+    const size_t cap = c.n / leaf_rows(c) + static_cast<size_t>(count) + 1;
+    auto* lists = static_cast<uint32_t*>(spare_scratch(c, "leaf_items", (2 + 2 * cap) * sizeof(uint32_t)));
+    if (!lists) {
+        enqueue_leaves(c, count, d_starts, d_ends, nullptr, {}, nullptr, nullptr, max_bucket);
+        return;
+    }
+    KNNG_CUDA(cudaMemsetAsync(lists, 0, 2 * sizeof(uint32_t), c.stream));
+    const LeafItems items{lists + 1 + cap, lists + 1 + 2 * cap};
+    enqueue_leaves(c, count, d_starts, d_ends, nullptr, items, lists, lists + 1, max_bucket);
 }
 
 void prepare_leaves_list(Context& c) {
@@ -869,13 +901,8 @@ void prepare_leaves_list(Context& c) {
     });
 }
 
-size_t leaf_items_bytes(uint32_t n) {
-    // Buckets of at least two points, and rows of at least 16 a block.
-    return (static_cast<size_t>(n) / kLeafWarps + n / 2 + 1) * sizeof(uint2);
-}
-
-void launch_leaves_list(Context& c, const uint32_t* d_starts, const uint32_t* d_ends, const uint32_t* d_count,
-                        void* d_items, uint32_t* d_n_items, uint32_t* d_work, uint32_t max_bucket, uint32_t* d_error) {
+void launch_leaves_list(Context& c, uint32_t* d_starts, uint32_t* d_ends, uint32_t cap, const uint32_t* d_count,
+                        uint32_t* d_n_items, uint32_t* d_work, uint32_t max_bucket, uint32_t* d_error) {
     if (c.leaf_tc) {
         KNNG_DISPATCH_D(c.d, {
             const size_t smem = LeafTc<D>::bytes(max_bucket);
@@ -891,7 +918,7 @@ void launch_leaves_list(Context& c, const uint32_t* d_starts, const uint32_t* d_
         KNNG_CUDA(cudaGetLastError());
         return;
     }
-    enqueue_leaves(c, 0, d_starts, d_ends, d_count, static_cast<uint2*>(d_items), d_n_items, d_work, max_bucket);
+    enqueue_leaves(c, 0, d_starts, d_ends, d_count, {d_starts + cap - 1, d_ends + cap - 1}, d_n_items, d_work, max_bucket);
 }
 
 }  // namespace knng

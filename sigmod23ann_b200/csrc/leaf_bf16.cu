@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(kBfThreads, kBfPerSm)
                 const uint32_t* __restrict__ idx, const uint32_t* __restrict__ pos, const float* __restrict__ norms_g,
                 const float* __restrict__ pts, int ld, float* __restrict__ set_dist, uint32_t* __restrict__ set_id,
                 uint32_t* __restrict__ set_size, uint32_t* __restrict__ set_maxslot, float* __restrict__ set_bound, int K,
-                bool own, uint32_t* __restrict__ error_flag, const uint2* __restrict__ items,
+                bool own, uint32_t* __restrict__ error_flag, LeafItems items,
                 const uint32_t* __restrict__ n_items, uint32_t* __restrict__ work) {
     using L = BfLayout<D>;
     using T = Tile16<D>;
@@ -237,10 +237,10 @@ __global__ void __launch_bounds__(kBfThreads, kBfPerSm)
     while (healthy) {
         if (tid == 0) next_s = atomicAdd(work, 1u);
         __syncthreads();
-        const uint32_t w = next_s;
+        const int64_t w = next_s;
         if (w >= total) break;
-        const uint2 item = items[w];
-        const uint32_t s0 = starts[item.x], b = ends[item.x] - s0, rb = item.y;
+        const uint32_t leaf = items.leaf[-w], rb = items.row[-w];
+        const uint32_t s0 = starts[leaf], b = ends[leaf] - s0;
         // Buckets of at most 129 points keep every other member: no estimates.
         const bool keep_all = b - 1 <= static_cast<uint32_t>(kKeep);
         for (uint32_t t = tid; t < b; t += kBfThreads) {
@@ -457,7 +457,7 @@ namespace {
 // The pass over the buckets [0, count) or [0, *dcount): its items and norms, then
 // a persistent grid.  *n_items and *work start at 0.
 void enqueue_bf16(Context& c, uint32_t count, const uint32_t* d_starts, const uint32_t* d_ends, const uint32_t* dcount,
-                  uint2* items, uint32_t* n_items, uint32_t* work, float* norms, uint32_t* d_error) {
+                  LeafItems items, uint32_t* n_items, uint32_t* work, float* norms, uint32_t* d_error) {
     uint32_t* pos = launch_leaf_items(c, count, d_starts, d_ends, dcount, kBfRows, items, n_items);
     KNNG_DISPATCH_D(c.d, {
         k_bf16_norms<D><<<c.sms * 8, 256, 0, c.stream>>>(d_starts, d_ends, count, dcount, c.indices, c.points, c.ld, norms);
@@ -478,15 +478,15 @@ void launch_leaves_bf16(Context& c, uint32_t count, const uint32_t* d_starts, co
     if (count == 0) return;
     if (max_bucket > static_cast<uint32_t>(kBfMaxBucket))
         fail(KNNG_ERR_INVALID_ARGUMENT, "the BF16 bucket pass takes buckets of at most 1024 points");
-    auto* items = static_cast<uint2*>(
-        scratch(c, "leaf_items", (c.n / kBfRows + static_cast<size_t>(count) + 1) * sizeof(uint2)));
-    auto* norms = static_cast<float*>(scratch(c, "bf16_norms", static_cast<size_t>(c.n) * sizeof(float)));
-    // Items, work counter, error word.
-    auto* counters = static_cast<uint32_t*>(scratch(c, "bf16_counters", 3 * sizeof(uint32_t)));
-    KNNG_CUDA(cudaMemsetAsync(counters, 0, 3 * sizeof(uint32_t), c.stream));
-    enqueue_bf16(c, count, d_starts, d_ends, nullptr, items, counters, counters + 1, norms, counters + 2);
+    // Item count, work counter, error word; the items; the norms.
+    const size_t cap = c.n / kBfRows + static_cast<size_t>(count) + 1;
+    auto* lists = static_cast<uint32_t*>(spare_scratch(c, "bf16_lists", (3 + 2 * cap + c.n) * sizeof(uint32_t)));
+    if (!lists) fail(KNNG_ERR_BUDGET, "device memory budget exceeded");
+    KNNG_CUDA(cudaMemsetAsync(lists, 0, 3 * sizeof(uint32_t), c.stream));
+    enqueue_bf16(c, count, d_starts, d_ends, nullptr, {lists + 2 + cap, lists + 2 + 2 * cap}, lists, lists + 1,
+                 reinterpret_cast<float*>(lists + 3 + 2 * cap), lists + 2);
     uint32_t h = 0;
-    download(c, &h, counters + 2, 1);
+    download(c, &h, lists + 2, 1);
     if (h) fail(KNNG_ERR_CUDA, "BF16 bucket pass: the MMA completion wait gave up");
 }
 
@@ -494,9 +494,10 @@ void prepare_leaves_bf16_list(Context& c) {
     KNNG_DISPATCH_D(c.d, { allow_max_smem(c, k_leaf_bf16<D>); });
 }
 
-void launch_leaves_bf16_list(Context& c, const uint32_t* d_starts, const uint32_t* d_ends, const uint32_t* d_count,
-                             void* d_items, uint32_t* d_n_items, uint32_t* d_work, float* d_norms, uint32_t* d_error) {
-    enqueue_bf16(c, 0, d_starts, d_ends, d_count, static_cast<uint2*>(d_items), d_n_items, d_work, d_norms, d_error);
+void launch_leaves_bf16_list(Context& c, uint32_t* d_starts, uint32_t* d_ends, uint32_t cap, const uint32_t* d_count,
+                             uint32_t* d_n_items, uint32_t* d_work, float* d_norms, uint32_t* d_error) {
+    enqueue_bf16(c, 0, d_starts, d_ends, d_count, {d_starts + cap - 1, d_ends + cap - 1}, d_n_items, d_work, d_norms,
+                 d_error);
 }
 
 }  // namespace knng

@@ -1153,7 +1153,6 @@ struct DevRep {
     std::vector<std::pair<void*, size_t>> allocs;
     uint32_t *set_offsets, *table;
     uint32_t *start, *end, *base, *attempt, *nstart, *nend, *nbase, *nattempt, *leaf_start, *leaf_end;
-    uint8_t* leaf_items;  // work items of the bucket pass
     LevelCounts* cnt;
     uint64_t* params;  // seed, repetition, max_leaf, 0
     int32_t* error;    // [0] Lloyd sums, [1] BF16 bucket pass
@@ -1298,7 +1297,6 @@ DevRep& ensure_devrep(Context& c, uint32_t max_leaf, uint32_t small_threshold) {
     r.nattempt = rep_alloc<uint32_t>(c, r, nc);
     r.leaf_start = rep_alloc<uint32_t>(c, r, r.n + r.nsets);
     r.leaf_end = rep_alloc<uint32_t>(c, r, r.n + r.nsets);
-    r.leaf_items = rep_alloc<uint8_t>(c, r, leaf_items_bytes(r.n));
     r.cnt = rep_alloc<LevelCounts>(c, r, 1);
     r.params = rep_alloc<uint64_t>(c, r, 4);
     r.error = rep_alloc<int32_t>(c, r, 4);
@@ -1380,12 +1378,12 @@ void enqueue_level(Context& c, DevRep& r, uint32_t lloyd_iters, cudaGraphConditi
 
 void enqueue_buckets(Context& c, DevRep& r, uint32_t max_leaf, uint32_t precision) {
     if (precision == KNNG_PRECISION_BF16_RERANK)
-        launch_leaves_bf16_list(c, r.leaf_start, r.leaf_end, &r.cnt->leaves, r.leaf_items, &r.cnt->leaf_items,
+        launch_leaves_bf16_list(c, r.leaf_start, r.leaf_end, r.n + r.nsets, &r.cnt->leaves, &r.cnt->leaf_items,
                                 &r.cnt->leaf_work,
                                 reinterpret_cast<float*>(r.lids),  // at least n entries, free once the tree is built
                                 reinterpret_cast<uint32_t*>(r.error + 1));
     else
-        launch_leaves_list(c, r.leaf_start, r.leaf_end, &r.cnt->leaves, r.leaf_items, &r.cnt->leaf_items,
+        launch_leaves_list(c, r.leaf_start, r.leaf_end, r.n + r.nsets, &r.cnt->leaves, &r.cnt->leaf_items,
                            &r.cnt->leaf_work, max_leaf - 1, reinterpret_cast<uint32_t*>(r.error + 1));
 }
 

@@ -3,11 +3,13 @@ windows, with empty, part-filled and full sets, against the oracle's pass over
 the same bucket."""
 from __future__ import annotations
 
+import os
+
 import numpy as np
 import pytest
 
 from helpers import assert_sets_equal
-from sigmod23ann_b200 import KnngContext, workloads
+from sigmod23ann_b200 import KnngContext, KnngError, default_params, workloads
 
 pytestmark = pytest.mark.gpu
 
@@ -68,14 +70,90 @@ def test_many_buckets_in_blocks_of_32_rows(knng_lib, oracle_lib):
         assert np.array_equal(got["id"][ids][filled], ids[o["id"]][filled])
 
 
+def _smallest_budget(call, high):
+    """The smallest budget, to 256 bytes, that `call` runs with on a fresh context."""
+    low = 1 << 20
+    while high - low > 256:
+        mid = (low + high) // 2
+        try:
+            with KnngContext(0, mid) as c:
+                call(c)
+            high = mid
+        except KnngError as e:
+            assert e.status == 4
+            low = mid
+    return high
+
+
+@pytest.mark.parametrize("n,d,k,leaf", [(9000, 100, 20, 300), (12_001, 64, 10, 90)])
+def test_the_pass_needs_no_memory_of_its_own(knng_lib, n, d, k, leaf):
+    """Buckets given by the caller run with the budget that points, order, sets
+    and the bucket bounds take up, without room for a list of row blocks, and to
+    the same sets (blocks of 16 and of 32 rows, empty buckets and single points
+    among them)."""
+    pts = workloads.gaussian_mixture(n=n, d=d, clusters=8, sigma=0.2, seed=n)
+    cuts = [0, 0, 1, 2, 5, 100, *range(100 + leaf, n, leaf), n]
+    starts, ends = np.array(cuts[:-1], np.uint32), np.array(cuts[1:], np.uint32)
+    got = {}
+
+    def call(c):
+        c.load_points(pts)
+        c.reset_sets(k)
+        for _ in range(2):
+            c.process_leaves(starts, ends)
+        got["sets"] = c.sets()
+
+    with KnngContext(0) as c:
+        call(c)
+    want = got["sets"]
+    held = n * (4 * d + 8 + 8 * k + 12) + 2 * (4 * len(starts) + 16)
+    assert _smallest_budget(call, 64 << 20) <= held + 256
+    with KnngContext(0, held) as c:
+        call(c)
+    assert_sets_equal(got["sets"], want, "without a list")
+    # A list that fitted gives way to what is allocated after it.
+    with KnngContext(0, held + 2 * (n // 16 + len(starts) + 8) * 4) as c:
+        call(c)
+        assert_sets_equal(got["sets"], want, "with a list")
+    room = held + 4 * n * k + 64
+    with KnngContext(0, room) as c:
+        call(c)
+        ids = c.finalize()
+    with KnngContext(0) as c:
+        call(c)
+        assert np.array_equal(c.finalize(), ids)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("offsets", [None, [0, 1, 2, 4, 7, 4000, 6001]])
+def test_items_fit_behind_the_leaves(knng_lib, precision, offsets):
+    """Repetitions with the smallest buckets (two points and one; point sets of one
+    point too), where leaves and row blocks fill their arrays: the lists of the
+    form that keeps its own."""
+    n = 6001
+    pts = workloads.gaussian_mixture(n=n, d=64, clusters=8, sigma=0.2, seed=5)
+    lists = []
+    for loop in ("graph", "device", "host"):
+        os.environ["KNNG_REP_LOOP"] = loop
+        try:
+            with KnngContext(0) as c:
+                p = default_params(k=7, reps=2, refine=0, max_leaf=3, max_leaf_odd=2, lloyd_iters=1, precision=precision)
+                if offsets is None:
+                    lists.append(c.build(pts, p))
+                else:
+                    lists.append(np.concatenate(c.build_batch([pts[a:b] for a, b in zip(offsets, offsets[1:])], p)))
+        finally:
+            os.environ.pop("KNNG_REP_LOOP", None)
+    assert np.array_equal(lists[0], lists[2])
+    assert np.array_equal(lists[1], lists[2])
+
+
 @pytest.mark.parametrize("n", [2, 33, 129, 130, 131, 160, 256, 257, 300, 1000])
 @pytest.mark.parametrize("d", [64, 100, 128])
 def test_precision_form_keeps_the_128_best(knng_lib, n, d):
     """Points with small integer coordinates: the BF16 estimates are the exact
     distances, with many ties, so the kept candidates of a bucket are the 128
     smallest by (distance, position) and lists of 128 hold just them."""
-    from sigmod23ann_b200 import default_params
-
     rng = np.random.default_rng(n + d)
     pts = np.zeros((n, d), np.float32)
     pts[:, :6] = rng.integers(-2, 3, (n, 6))
