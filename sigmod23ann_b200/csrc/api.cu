@@ -55,7 +55,7 @@ void* dev_alloc(Context& c, size_t bytes) {
     if (bytes == 0) bytes = 16;
     if (c.held + bytes > c.budget) {  // the spare scratch gives way
         for (auto& e : c.scratch) {
-            if (!e.second.spare) continue;
+            if (!e.second.spare || c.held + bytes <= c.budget) continue;
             dev_free(c, e.second.ptr, e.second.bytes);
             e.second.ptr = nullptr;
             e.second.bytes = 0;
@@ -99,9 +99,13 @@ void* scratch(Context& c, const char* name, size_t bytes) {
 void* spare_scratch(Context& c, const char* name, size_t bytes) {
     if (scratch_bytes(c, name) < bytes && c.held - scratch_bytes(c, name) + bytes > c.budget) return nullptr;
     void* p = scratch(c, name, bytes);
-    for (auto& e : c.scratch)
-        if (e.first == name) e.second.spare = true;
+    set_spare(c, name, true);
     return p;
+}
+
+void set_spare(Context& c, const char* name, bool spare) {
+    for (auto& e : c.scratch)
+        if (e.first == name) e.second.spare = spare;
 }
 
 // --------------------------------------------------------------- sizing rules

@@ -142,6 +142,8 @@ void* scratch(Context& c, const char* name, size_t bytes);
 // Scratch that a call can do without: null when the budget has no room for it.
 // It holds until the next allocation at most, which may take its room.
 void* spare_scratch(Context& c, const char* name, size_t bytes);
+// Marks the named scratch as spare, or as needed again.
+void set_spare(Context& c, const char* name, bool spare);
 // Bytes currently held by the named scratch allocation (0 if none).
 size_t scratch_bytes(const Context& c, const char* name);
 void release_all(Context& c);

@@ -1154,8 +1154,29 @@ uint64_t run_refine_pointwise(Context& c, const uint32_t* snap, const uint32_t* 
     return h;
 }
 
+namespace {
+
+// The large scratch of a pass, beside its snapshots (which the next pass looks
+// at).  A join takes up to all of the budget for it, so between passes it is
+// spare: whatever is allocated then, the finished lists for instance, may have
+// its room.
+constexpr const char* kPassScratch[] = {"refine_snap_d", "rev_count", "rev_cursor", "rev_offsets", "rev_ids",
+                                        "join_masks",    "apply_big", "apply_lost"};
+struct PassScratch {
+    Context& c;
+    explicit PassScratch(Context& ctx) : c(ctx) { mark(false); }
+    ~PassScratch() { mark(true); }
+    void mark(bool spare) {
+        for (const char* name : kPassScratch) set_spare(c, name, spare);
+        set_spare(c, "refine_keys", spare);
+    }
+};
+
+}  // namespace
+
 uint64_t run_refine(Context& c) {
     if (c.n == 0) return 0;
+    PassScratch pass_scratch(c);
     const int K = static_cast<int>(c.k);
     const uint32_t n = c.n;
     const size_t entries = static_cast<size_t>(n) * K;
@@ -1199,9 +1220,7 @@ uint64_t run_refine(Context& c) {
     // leaves the pass to the per-point kernel.
     const uint64_t fixed = entries * 4 + static_cast<uint64_t>(n) * 24;
     uint64_t held_mine = 0;
-    for (const char* name : {"refine_snap_d", "rev_count", "rev_cursor", "rev_offsets", "rev_ids", "join_masks", "apply_big",
-                             "apply_lost"})
-        held_mine += scratch_bytes(c, name);
+    for (const char* name : kPassScratch) held_mine += scratch_bytes(c, name);
     // The reserve holds the other scratch, the per-point pass's least among it.
     const uint64_t reserve =
         std::max<uint64_t>(std::min<uint64_t>(256ull << 20, c.budget / 8), pointwise_block_bytes(c) + (64u << 10));

@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 
 from helpers import assert_sets_equal
-from sigmod23ann_b200 import KnngContext, Stats, workloads
+from sigmod23ann_b200 import KnngContext, Stats, default_params, workloads
 
 pytestmark = pytest.mark.gpu
 
@@ -77,6 +77,26 @@ def test_small_budgets_take_ranges_of_points(knng_lib):
         assert changed == want_changed
         seen.add(int(st.refine_join_launches))
     assert max(seen) > 1, seen
+
+
+@pytest.mark.parametrize("n,d,k,passes", [(20_000, 64, 10, 2), (12_000, 100, 60, 1), (12_000, 100, 60, 2)])
+def test_finished_lists_fit_whatever_the_passes_took(knng_lib, n, d, k, passes):
+    """From the budget on that a whole build has always needed (its buffers, a
+    pass's snapshots and per-edge lists, the finished lists), every budget does:
+    a pass that takes its points in ranges takes what there is, and gives way to
+    the lists.  The lists are the same."""
+    pts = workloads.gaussian_mixture(n=n, d=d, clusters=16, sigma=0.2, seed=n + k)
+    p = default_params(k=k, reps=1, refine=passes, max_leaf=257, max_leaf_odd=0, lloyd_iters=1, seed=5)
+    with KnngContext(0) as c:
+        want = c.build(pts, p, want_dists=True)
+    need = n * (4 * d + 8 + 8 * k + 12)  # points, order, sets
+    need += n * 64 + (4 << 20)           # a repetition's buffers, small scratch
+    need += n * (8 * k + 16) + n * k * 4  # snapshots and their marks, per-edge lists
+    need += n * k * 8                    # the finished lists
+    for share in range(0, 24):
+        with KnngContext(0, need + n * k * share) as c:
+            ids, dists = c.build(pts, p, want_dists=True)
+        assert np.array_equal(ids, want[0]) and np.array_equal(dists, want[1]), share
 
 
 def test_distances_of_given_sets_do_not_steer_the_filter(knng_lib):
