@@ -48,6 +48,14 @@ void check_cuda(cudaError_t e, const char* what) {
 
 bool dim_supported(uint32_t d) { return d == 64 || d == 100 || d == 128; }
 
+namespace {
+void free_buffer(Context& c, DeviceBuffer& b) {
+    dev_free(c, b.ptr, b.bytes);
+    b.ptr = nullptr;
+    b.bytes = 0;
+}
+}  // namespace
+
 // Device memory is stream-ordered on the context's stream (all of the
 // context's work runs there), so allocating or freeing does not synchronise
 // the device under other contexts' work.
@@ -55,10 +63,7 @@ void* dev_alloc(Context& c, size_t bytes) {
     if (bytes == 0) bytes = 16;
     if (c.held + bytes > c.budget) {  // the spare scratch gives way
         for (auto& e : c.scratch) {
-            if (!e.second.spare || c.held + bytes <= c.budget) continue;
-            dev_free(c, e.second.ptr, e.second.bytes);
-            e.second.ptr = nullptr;
-            e.second.bytes = 0;
+            if (e.second.spare && c.held + bytes > c.budget) free_buffer(c, e.second);
         }
     }
     if (c.held + bytes > c.budget) fail(KNNG_ERR_BUDGET, "device memory budget exceeded");
@@ -81,9 +86,7 @@ void* scratch(Context& c, const char* name, size_t bytes) {
             KNNG_CUDA(cudaStreamSynchronize(c.stream));
             size_t grown = std::max(bytes, e.second.bytes * 3 / 2);
             if (c.held - e.second.bytes + grown > c.budget) grown = bytes;
-            dev_free(c, e.second.ptr, e.second.bytes);
-            e.second.ptr = nullptr;
-            e.second.bytes = 0;
+            free_buffer(c, e.second);
             e.second.ptr = dev_alloc(c, grown);
             e.second.bytes = grown;
             return e.second.ptr;
@@ -106,6 +109,17 @@ void* spare_scratch(Context& c, const char* name, size_t bytes) {
 void set_spare(Context& c, const char* name, bool spare) {
     for (auto& e : c.scratch)
         if (e.first == name) e.second.spare = spare;
+}
+
+uint64_t spare_bytes(const Context& c) {
+    uint64_t bytes = 0;
+    for (const auto& e : c.scratch) bytes += e.second.spare ? e.second.bytes : 0;
+    return bytes;
+}
+
+void scratch_free(Context& c, const char* name) {
+    for (auto& e : c.scratch)
+        if (e.first == name) free_buffer(c, e.second);
 }
 
 // --------------------------------------------------------------- sizing rules

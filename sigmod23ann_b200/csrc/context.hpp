@@ -144,6 +144,10 @@ void* scratch(Context& c, const char* name, size_t bytes);
 void* spare_scratch(Context& c, const char* name, size_t bytes);
 // Marks the named scratch as spare, or as needed again.
 void set_spare(Context& c, const char* name, bool spare);
+// Bytes that spare scratch holds.
+uint64_t spare_bytes(const Context& c);
+// Frees the named scratch.
+void scratch_free(Context& c, const char* name);
 // Bytes currently held by the named scratch allocation (0 if none).
 size_t scratch_bytes(const Context& c, const char* name);
 void release_all(Context& c);

@@ -1122,8 +1122,9 @@ struct PointwiseScratch {
     uint32_t* changed;
 };
 PointwiseScratch pointwise_scratch(Context& c, uint32_t blocks) {
-    return {static_cast<unsigned long long*>(scratch(c, "refine_keys", blocks * pointwise_block_bytes(c))),
-            static_cast<uint32_t*>(scratch(c, "refine_changed", sizeof(uint32_t)))};
+    auto* keys = static_cast<unsigned long long*>(scratch(c, "refine_keys", blocks * pointwise_block_bytes(c)));
+    set_spare(c, "refine_keys", false);
+    return {keys, static_cast<uint32_t*>(scratch(c, "refine_changed", sizeof(uint32_t)))};
 }
 
 }  // namespace
@@ -1137,7 +1138,8 @@ uint64_t run_refine_pointwise(Context& c, const uint32_t* snap, const uint32_t* 
     // Each block's warps need cap survivor keys; fewer blocks (a longer grid
     // stride) when the budget leaves less room.
     const uint64_t per_block = pointwise_block_bytes(c);
-    const uint64_t held_other = c.held - scratch_bytes(c, "refine_keys");
+    set_spare(c, "refine_keys", false);
+    const uint64_t held_other = c.held - scratch_bytes(c, "refine_keys") - spare_bytes(c);
     const uint64_t room = c.budget > held_other + (16ull << 20) ? c.budget - held_other - (16ull << 20) : 0;
     blocks = static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>(blocks, room / per_block)));
     const auto [keys, changed] = pointwise_scratch(c, blocks);
@@ -1156,40 +1158,74 @@ uint64_t run_refine_pointwise(Context& c, const uint32_t* snap, const uint32_t* 
 
 namespace {
 
-// The large scratch of a pass, beside its snapshots (which the next pass looks
-// at).  A join takes up to all of the budget for it, so between passes it is
-// spare: whatever is allocated then, the finished lists for instance, may have
-// its room.
-constexpr const char* kPassScratch[] = {"refine_snap_d", "rev_count", "rev_cursor", "rev_offsets", "rev_ids",
-                                        "join_masks",    "apply_big", "apply_lost"};
-struct PassScratch {
+// The lists of a join pass, and what they take for n points, ranges of `step`.
+// A join takes up to all of the budget for them, so but during the pass they are
+// spare: whatever is allocated then, the finished lists or the next pass's
+// snapshot for instance, may have their room.
+struct PassLists {
+    static constexpr const char* kNames[] = {"refine_snap_d", "rev_count",  "rev_cursor", "rev_offsets",
+                                             "rev_ids",       "join_masks", "apply_big",  "apply_lost"};
     Context& c;
-    explicit PassScratch(Context& ctx) : c(ctx) { mark(false); }
-    ~PassScratch() { mark(true); }
-    void mark(bool spare) {
-        for (const char* name : kPassScratch) set_spare(c, name, spare);
-        set_spare(c, "refine_keys", spare);
+    explicit PassLists(Context& ctx) : c(ctx) {}
+    ~PassLists() {
+        mark(true);
+        set_spare(c, "refine_keys", true);
     }
+    void mark(bool spare) {
+        for (const char* name : kNames) set_spare(c, name, spare);
+    }
+    // Keeps those of the last pass that are large enough, unless (its ranges may
+    // have been larger) they would leave less than `reserve` of the budget.
+    void take(const uint64_t (&need)[std::size(kNames)], uint64_t reserve) {
+        mark(false);
+        uint64_t more = 0;
+        for (size_t i = 0; i < std::size(kNames); ++i)
+            if (scratch_bytes(c, kNames[i]) < need[i]) {
+                scratch_free(c, kNames[i]);
+                more += need[i];
+            }
+        if (c.held - spare_bytes(c) + more + reserve > c.budget)
+            for (const char* name : kNames) scratch_free(c, name);
+        for (size_t i = 0; i < std::size(kNames); ++i) ptr[i] = scratch(c, kNames[i], need[i]);
+    }
+    void* ptr[std::size(kNames)] = {};
 };
 
 }  // namespace
 
 uint64_t run_refine(Context& c) {
     if (c.n == 0) return 0;
-    PassScratch pass_scratch(c);
+    PassLists lists(c);
     const int K = static_cast<int>(c.k);
     const uint32_t n = c.n;
     const size_t entries = static_cast<size_t>(n) * K;
+    // Points a range of the join takes beside `more` bytes: their edges' bits (16
+    // bytes) and reverse entries (4) have to fit what the rest leaves of the
+    // budget, and edge numbers 31 bits.  The reserve holds the other scratch, the
+    // per-point pass's least among it.
+    const uint64_t fixed = entries * 4 + static_cast<uint64_t>(n) * 24;
+    const uint64_t reserve =
+        std::max<uint64_t>(std::min<uint64_t>(256ull << 20, c.budget / 8), pointwise_block_bytes(c) + (64u << 10));
+    auto fit_beside = [&](uint64_t more) {
+        const uint64_t used = c.held - spare_bytes(c) + more + fixed + reserve;
+        const uint64_t room = c.budget > used ? c.budget - used : 0;
+        return std::min<uint64_t>({n, room / (20ull * K), ((1ull << 31) - 1) / K});
+    };
+    // A budget without room for a 64th of the points leaves the pass to the
+    // per-point kernel.
+    const uint64_t fit_least = (n + 63) / 64;
     // The join skips pairs the previous join pass offered (both edges in that
     // pass's lists): the snapshot is made in one of two buffers in turn, the
     // other holding the previous pass's lists, and marks each entry that was
-    // already there.
+    // already there.  (Not where that would cost more than half a range.)
     const size_t old_bytes = static_cast<size_t>(n) * kOldWords * 4;
     static const char* const snap_names[2] = {"refine_snap", "refine_snap_other"};
     const char* other = snap_names[c.snap_flip ^ 1u];
     const uint64_t more = (scratch_bytes(c, other) >= entries * 4 ? 0 : entries * 4) +
                           (scratch_bytes(c, "refine_old") >= old_bytes ? 0 : old_bytes);
-    const bool marks = c.refine_mode == 0 && c.refine_skip_old && c.snap_prev_valid && c.held + more <= c.budget;
+    const bool marks = c.refine_mode == 0 && c.refine_skip_old && c.snap_prev_valid &&
+                       fit_beside(more) >= std::max(fit_least, fit_beside(0) / 2);
+    c.snap_prev_valid = false;  // valid again once this pass completes
     const uint32_t* prev = nullptr;
     uint32_t* old = nullptr;
     if (marks) {
@@ -1198,7 +1234,6 @@ uint64_t run_refine(Context& c) {
         c.snap_flip ^= 1u;
     }
     uint32_t* snap = static_cast<uint32_t*>(scratch(c, snap_names[c.snap_flip], entries * 4));
-    c.snap_prev_valid = false;  // valid again once this pass completes
     const uint32_t sblocks = std::min<uint32_t>((n + kSnapWarps - 1) / kSnapWarps, 148 * 8);
     auto snapshot = [&](float* snap_d) {
         auto kernel = n <= kShortIds ? k_snapshot<uint32_t> : k_snapshot<unsigned long long>;
@@ -1214,20 +1249,8 @@ uint64_t run_refine(Context& c) {
     };
     if (c.refine_mode == 1) return pointwise();
 
-    // Points a range of the join takes: their edges' bits (16 bytes) and
-    // reverse entries (4) have to fit what the rest leaves of the budget, and
-    // edge numbers 31 bits.  A budget without room for a 64th of the points
-    // leaves the pass to the per-point kernel.
-    const uint64_t fixed = entries * 4 + static_cast<uint64_t>(n) * 24;
-    uint64_t held_mine = 0;
-    for (const char* name : kPassScratch) held_mine += scratch_bytes(c, name);
-    // The reserve holds the other scratch, the per-point pass's least among it.
-    const uint64_t reserve =
-        std::max<uint64_t>(std::min<uint64_t>(256ull << 20, c.budget / 8), pointwise_block_bytes(c) + (64u << 10));
-    const uint64_t used = c.held - held_mine + fixed + reserve;
-    const uint64_t room = c.budget > used ? c.budget - used : 0;
-    const uint64_t fit = std::min<uint64_t>({n, room / (20ull * K), ((1ull << 31) - 1) / K});
-    if (fit < (n + 63) / 64) return pointwise();
+    const uint64_t fit = fit_beside(0);
+    if (fit < fit_least) return pointwise();
     const uint32_t rounds = static_cast<uint32_t>((n + fit - 1) / fit);
     const uint32_t step = (n + rounds - 1) / rounds;
 
@@ -1240,7 +1263,19 @@ uint64_t run_refine(Context& c) {
     cudaEvent_t ev[4];
     for (auto& e : ev) KNNG_CUDA(cudaEventCreate(&e));
     KNNG_CUDA(cudaEventRecord(ev[0], c.stream));
-    auto* snap_d = static_cast<float*>(scratch(c, "refine_snap_d", entries * sizeof(float)));
+    const uint64_t point = static_cast<uint64_t>(n) + 1, edges = static_cast<uint64_t>(step) * K;
+    lists.take({entries * sizeof(float), point * sizeof(uint32_t), point * sizeof(uint32_t),
+                point * sizeof(unsigned long long), edges * sizeof(uint32_t), edges * sizeof(uint4),
+                step * sizeof(uint32_t), step * sizeof(uint32_t)},
+               reserve);
+    auto* snap_d = static_cast<float*>(lists.ptr[0]);
+    auto* cnt = static_cast<uint32_t*>(lists.ptr[1]);
+    auto* cur = static_cast<uint32_t*>(lists.ptr[2]);
+    auto* off = static_cast<unsigned long long*>(lists.ptr[3]);
+    auto* rev = static_cast<uint32_t*>(lists.ptr[4]);
+    auto* masks = static_cast<uint4*>(lists.ptr[5]);
+    auto* big = static_cast<uint32_t*>(lists.ptr[6]);
+    auto* lost = static_cast<uint32_t*>(lists.ptr[7]);
     snapshot(c.dists_own ? snap_d : nullptr);
     if (!c.dists_own) {
         KNNG_DISPATCH_D(c.d, {
@@ -1249,14 +1284,6 @@ uint64_t run_refine(Context& c) {
         ++c.launches;
         KNNG_CUDA(cudaGetLastError());
     }
-    auto* cnt = static_cast<uint32_t*>(scratch(c, "rev_count", (static_cast<size_t>(n) + 1) * sizeof(uint32_t)));
-    auto* cur = static_cast<uint32_t*>(scratch(c, "rev_cursor", (static_cast<size_t>(n) + 1) * sizeof(uint32_t)));
-    auto* off = static_cast<unsigned long long*>(
-        scratch(c, "rev_offsets", (static_cast<size_t>(n) + 1) * sizeof(unsigned long long)));
-    auto* rev = static_cast<uint32_t*>(scratch(c, "rev_ids", static_cast<size_t>(step) * K * sizeof(uint32_t)));
-    auto* masks = static_cast<uint4*>(scratch(c, "join_masks", static_cast<size_t>(step) * K * sizeof(uint4)));
-    auto* big = static_cast<uint32_t*>(scratch(c, "apply_big", static_cast<size_t>(step) * sizeof(uint32_t)));
-    auto* lost = static_cast<uint32_t*>(scratch(c, "apply_lost", static_cast<size_t>(step) * sizeof(uint32_t)));
     // What the pass's kernels count, and its error word.
     struct Counts {
         unsigned long long join[5];  // pairs, filter-passing, members, exact distances, candidate records

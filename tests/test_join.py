@@ -99,6 +99,29 @@ def test_finished_lists_fit_whatever_the_passes_took(knng_lib, n, d, k, passes):
         assert np.array_equal(ids, want[0]) and np.array_equal(dists, want[1]), share
 
 
+@pytest.mark.parametrize("n,d,k,passes", [(20_000, 64, 10, 2), (12_000, 100, 60, 1), (12_000, 100, 60, 2)])
+def test_a_context_builds_again_under_any_budget(knng_lib, n, d, k, passes):
+    """The same builds three times on one context: what the earlier ones hold (the
+    finished lists, a pass's lists of other ranges) is in no later one's way."""
+    pts = workloads.gaussian_mixture(n=n, d=d, clusters=16, sigma=0.2, seed=n + k)
+    p = default_params(k=k, reps=1, refine=passes, max_leaf=257, max_leaf_odd=0, lloyd_iters=1, seed=5)
+    with KnngContext(0) as c:
+        want = c.build(pts, p, want_dists=True)
+    least = n * (4 * d + 8 + 8 * k + 12)  # points, order, sets
+    least += n * 64 + (4 << 20)           # a repetition's buffers, small scratch
+    least += n * 4 * k                    # a pass's snapshot
+    least += n * k * 8                    # the finished lists
+    joins = set()
+    for share in range(0, 40):
+        with KnngContext(0, least + n * k * share) as c:
+            for _ in range(3):
+                st = Stats()
+                ids, dists = c.build(pts, p, want_dists=True, stats=st)
+                assert np.array_equal(ids, want[0]) and np.array_equal(dists, want[1]), share
+                joins.add(int(st.refine_join_launches))
+    assert max(joins) > passes, joins  # ranges among them
+
+
 def test_distances_of_given_sets_do_not_steer_the_filter(knng_lib):
     """Sets handed over may hold any distances (here a thousandth of the real
     ones, with the real bounds): the filter's norms come from the points."""
