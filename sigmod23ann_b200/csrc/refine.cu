@@ -1196,6 +1196,7 @@ struct PassLists {
 uint64_t run_refine(Context& c) {
     if (c.n == 0) return 0;
     PassLists lists(c);
+    c.last_refine = {};  // a pass that goes point by point has no join to report
     const int K = static_cast<int>(c.k);
     const uint32_t n = c.n;
     const size_t entries = static_cast<size_t>(n) * K;

@@ -122,6 +122,39 @@ def test_a_context_builds_again_under_any_budget(knng_lib, n, d, k, passes):
     assert max(joins) > passes, joins  # ranges among them
 
 
+@pytest.mark.parametrize("n,d,k", [(12_000, 64, 50), (9_000, 100, 100)])
+def test_no_room_for_a_64th_goes_point_by_point(knng_lib, n, d, k):
+    """A budget with room for less than a 64th of the points' join beside its
+    reserve: the pass goes point by point, to the same sets, and reports no join,
+    also where the pass before it on that context had one."""
+    pts = workloads.gaussian_mixture(n=n, d=d, clusters=16, sigma=0.2, seed=8)
+    before = _sets_after_reps(pts, k, 129)
+    want, want_changed, _ = _pass_from(pts, k, before, pointwise=True)
+    held = n * (4 * d + 8 + 8 * k + 12)           # points, order, sets
+    lists = n * k * 8 + n * 24                    # snapshot, its distances; counts and offsets
+    edges = n * k * 20                            # a full range
+    for part, joins in ((100, 0), (2, None)):     # of the edges, beside an eighth in reserve
+        got, changed, st = _pass_from(pts, k, before, budget=(held + lists + edges // part) * 8 // 7)
+        assert_sets_equal(got, want, f"1/{part} of the edges")
+        assert changed == want_changed
+        assert st.refine_join_launches > 1 if joins is None else st.refine_join_launches == 0
+    # A pass with room, then one without: the finished lists are held by then.
+    want, want_changed, _ = _pass_from(pts, k, before, pointwise=True, passes=2)
+    with KnngContext(0, (held + lists + edges // 10) * 8 // 7) as c:
+        c.load_points(pts)
+        c.reset_sets(k)
+        c.set_sets(before)
+        first, second = Stats(), Stats()
+        changed = [c.refine(first)]
+        c.finalize(want_dists=True)
+        changed.append(c.refine(second))
+        assert_sets_equal(c.sets(), want, "with and without room")
+    assert changed == want_changed
+    assert first.refine_join_launches > 1
+    assert second.refine_join_launches == 0
+    assert second.refine_pairs == 0 and second.refine_exact == 0 and second.ms_refine_join == 0
+
+
 def test_distances_of_given_sets_do_not_steer_the_filter(knng_lib):
     """Sets handed over may hold any distances (here a thousandth of the real
     ones, with the real bounds): the filter's norms come from the points."""
