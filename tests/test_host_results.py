@@ -4,6 +4,7 @@ against the device-resident build's lists."""
 from __future__ import annotations
 
 import threading
+from concurrent.futures import ThreadPoolExecutor
 
 import numpy as np
 import pytest
@@ -57,3 +58,24 @@ def test_contexts_in_threads(knng_lib):
     for t in threads:
         t.join()
     assert not bad
+
+
+def test_every_thread_finishes_its_builds(knng_lib):
+    """Contexts in threads as above, with distances, each build's outcome looked at:
+    an error in a thread fails the test."""
+    sets = [workloads.gaussian_mixture(n=22_000 + 1000 * i, d=64, clusters=8, sigma=0.2, seed=i) for i in range(4)]
+    want = [_device_lists(p, 100) for p in sets]
+
+    def work(i: int) -> int:
+        done = 0
+        for _ in range(3):
+            with KnngContext(0, 4 << 30) as c:
+                for _ in range(2):
+                    ids, dist = c.build(sets[i], default_params(k=100, **PARAMS), want_dists=True)
+                    assert np.array_equal(ids, want[i][0]), i
+                    assert np.array_equal(dist.view(np.uint32), want[i][1].view(np.uint32)), i
+                    done += 1
+        return done
+
+    with ThreadPoolExecutor(4) as pool:
+        assert [f.result() for f in [pool.submit(work, i) for i in range(4)]] == [6] * 4
