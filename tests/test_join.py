@@ -155,6 +155,29 @@ def test_no_room_for_a_64th_goes_point_by_point(knng_lib, n, d, k):
     assert second.refine_pairs == 0 and second.refine_exact == 0 and second.ms_refine_join == 0
 
 
+@pytest.mark.parametrize("n,d,k", [(12_001, 64, 50), (9_000, 128, 100), (10_000, 100, 17)])
+def test_ranges_with_the_previous_lists(knng_lib, monkeypatch, n, d, k):
+    """Three passes in several ranges each, with room for the previous pass's lists:
+    later passes leave out the pairs those offered (edges marked as old in reverse
+    lists that start past the first point).  The sets and changes are those of the
+    per-point passes; with the marks switched off more pairs pass the filter."""
+    pts = workloads.gaussian_mixture(n=n, d=d, clusters=16, sigma=0.2, seed=14)
+    before = _sets_after_reps(pts, k, 129, reps=1)
+    want, want_changed, _ = _pass_from(pts, k, before, pointwise=True, passes=3)
+    need = n * (4 * d + 8 + 8 * k + 12) + n * k * 8 + n * 24  # points, order, sets; snapshot, distances, offsets
+    need += n * (4 * k + 16)                                  # the previous lists and the marks
+    need = (need + n * k * 20 * 2 // 5) * 8 // 7              # two fifths of the edges, an eighth in reserve
+    got, changed, st = _pass_from(pts, k, before, budget=need, passes=3)
+    assert_sets_equal(got, want, "in ranges")
+    assert changed == want_changed
+    assert st.refine_join_launches > 2 * 3
+    monkeypatch.setenv("KNNG_REFINE_SKIP", "0")
+    all_got, all_changed, all_st = _pass_from(pts, k, before, budget=need, passes=3)
+    assert_sets_equal(all_got, want, "every pair offered")
+    assert all_changed == want_changed
+    assert st.refine_filter_pass < 0.9 * all_st.refine_filter_pass
+
+
 def test_distances_of_given_sets_do_not_steer_the_filter(knng_lib):
     """Sets handed over may hold any distances (here a thousandth of the real
     ones, with the real bounds): the filter's norms come from the points."""
