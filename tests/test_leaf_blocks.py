@@ -44,6 +44,26 @@ def test_one_bucket(knng_lib, oracle_lib, n, d, k):
         assert_sets_equal(c.sets(), o, "handed over")
 
 
+# Column blocks of 128, and the mark window of 1,024 to the point; with blocks of
+# 16 rows here, and of 32 (other points in the set, in no bucket) below.
+@pytest.mark.parametrize("n", [127, 128, 129, 255, 256, 257, 1024, 1152, 1153, 2048])
+@pytest.mark.parametrize("d,k", [(64, 10), (100, 100), (128, 128)])
+def test_column_block_edges(knng_lib, oracle_lib, n, d, k):
+    pts = workloads.gaussian_mixture(n=n, d=d, clusters=4, sigma=0.2, seed=n + 1)
+    pts[50:60] = pts[40:50]  # equal distances: the update's tie order
+    o = _oracle_bucket_sets(oracle_lib, pts, k, 1)
+    rest = workloads.gaussian_mixture(n=9600, d=d, clusters=4, sigma=0.2, seed=n)
+    for held in (pts, np.concatenate([pts, rest])):
+        with KnngContext(0) as c:
+            c.load_points(held)
+            c.reset_sets(k)
+            for _ in range(2):  # the second pass meets every member again
+                c.begin_rep()
+                c.process_leaves([0], [n])
+                got = {key: v[:n] for key, v in c.sets().items()}
+                assert_sets_equal(got, o, f"n {n} d {d} k {k} of {len(held)}")
+
+
 def test_many_buckets_in_blocks_of_32_rows(knng_lib, oracle_lib):
     n, d, k = 12_000, 100, 100
     pts = workloads.gaussian_mixture(n=n, d=d, clusters=8, sigma=0.2, seed=3)
