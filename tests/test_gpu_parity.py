@@ -660,3 +660,40 @@ def test_build_kd_matches_oracle(oracle_lib, ctx):
         oids, odist = o.finalize()
         np.testing.assert_array_equal(ids, oids)
         np.testing.assert_array_equal(dist.view(np.uint32), odist.view(np.uint32))
+
+
+def test_timed_build_counts_the_upload(knng_lib):
+    """The wall-clock budget of knng_build_timed runs from the call's beginning: a
+    budget that the upload alone outlasts (rows far apart in pageable memory)
+    gives one repetition, though several would fit into it."""
+    import ctypes
+    import time
+
+    from sigmod23ann_b200.api import Stats
+
+    n, d = 300_000, 100
+    rows = np.zeros((n, 1024), np.float32)
+    rows[:, :d] = workloads.gaussian_mixture(n=n, d=d, clusters=16, sigma=0.2, seed=6)
+    at = rows.ctypes.data_as(ctypes.c_void_p)
+    ids = np.empty((n, 1), np.uint32)
+    with KnngContext(0) as ctx:
+        def upload() -> float:
+            t = time.perf_counter()
+            assert knng_lib.knng_load_points(ctx._h, at, n, d, rows.strides[0], 0) == 0
+            return (time.perf_counter() - t) * 1e3
+
+        def repetitions(build_ms: int) -> int:
+            st = Stats()
+            p = default_params(k=1, reps=0, refine=0, max_leaf=1025, max_leaf_odd=0, lloyd_iters=1, seed=1)
+            assert knng_lib.knng_build_timed(ctx._h, at, n, d, rows.strides[0], ctypes.byref(p), build_ms, 0,
+                                             ids.ctypes.data_as(ctypes.c_void_p), None, ctypes.byref(st)) == 0
+            return int(st.reps_done)
+
+        repetitions(1)  # buffers and the graph are there
+        budget = int(0.6 * min(upload() for _ in range(3)))
+        t = time.perf_counter()
+        many = repetitions(1000)
+        each = (time.perf_counter() - t) * 1e3 / many
+        if budget < 2 * each:
+            pytest.skip(f"an upload of {budget / 0.6:.1f} ms against repetitions of {each:.1f} ms tells nothing")
+        assert repetitions(budget) == 1
