@@ -670,7 +670,7 @@ void run_rep(Context& c, uint32_t max_leaf, uint32_t lloyd_iters, uint32_t small
     if (precision == KNNG_PRECISION_BF16_RERANK)
         launch_leaves_bf16(c, nl, d_ls, d_le, max_bucket);
     else
-        launch_leaves(c, nl, d_ls, d_le, max_bucket, nullptr);
+        launch_leaves(c, nl, d_ls, d_le, max_bucket);
     const double leaf_ms = leaf_t.stop(c);
     st.ms_leaf += leaf_ms;
     if (stats) {
@@ -1088,7 +1088,7 @@ knng_status knng_process_leaves(knng_context* ctx, uint32_t count, const uint32_
             if (order[i].first < order[i - 1].second) knng::fail(KNNG_ERR_INVALID_ARGUMENT, "buckets overlap");
         uint32_t* d_s = knng::upload(c, "pl_start", starts, count);
         uint32_t* d_e = knng::upload(c, "pl_end", ends, count);
-        knng::launch_leaves(c, count, d_s, d_e, max_bucket, nullptr);
+        knng::launch_leaves(c, count, d_s, d_e, max_bucket);
         KNNG_CUDA(cudaStreamSynchronize(c.stream));
     });
 }

@@ -1,6 +1,6 @@
 // Device-side building blocks shared by the k-NN graph kernels.
 //
-//  * canonical_distance / canonical_dot: the reference's FP32 evaluation order
+//  * canonical_distance4 / canonical_dot: the reference's FP32 evaluation order
 //    (src/LinearAlgebra.hpp:53-77 and :179-200): eight lanes, lane l an FMA
 //    chain over dims l, l+8, ... below the largest multiple of 8 <= D, lanes
 //    summed left to right into 0.0f, then each tail dim added as a separately
@@ -27,31 +27,6 @@ constexpr unsigned kFull = 0xFFFFFFFFu;
 // ---------------------------------------------------------------- arithmetic
 
 template <int D>
-__device__ __forceinline__ float canonical_distance(const float* __restrict__ a, const float* __restrict__ b) {
-    constexpr int M = D / 8 * 8;
-    float lane[8];
-#pragma unroll
-    for (int l = 0; l < 8; ++l) lane[l] = 0.0f;
-#pragma unroll
-    for (int base = 0; base < M; base += 8) {
-#pragma unroll
-        for (int l = 0; l < 8; ++l) {
-            float diff = __fsub_rn(a[base + l], b[base + l]);
-            lane[l] = __fmaf_rn(diff, diff, lane[l]);
-        }
-    }
-    float acc = 0.0f;
-#pragma unroll
-    for (int l = 0; l < 8; ++l) acc = __fadd_rn(acc, lane[l]);
-#pragma unroll
-    for (int i = M; i < D; ++i) {
-        float diff = __fsub_rn(a[i], b[i]);
-        acc = __fadd_rn(acc, __fmul_rn(diff, diff));
-    }
-    return acc;
-}
-
-template <int D>
 __device__ __forceinline__ float canonical_dot(const float* __restrict__ a, const float* __restrict__ b) {
     constexpr int M = D / 8 * 8;
     float lane[8];
@@ -70,39 +45,7 @@ __device__ __forceinline__ float canonical_dot(const float* __restrict__ a, cons
     return acc;
 }
 
-// Same order, operands read as float4 (both rows 16-byte aligned, D % 4 == 0).
-template <int D>
-__device__ __forceinline__ float canonical_dot4(const float4* __restrict__ a, const float4* __restrict__ b) {
-    static_assert(D % 4 == 0, "float4 path needs D % 4 == 0");
-    constexpr int M = D / 8 * 8;
-    float lane[8];
-#pragma unroll
-    for (int l = 0; l < 8; ++l) lane[l] = 0.0f;
-#pragma unroll
-    for (int q = 0; q < M / 4; ++q) {
-        float4 x = a[q];
-        float4 y = b[q];
-        const int l0 = (q & 1) * 4;
-        lane[l0 + 0] = __fmaf_rn(y.x, x.x, lane[l0 + 0]);
-        lane[l0 + 1] = __fmaf_rn(y.y, x.y, lane[l0 + 1]);
-        lane[l0 + 2] = __fmaf_rn(y.z, x.z, lane[l0 + 2]);
-        lane[l0 + 3] = __fmaf_rn(y.w, x.w, lane[l0 + 3]);
-    }
-    float acc = 0.0f;
-#pragma unroll
-    for (int l = 0; l < 8; ++l) acc = __fadd_rn(acc, lane[l]);
-#pragma unroll
-    for (int q = M / 4; q < D / 4; ++q) {
-        float4 x = a[q];
-        float4 y = b[q];
-        acc = __fadd_rn(acc, __fmul_rn(x.x, y.x));
-        acc = __fadd_rn(acc, __fmul_rn(x.y, y.y));
-        acc = __fadd_rn(acc, __fmul_rn(x.z, y.z));
-        acc = __fadd_rn(acc, __fmul_rn(x.w, y.w));
-    }
-    return acc;
-}
-
+// Rows read as float4 (16-byte aligned, D % 4 == 0).
 template <int D>
 __device__ __forceinline__ float canonical_distance4(const float4* __restrict__ a, const float4* __restrict__ b) {
     static_assert(D % 4 == 0, "float4 path needs D % 4 == 0");
@@ -128,45 +71,6 @@ __device__ __forceinline__ float canonical_distance4(const float4* __restrict__ 
     for (int q = M / 4; q < D / 4; ++q) {
         float4 x = a[q];
         float4 y = b[q];
-        float d0 = __fsub_rn(x.x, y.x), d1 = __fsub_rn(x.y, y.y), d2 = __fsub_rn(x.z, y.z), d3 = __fsub_rn(x.w, y.w);
-        acc = __fadd_rn(acc, __fmul_rn(d0, d0));
-        acc = __fadd_rn(acc, __fmul_rn(d1, d1));
-        acc = __fadd_rn(acc, __fmul_rn(d2, d2));
-        acc = __fadd_rn(acc, __fmul_rn(d3, d3));
-    }
-    return acc;
-}
-
-// The same order as canonical_distance4, one 8-dimension step at a time
-// (four float4 loads live per step): for callers with little register room.
-template <int D>
-__device__ __forceinline__ float canonical_distance4_lean(const float4* __restrict__ a, const float4* __restrict__ b) {
-    static_assert(D % 4 == 0, "float4 path needs D % 4 == 0");
-    constexpr int M = D / 8 * 8;
-    float lane[8];
-#pragma unroll
-    for (int l = 0; l < 8; ++l) lane[l] = 0.0f;
-#pragma unroll 1
-    for (int q = 0; q < M / 4; q += 2) {
-        const float4 x0 = a[q], x1 = a[q + 1];
-        const float4 y0 = b[q], y1 = b[q + 1];
-        float d;
-        d = __fsub_rn(x0.x, y0.x); lane[0] = __fmaf_rn(d, d, lane[0]);
-        d = __fsub_rn(x0.y, y0.y); lane[1] = __fmaf_rn(d, d, lane[1]);
-        d = __fsub_rn(x0.z, y0.z); lane[2] = __fmaf_rn(d, d, lane[2]);
-        d = __fsub_rn(x0.w, y0.w); lane[3] = __fmaf_rn(d, d, lane[3]);
-        d = __fsub_rn(x1.x, y1.x); lane[4] = __fmaf_rn(d, d, lane[4]);
-        d = __fsub_rn(x1.y, y1.y); lane[5] = __fmaf_rn(d, d, lane[5]);
-        d = __fsub_rn(x1.z, y1.z); lane[6] = __fmaf_rn(d, d, lane[6]);
-        d = __fsub_rn(x1.w, y1.w); lane[7] = __fmaf_rn(d, d, lane[7]);
-    }
-    float acc = 0.0f;
-#pragma unroll
-    for (int l = 0; l < 8; ++l) acc = __fadd_rn(acc, lane[l]);
-#pragma unroll
-    for (int q = M / 4; q < D / 4; ++q) {
-        const float4 x = a[q];
-        const float4 y = b[q];
         float d0 = __fsub_rn(x.x, y.x), d1 = __fsub_rn(x.y, y.y), d2 = __fsub_rn(x.z, y.z), d3 = __fsub_rn(x.w, y.w);
         acc = __fadd_rn(acc, __fmul_rn(d0, d0));
         acc = __fadd_rn(acc, __fmul_rn(d1, d1));
@@ -204,7 +108,7 @@ __device__ __forceinline__ float load_now(const float* p) {
     return v;
 }
 
-// canonical_distance of `mine` (p's row) and the rows of 32 points, lane t's
+// canonical_distance4 of `mine` (p's row) and the rows of 32 points, lane t's
 // point id t; every lane returns its own.  A group of eight lanes reads its
 // eight rows one after the other, a lane a chain (32 bytes of each row a load);
 // the chains are then exchanged within the group, so that each lane sums the

@@ -273,7 +273,7 @@ uint32_t sample_count(uint32_t n);
 uint32_t start_count(uint32_t n);
 // leaf.cu
 void launch_leaves(Context& c, uint32_t count, const uint32_t* d_starts, const uint32_t* d_ends,
-                   uint32_t max_bucket, uint64_t* evals);
+                   uint32_t max_bucket);
 // Work items of a bucket pass, row blocks: item i is rows from row[-i] on of
 // bucket leaf[-i], both arrays written from their last entry downwards.  So
 // they fit behind the bucket list itself, in arrays of one entry per point and

@@ -455,7 +455,7 @@ void run_rep_kd(Context& c, uint32_t max_leaf, uint32_t new_dims, uint64_t seed,
     if (nl > 0) {
         uint32_t* d_ls = upload(c, "kd_leaf_start", leaf_start.data(), nl);
         uint32_t* d_le = upload(c, "kd_leaf_end", leaf_end.data(), nl);
-        launch_leaves(c, nl, d_ls, d_le, max_bucket, nullptr);
+        launch_leaves(c, nl, d_ls, d_le, max_bucket);
     }
     KNNG_CUDA(cudaEventRecord(ev[2], c.stream));
     KNNG_CUDA(cudaEventSynchronize(ev[2]));

@@ -856,9 +856,8 @@ void enqueue_leaves(Context& c, uint32_t count, const uint32_t* d_starts, const 
 }  // namespace
 
 void launch_leaves(Context& c, uint32_t count, const uint32_t* d_starts, const uint32_t* d_ends,
-                   uint32_t max_bucket, uint64_t* evals) {
+                   uint32_t max_bucket) {
     if (count == 0) return;
-    (void)evals;
     if (c.leaf_tc) {
         auto* err = static_cast<uint32_t*>(scratch(c, "leaf_error", sizeof(uint32_t)));
         KNNG_CUDA(cudaMemsetAsync(err, 0, sizeof(uint32_t), c.stream));

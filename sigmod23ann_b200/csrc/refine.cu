@@ -675,7 +675,7 @@ __device__ __forceinline__ uint32_t table_insert(uint32_t* table, uint32_t bucke
     return 0u;
 }
 
-// canonical_distance of two rows held by the eight lanes of the group whose
+// canonical_distance4 of two rows held by the eight lanes of the group whose
 // first lane is g0; every lane of the group returns it.  All 32 lanes call it.
 template <int D>
 __device__ __forceinline__ float group_distance(const ChainRow<D>& a, const ChainRow<D>& b, int g0) {
