@@ -557,8 +557,11 @@ __global__ void __launch_bounds__(kSeqThreads)
         uint32_t cnt = 0;
         for (uint32_t t = 0; t < ntiles; ++t, ++g) {
             const uint32_t s = g % S;
-            if (!__all_sync(kFull, tc::mbar_wait_limited(&full[s], (g / S) & 1u))) {  // as one, like the copiers
-                if (lane == 0) atomicExch(error_flag, 1);
+            // A lane that gives up says so and exits.  What follows takes no value from
+            // another lane, only barriers of the warp, which pass over exited lanes
+            // (a vote, as the copiers have, would be on the chain of adds).
+            if (!tc::mbar_wait_limited(&full[s], (g / S) & 1u)) {
+                atomicExch(error_flag, 1);
                 return;
             }
             const uint32_t mine = counts[s][side];
@@ -1072,9 +1075,8 @@ void launch_lloyd(Context& c, uint32_t count, const uint32_t* h_starts, const ui
                   uint32_t iters, float* d_coefs, float* d_offsets, int32_t* d_ok) {
     if (count == 0) return;
     // Each node's Lloyd set is its list (large nodes) or its whole range
-    // (small nodes).  Its entries get a 16-byte aligned block of the flag / id
-    // arrays (the bulk copies of the sums kernel read whole 16-byte pieces),
-    // and are cut into kChunk-entry items for the side kernel.
+    // (small nodes).  Its entries get a block of the flag / id arrays and are cut
+    // into kChunk-entry items for the side kernel.
     std::vector<Item> items;
     std::vector<SeqNode> nodes(count);
     uint64_t fnext = 0;
@@ -1526,7 +1528,7 @@ void run_rep_device(Context& c, uint32_t max_leaf, uint32_t lloyd_iters, uint32_
     if (graph) c.launches += 2 + bucket_kernels + static_cast<uint64_t>(h.iterations) * (kLevelLaunches + 2 * lloyd_iters);
     int32_t err[4] = {0, 0, 0, 0};
     download(c, err, r.error, 4);
-    if (err[0]) fail(KNNG_ERR_CUDA, "Lloyd sums: a bulk-copy wait gave up");
+    if (err[0]) fail(KNNG_ERR_CUDA, "Lloyd sums: a copy wait gave up");
     if (err[1]) fail(KNNG_ERR_CUDA, "bucket pass: the MMA completion wait gave up");
     if (err[2]) fail(KNNG_ERR_CUDA, "tree levels: the level loop ran past its iteration limit");
     out.leaf_start.resize(h.leaves);
