@@ -303,7 +303,7 @@ knng_status knng_debug_tile_gram_bf16(knng_context* ctx, const float* a, uint32_
                                       uint32_t d, float* out);
 
 /* Poll limit of the waits the tree-construction and refinement kernels make
- * on their own bulk copies and tensor-core operations, on the context's device
+ * on their own copies and tensor-core operations, on the context's device
  * (default 2^26 polls).  After a wait runs out the kernel records the failure,
  * drains its copies in flight with the default limit and returns; the call
  * reports KNNG_ERR_CUDA and the context stays usable.  A test sets a limit of

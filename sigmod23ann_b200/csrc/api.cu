@@ -48,24 +48,13 @@ void check_cuda(cudaError_t e, const char* what) {
 
 bool dim_supported(uint32_t d) { return d == 64 || d == 100 || d == 128; }
 
-namespace {
-void free_buffer(Context& c, DeviceBuffer& b) {
-    dev_free(c, b.ptr, b.bytes);
-    b.ptr = nullptr;
-    b.bytes = 0;
-}
-}  // namespace
-
 // Device memory is stream-ordered on the context's stream (all of the
 // context's work runs there), so allocating or freeing does not synchronise
 // the device under other contexts' work.
 void* dev_alloc(Context& c, size_t bytes) {
     if (bytes == 0) bytes = 16;
-    if (c.held + bytes > c.budget) {  // the spare scratch gives way
-        for (auto& e : c.scratch) {
-            if (e.second.spare && c.held + bytes > c.budget) free_buffer(c, e.second);
-        }
-    }
+    for (int i = 0; i < kSpareCount && c.held + bytes > c.budget; ++i)
+        if (!((c.spare_in_use >> i) & 1u)) spare_free(c, static_cast<SpareBuffer>(i));
     if (c.held + bytes > c.budget) fail(KNNG_ERR_BUDGET, "device memory budget exceeded");
     void* p = nullptr;
     check_cuda(cudaMallocAsync(&p, bytes, c.stream), "cudaMallocAsync");
@@ -86,7 +75,9 @@ void* scratch(Context& c, const char* name, size_t bytes) {
             KNNG_CUDA(cudaStreamSynchronize(c.stream));
             size_t grown = std::max(bytes, e.second.bytes * 3 / 2);
             if (c.held - e.second.bytes + grown > c.budget) grown = bytes;
-            free_buffer(c, e.second);
+            dev_free(c, e.second.ptr, e.second.bytes);
+            e.second.ptr = nullptr;
+            e.second.bytes = 0;
             e.second.ptr = dev_alloc(c, grown);
             e.second.bytes = grown;
             return e.second.ptr;
@@ -99,27 +90,32 @@ void* scratch(Context& c, const char* name, size_t bytes) {
     return b.ptr;
 }
 
-void* spare_scratch(Context& c, const char* name, size_t bytes) {
-    if (scratch_bytes(c, name) < bytes && c.held - scratch_bytes(c, name) + bytes > c.budget) return nullptr;
-    void* p = scratch(c, name, bytes);
-    set_spare(c, name, true);
-    return p;
+void* spare_take(Context& c, SpareBuffer which, size_t bytes) {
+    DeviceBuffer& b = c.spare[which];
+    if (b.bytes < bytes) {
+        spare_free(c, which);
+        b.ptr = dev_alloc(c, bytes);
+        b.bytes = bytes;
+    }
+    c.spare_in_use |= 1u << which;
+    return b.ptr;
 }
 
-void set_spare(Context& c, const char* name, bool spare) {
-    for (auto& e : c.scratch)
-        if (e.first == name) e.second.spare = spare;
+void spare_done(Context& c, SpareBuffer first, SpareBuffer last) {
+    for (int i = first; i <= last; ++i) c.spare_in_use &= ~(1u << i);
+}
+
+void spare_free(Context& c, SpareBuffer which) {
+    DeviceBuffer& b = c.spare[which];
+    dev_free(c, b.ptr, b.bytes);
+    b = {};
+    c.spare_in_use &= ~(1u << which);
 }
 
 uint64_t spare_bytes(const Context& c) {
     uint64_t bytes = 0;
-    for (const auto& e : c.scratch) bytes += e.second.spare ? e.second.bytes : 0;
+    for (int i = 0; i < kSpareCount; ++i) bytes += (c.spare_in_use >> i) & 1u ? 0 : c.spare[i].bytes;
     return bytes;
-}
-
-void scratch_free(Context& c, const char* name) {
-    for (auto& e : c.scratch)
-        if (e.first == name) free_buffer(c, e.second);
 }
 
 // --------------------------------------------------------------- sizing rules
@@ -360,6 +356,7 @@ void release_all(Context& c) {
     c.indices = c.indices_tmp = nullptr;
     for (auto& e : c.scratch) dev_free(c, e.second.ptr, e.second.bytes);
     c.scratch.clear();
+    for (int i = 0; i < kSpareCount; ++i) spare_free(c, static_cast<SpareBuffer>(i));
     c.n = 0;
 }
 
@@ -543,7 +540,7 @@ std::vector<uint32_t> split_level(Context& c, const std::vector<Node>& active, u
         launch_lloyd(c, cnt, hs.data(), he.data(), lloyd_off.data(), lloyd, c1, c2, lloyd_iters, coefs, offs, ok);
         std::vector<int32_t> hok(cnt + 1);
         download(c, hok.data(), ok, cnt + 1);
-        if (hok[cnt]) fail(KNNG_ERR_CUDA, "Lloyd sums: a bulk-copy wait gave up");
+        if (hok[cnt]) fail(KNNG_ERR_CUDA, "Lloyd sums: a copy wait gave up");
         // Partition the nodes that seeded and converged.
         std::vector<uint32_t> sel;
         for (uint32_t t = 0; t < cnt; ++t) {
@@ -1065,7 +1062,7 @@ knng_status knng_lloyd(knng_context* ctx, uint32_t count, const uint32_t* starts
         knng::download(c, out_offsets, d_offs, count);
         std::vector<int32_t> hok(count + 1);
         knng::download(c, hok.data(), d_ok, count + 1);
-        if (hok[count]) knng::fail(KNNG_ERR_CUDA, "Lloyd sums: a bulk-copy wait gave up");
+        if (hok[count]) knng::fail(KNNG_ERR_CUDA, "Lloyd sums: a copy wait gave up");
         std::memcpy(out_ok, hok.data(), count * sizeof(int32_t));
     });
 }

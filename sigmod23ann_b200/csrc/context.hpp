@@ -27,7 +27,25 @@ void check_cuda(cudaError_t e, const char* what);
 struct DeviceBuffer {
     void* ptr = nullptr;
     size_t bytes = 0;
-    bool spare = false;  // given back when another allocation needs the room
+};
+
+// Memory that a context keeps from call to call but can do without: a call takes
+// what it needs of it, and outside such a call it gives way to any allocation
+// that the budget has no other room for.
+enum SpareBuffer {
+    kSpareLeafLists,  // work items of a bucket pass over a host list (and norms)
+    // A join pass: list distances, counts, cursors and offsets of the reverse
+    // lists, these, the edges' bits, the queues of the replay.
+    kSpareSnapD,
+    kSpareRevCount,
+    kSpareRevCursor,
+    kSpareRevOffsets,
+    kSpareRevIds,
+    kSpareMasks,
+    kSpareBig,
+    kSpareLost,
+    kSpareKeys,  // the per-point pass's survivors
+    kSpareCount
 };
 
 struct Timer {
@@ -71,6 +89,8 @@ struct Context {
 
     // Named scratch allocations, grown on demand and reused across calls.
     std::vector<std::pair<std::string, DeviceBuffer>> scratch;
+    DeviceBuffer spare[kSpareCount];
+    uint32_t spare_in_use = 0;  // bit per buffer
 
     uint64_t launches = 0;
 
@@ -139,15 +159,12 @@ struct Context {
 void* dev_alloc(Context& c, size_t bytes);
 void dev_free(Context& c, void* p, size_t bytes);
 void* scratch(Context& c, const char* name, size_t bytes);
-// Scratch that a call can do without: null when the budget has no room for it.
-// It holds until the next allocation at most, which may take its room.
-void* spare_scratch(Context& c, const char* name, size_t bytes);
-// Marks the named scratch as spare, or as needed again.
-void set_spare(Context& c, const char* name, bool spare);
-// Bytes that spare scratch holds.
+// At least `bytes` of a spare buffer, in use until spare_done.
+void* spare_take(Context& c, SpareBuffer which, size_t bytes);
+void spare_done(Context& c, SpareBuffer first, SpareBuffer last);
+void spare_free(Context& c, SpareBuffer which);
+// Bytes held by the spare buffers that are not in use.
 uint64_t spare_bytes(const Context& c);
-// Frees the named scratch.
-void scratch_free(Context& c, const char* name);
 // Bytes currently held by the named scratch allocation (0 if none).
 size_t scratch_bytes(const Context& c, const char* name);
 void release_all(Context& c);

@@ -216,9 +216,9 @@ __global__ void k_leaf_items(const uint32_t* starts, const uint32_t* ends, uint3
 }
 
 // A persistent grid takes row blocks of P * 16 rows (P rows a warp) from the
-// work counter.  Without a list of them (items.leaf null: a budget too small for
-// one) the grid has a CTA for every (bucket of `count`, block of the largest
-// bucket), and those past their bucket's end return at once.
+// work counter.  Without a list of them (kList false: a budget too small for one)
+// the grid has a CTA for every (bucket of `count`, block of the largest bucket),
+// and those past their bucket's end return at once.
 //
 // kOwn: the sets hold distances of these points.  A set's members are then
 // left out of its offers, marked beforehand by their bucket positions (`pos`):
@@ -235,13 +235,14 @@ __global__ void k_leaf_items(const uint32_t* starts, const uint32_t* ends, uint3
 // repetitions): 106 ms, from 189 with a CTA per bucket, the check in every
 // offer and one column an instruction; 125 with blocks of 32 x 64 and a row by
 // four columns a thread.
-template <int D, int P, bool kOwn>
+template <int D, int P, bool kOwn, bool kList>
 __global__ void __launch_bounds__(kLeafThreads, 2)
     k_leaf(const uint32_t* __restrict__ starts, const uint32_t* __restrict__ ends, const uint32_t* __restrict__ idx,
            const uint32_t* __restrict__ pos, const float* __restrict__ pts, int ld, float* __restrict__ set_dist,
            uint32_t* __restrict__ set_id, uint32_t* __restrict__ set_size, uint32_t* __restrict__ set_maxslot,
-           float* __restrict__ set_bound, int K, LeafItems items, const uint32_t* __restrict__ n_items,
-           uint32_t* __restrict__ work, uint32_t count) {
+           float* __restrict__ set_bound, int K, const uint32_t* __restrict__ item_leaf,
+           const uint32_t* __restrict__ item_row, const uint32_t* __restrict__ n_items, uint32_t* __restrict__ work,
+           uint32_t count) {
     constexpr int R = P * kLeafWarps;
     extern __shared__ float4 smem4[];
     float* I = reinterpret_cast<float*>(smem4);
@@ -252,22 +253,22 @@ __global__ void __launch_bounds__(kLeafThreads, 2)
     __shared__ uint32_t next_s;
     __shared__ uint8_t place_s[kLeafWarps][kWarp];
     const int lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
-    const uint32_t total = items.leaf ? *n_items : 0u;
+    const uint32_t total = kList ? *n_items : 0u;
     for (;;) {
         uint32_t leaf, ib;
-        if (items.leaf) {
+        if constexpr (kList) {
             if (threadIdx.x == 0) next_s = atomicAdd(work, 1u);
             __syncthreads();
             const int64_t w = next_s;
             if (w >= total) break;
-            leaf = items.leaf[-w];
-            ib = items.row[-w];
+            leaf = item_leaf[-w];
+            ib = item_row[-w];
         } else {
             leaf = blockIdx.x % count;
             ib = blockIdx.x / count * R;
         }
         const uint32_t s = starts[leaf], b = ends[leaf] - s;
-        if (ib >= b || b < 2) break;  // only without a list
+        if (!kList && (ib >= b || b < 2)) break;
         for (uint32_t t = threadIdx.x; t < b; t += kLeafThreads) ids[t] = idx[s + t];
         __syncthreads();
         fill_tile<D, R, true>(I, pts, ld, b - ib, [&](uint32_t r) { return ids[ib + r]; });
@@ -329,7 +330,7 @@ __global__ void __launch_bounds__(kLeafThreads, 2)
             const uint32_t p = ib + warp * P + u;
             if (p < b) set_store(sets[u], set_dist, set_id, set_size, set_maxslot, set_bound, ids[p], K, lane);
         }
-        if (!items.leaf) break;
+        if constexpr (!kList) break;
         __syncthreads();  // everyone is done with ids, I and the work word
     }
 }
@@ -832,13 +833,15 @@ void enqueue_leaves(Context& c, uint32_t count, const uint32_t* d_starts, const 
                             static_cast<size_t>(rows) * kMarkWords * sizeof(uint32_t) +
                             static_cast<size_t>(std::max<uint32_t>(max_bucket, 1)) * sizeof(uint32_t);
         if (smem > 227 * 1024) fail(KNNG_ERR_INVALID_ARGUMENT, "bucket too large for the bucket kernel");
-        auto kern = rows == kLeafWarps ? (c.dists_own ? k_leaf<D, 1, true> : k_leaf<D, 1, false>)
-                                       : (c.dists_own ? k_leaf<D, 2, true> : k_leaf<D, 2, false>);
+        auto kern = items.leaf ? rows == kLeafWarps ? (c.dists_own ? k_leaf<D, 1, true, true> : k_leaf<D, 1, false, true>)
+                                                    : (c.dists_own ? k_leaf<D, 2, true, true> : k_leaf<D, 2, false, true>)
+                    : rows == kLeafWarps ? (c.dists_own ? k_leaf<D, 1, true, false> : k_leaf<D, 1, false, false>)
+                                         : (c.dists_own ? k_leaf<D, 2, true, false> : k_leaf<D, 2, false, false>);
         allow_max_smem(c, kern);
         auto run = [&](uint32_t grid, uint32_t first, uint32_t buckets) {
             kern<<<grid, kLeafThreads, smem, c.stream>>>(
                 d_starts + first, d_ends + first, c.indices, pos, c.points, c.ld, c.set_dist, c.set_id, c.set_size,
-                c.set_maxslot, c.set_bound, static_cast<int>(c.k), items, n_items, work, buckets);
+                c.set_maxslot, c.set_bound, static_cast<int>(c.k), items.leaf, items.row, n_items, work, buckets);
             ++c.launches;
         };
         if (items.leaf) {
@@ -878,13 +881,16 @@ void launch_leaves(Context& c, uint32_t count, const uint32_t* d_starts, const u
         return;
     }
     // Two counters and the row blocks, at most one more than n / rows of each
-    // bucket.  A budget without room for them runs the pass without a list.
-    const size_t cap = c.n / leaf_rows(c) + static_cast<size_t>(count) + 1;
-    auto* lists = static_cast<uint32_t*>(spare_scratch(c, "leaf_items", (2 + 2 * cap) * sizeof(uint32_t)));
-    if (!lists) {
+    // bucket (and to a whole 1,024, for the next list that is a little longer).  A
+    // budget without room for them runs the pass without a list.
+    const size_t cap = (c.n / leaf_rows(c) + static_cast<size_t>(count) + 1024) / 1024 * 1024;
+    const size_t bytes = (2 + 2 * cap) * sizeof(uint32_t);
+    if (c.held - spare_bytes(c) + bytes > c.budget) {
         enqueue_leaves(c, count, d_starts, d_ends, nullptr, {}, nullptr, nullptr, max_bucket);
         return;
     }
+    auto* lists = static_cast<uint32_t*>(spare_take(c, kSpareLeafLists, bytes));
+    spare_done(c, kSpareLeafLists, kSpareLeafLists);  // stream-ordered: the pass is in front of what takes its room
     KNNG_CUDA(cudaMemsetAsync(lists, 0, 2 * sizeof(uint32_t), c.stream));
     const LeafItems items{lists + 1 + cap, lists + 1 + 2 * cap};
     enqueue_leaves(c, count, d_starts, d_ends, nullptr, items, lists, lists + 1, max_bucket);
@@ -892,10 +898,10 @@ void launch_leaves(Context& c, uint32_t count, const uint32_t* d_starts, const u
 
 void prepare_leaves_list(Context& c) {
     KNNG_DISPATCH_D(c.d, {
-        allow_max_smem(c, k_leaf<D, 1, true>);
-        allow_max_smem(c, k_leaf<D, 2, true>);
-        allow_max_smem(c, k_leaf<D, 1, false>);
-        allow_max_smem(c, k_leaf<D, 2, false>);
+        allow_max_smem(c, k_leaf<D, 1, true, true>);
+        allow_max_smem(c, k_leaf<D, 2, true, true>);
+        allow_max_smem(c, k_leaf<D, 1, false, true>);
+        allow_max_smem(c, k_leaf<D, 2, false, true>);
         allow_max_smem(c, k_leaf_tc<D>);
     });
 }

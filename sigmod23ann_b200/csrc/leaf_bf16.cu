@@ -480,8 +480,8 @@ void launch_leaves_bf16(Context& c, uint32_t count, const uint32_t* d_starts, co
         fail(KNNG_ERR_INVALID_ARGUMENT, "the BF16 bucket pass takes buckets of at most 1024 points");
     // Item count, work counter, error word; the items; the norms.
     const size_t cap = c.n / kBfRows + static_cast<size_t>(count) + 1;
-    auto* lists = static_cast<uint32_t*>(spare_scratch(c, "bf16_lists", (3 + 2 * cap + c.n) * sizeof(uint32_t)));
-    if (!lists) fail(KNNG_ERR_BUDGET, "device memory budget exceeded");
+    auto* lists = static_cast<uint32_t*>(spare_take(c, kSpareLeafLists, (3 + 2 * cap + c.n) * sizeof(uint32_t)));
+    spare_done(c, kSpareLeafLists, kSpareLeafLists);  // nothing is allocated before the pass is on the stream
     KNNG_CUDA(cudaMemsetAsync(lists, 0, 3 * sizeof(uint32_t), c.stream));
     enqueue_bf16(c, count, d_starts, d_ends, nullptr, {lists + 2 + cap, lists + 2 + 2 * cap}, lists, lists + 1,
                  reinterpret_cast<float*>(lists + 3 + 2 * cap), lists + 2);

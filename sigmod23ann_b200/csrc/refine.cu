@@ -1122,9 +1122,8 @@ struct PointwiseScratch {
     uint32_t* changed;
 };
 PointwiseScratch pointwise_scratch(Context& c, uint32_t blocks) {
-    auto* keys = static_cast<unsigned long long*>(scratch(c, "refine_keys", blocks * pointwise_block_bytes(c)));
-    set_spare(c, "refine_keys", false);
-    return {keys, static_cast<uint32_t*>(scratch(c, "refine_changed", sizeof(uint32_t)))};
+    return {static_cast<unsigned long long*>(spare_take(c, kSpareKeys, blocks * pointwise_block_bytes(c))),
+            static_cast<uint32_t*>(scratch(c, "refine_changed", sizeof(uint32_t)))};
 }
 
 }  // namespace
@@ -1138,8 +1137,8 @@ uint64_t run_refine_pointwise(Context& c, const uint32_t* snap, const uint32_t* 
     // Each block's warps need cap survivor keys; fewer blocks (a longer grid
     // stride) when the budget leaves less room.
     const uint64_t per_block = pointwise_block_bytes(c);
-    set_spare(c, "refine_keys", false);
-    const uint64_t held_other = c.held - scratch_bytes(c, "refine_keys") - spare_bytes(c);
+    spare_done(c, kSpareKeys, kSpareKeys);
+    const uint64_t held_other = c.held - spare_bytes(c);
     const uint64_t room = c.budget > held_other + (16ull << 20) ? c.budget - held_other - (16ull << 20) : 0;
     blocks = static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>(blocks, room / per_block)));
     const auto [keys, changed] = pointwise_scratch(c, blocks);
@@ -1158,37 +1157,31 @@ uint64_t run_refine_pointwise(Context& c, const uint32_t* snap, const uint32_t* 
 
 namespace {
 
-// The lists of a join pass, and what they take for n points, ranges of `step`.
-// A join takes up to all of the budget for them, so but during the pass they are
-// spare: whatever is allocated then, the finished lists or the next pass's
-// snapshot for instance, may have their room.
+// The lists of a join pass.  A join takes up to all of the budget for them, so
+// they are spare buffers: the finished lists or the next pass's snapshot, for
+// instance, may have their room.  This object gives them back at a pass's end.
 struct PassLists {
-    static constexpr const char* kNames[] = {"refine_snap_d", "rev_count",  "rev_cursor", "rev_offsets",
-                                             "rev_ids",       "join_masks", "apply_big",  "apply_lost"};
+    static constexpr int kFirst = kSpareSnapD, kLast = kSpareLost;
     Context& c;
     explicit PassLists(Context& ctx) : c(ctx) {}
-    ~PassLists() {
-        mark(true);
-        set_spare(c, "refine_keys", true);
-    }
-    void mark(bool spare) {
-        for (const char* name : kNames) set_spare(c, name, spare);
-    }
+    ~PassLists() { spare_done(c, kSpareSnapD, kSpareKeys); }
     // Keeps those of the last pass that are large enough, unless (its ranges may
     // have been larger) they would leave less than `reserve` of the budget.
-    void take(const uint64_t (&need)[std::size(kNames)], uint64_t reserve) {
-        mark(false);
-        uint64_t more = 0;
-        for (size_t i = 0; i < std::size(kNames); ++i)
-            if (scratch_bytes(c, kNames[i]) < need[i]) {
-                scratch_free(c, kNames[i]);
-                more += need[i];
-            }
-        if (c.held - spare_bytes(c) + more + reserve > c.budget)
-            for (const char* name : kNames) scratch_free(c, name);
-        for (size_t i = 0; i < std::size(kNames); ++i) ptr[i] = scratch(c, kNames[i], need[i]);
+    void take(const uint64_t (&need)[kLast - kFirst + 1], uint64_t reserve) {
+        uint64_t all = 0;
+        for (int i = kFirst; i <= kLast; ++i) {
+            if (c.spare[i].bytes < need[i - kFirst]) spare_free(c, static_cast<SpareBuffer>(i));
+            all += std::max<uint64_t>(c.spare[i].bytes, need[i - kFirst]);
+        }
+        if (c.held - spare_bytes(c) + all + reserve > c.budget)
+            for (int i = kFirst; i <= kLast; ++i) spare_free(c, static_cast<SpareBuffer>(i));
+        for (int i = kFirst; i <= kLast; ++i) c.spare_in_use |= 1u << i;
+        for (int i = kFirst; i <= kLast; ++i) spare_take(c, static_cast<SpareBuffer>(i), need[i - kFirst]);
     }
-    void* ptr[std::size(kNames)] = {};
+    template <class T>
+    T* list(SpareBuffer which) const {
+        return static_cast<T*>(c.spare[which].ptr);
+    }
 };
 
 }  // namespace
@@ -1269,14 +1262,14 @@ uint64_t run_refine(Context& c) {
                 point * sizeof(unsigned long long), edges * sizeof(uint32_t), edges * sizeof(uint4),
                 step * sizeof(uint32_t), step * sizeof(uint32_t)},
                reserve);
-    auto* snap_d = static_cast<float*>(lists.ptr[0]);
-    auto* cnt = static_cast<uint32_t*>(lists.ptr[1]);
-    auto* cur = static_cast<uint32_t*>(lists.ptr[2]);
-    auto* off = static_cast<unsigned long long*>(lists.ptr[3]);
-    auto* rev = static_cast<uint32_t*>(lists.ptr[4]);
-    auto* masks = static_cast<uint4*>(lists.ptr[5]);
-    auto* big = static_cast<uint32_t*>(lists.ptr[6]);
-    auto* lost = static_cast<uint32_t*>(lists.ptr[7]);
+    auto* snap_d = lists.list<float>(kSpareSnapD);
+    auto* cnt = lists.list<uint32_t>(kSpareRevCount);
+    auto* cur = lists.list<uint32_t>(kSpareRevCursor);
+    auto* off = lists.list<unsigned long long>(kSpareRevOffsets);
+    auto* rev = lists.list<uint32_t>(kSpareRevIds);
+    auto* masks = lists.list<uint4>(kSpareMasks);
+    auto* big = lists.list<uint32_t>(kSpareBig);
+    auto* lost = lists.list<uint32_t>(kSpareLost);
     snapshot(c.dists_own ? snap_d : nullptr);
     if (!c.dists_own) {
         KNNG_DISPATCH_D(c.d, {
