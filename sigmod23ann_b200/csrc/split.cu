@@ -1253,18 +1253,26 @@ void release_buffers(Context& c, DevRep& r) {
 
 // Buffers for the context's points and sets at bucket bound `max_leaf`.
 DevRep& ensure_devrep(Context& c, uint32_t max_leaf, uint32_t small_threshold) {
-    if (!c.devrep) {
-        c.devrep = new DevRep();
-        for (auto& e : c.devrep->ev) KNNG_CUDA(cudaEventCreate(&e));
-        c.devrep->h_params = static_cast<uint64_t*>(pinned_take(4 * sizeof(uint64_t)));
-        if (!c.devrep->h_params) fail(KNNG_ERR_OUT_OF_MEMORY, "no pinned host memory");
-    }
+    if (!c.devrep) c.devrep = new DevRep();
     DevRep& r = *c.devrep;
+    for (auto& e : r.ev)
+        if (!e) KNNG_CUDA(cudaEventCreate(&e));
+    if (!r.h_params) r.h_params = static_cast<uint64_t*>(pinned_take(4 * sizeof(uint64_t)));
+    if (!r.h_params) fail(KNNG_ERR_OUT_OF_MEMORY, "no pinned host memory");
     const bool same = r.n == c.n && r.h_set_offsets == c.set_offsets && r.min_leaf <= max_leaf &&
                       r.small_threshold == small_threshold;
     if (same) return r;
     KNNG_CUDA(cudaStreamSynchronize(c.stream));
     release_buffers(c, r);
+    // A failure below leaves no buffers, and so a record that fits no point set.
+    struct Whole {
+        Context& c;
+        DevRep& r;
+        bool done = false;
+        ~Whole() {
+            if (!done) release_buffers(c, r);
+        }
+    } whole{c, r};
     r.n = c.n;
     r.h_set_offsets = c.set_offsets;
     r.nsets = static_cast<uint32_t>(c.set_offsets.size() - 1);
@@ -1323,6 +1331,7 @@ DevRep& ensure_devrep(Context& c, uint32_t max_leaf, uint32_t small_threshold) {
     r.item_true = rep_alloc<uint32_t>(c, r, r.part_item_cap + 1);
     r.prefix = rep_alloc<uint32_t>(c, r, r.part_item_cap + 1);
     KNNG_CUDA(cudaStreamSynchronize(c.stream));
+    whole.done = true;
     return r;
 }
 

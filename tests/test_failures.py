@@ -132,3 +132,27 @@ def test_a_pass_in_ranges_is_whole_or_not_started(knng_lib, monkeypatch, fails_i
                 assert a.refine(st) == changed
                 assert _same_sets(want, a.sets())
                 assert st.refine_join_launches == fails_in + 1 and st.refine_lost > 0
+
+
+def test_a_repetition_that_found_no_room_leaves_nothing_half_made(knng_lib):
+    """A budget that holds the points and sets but not a repetition's buffers: each
+    try is refused anew, on the same context, and one that fits then runs."""
+    n, d = 20_000, 64
+    pts = workloads.gaussian_mixture(n=n, d=d, clusters=8, sigma=0.2, seed=35)
+    few = default_params(k=10, reps=2, refine=0, max_leaf=129, max_leaf_odd=0, lloyd_iters=1, seed=3)
+    many = default_params(k=64, reps=2, refine=0, max_leaf=129, max_leaf_odd=0, lloyd_iters=1, seed=3)
+    with KnngContext(0) as ref:
+        want = ref.build(pts, few)
+    for room in (0, 100 << 10, 300 << 10, 500 << 10):
+        with KnngContext(0, n * (4 * d + 8 + 8 * 64 + 12) + room) as ctx:
+            for _ in range(3):
+                with pytest.raises(KnngError) as e:
+                    ctx.build(pts, many)
+                assert e.value.status == 4
+            ctx.load_points(pts)
+            ctx.reset_sets(64)
+            for _ in range(2):
+                with pytest.raises(KnngError) as e:
+                    ctx.run_rep(129, 1, 3000, seed=3, rep_index=0)
+                assert e.value.status == 4
+            assert np.array_equal(ctx.build(pts, few), want)
