@@ -401,11 +401,16 @@ void alloc_sets(Context& c, uint32_t k) {
     free_sets(c);
     c.k = k;
     const size_t nk = static_cast<size_t>(c.n) * k;
-    c.set_dist = static_cast<float*>(dev_alloc(c, nk * sizeof(float)));
-    c.set_id = static_cast<uint32_t*>(dev_alloc(c, nk * sizeof(uint32_t)));
-    c.set_size = static_cast<uint32_t*>(dev_alloc(c, c.n * sizeof(uint32_t)));
-    c.set_maxslot = static_cast<uint32_t*>(dev_alloc(c, c.n * sizeof(uint32_t)));
-    c.set_bound = static_cast<float*>(dev_alloc(c, c.n * sizeof(float)));
+    try {
+        c.set_dist = static_cast<float*>(dev_alloc(c, nk * sizeof(float)));
+        c.set_id = static_cast<uint32_t*>(dev_alloc(c, nk * sizeof(uint32_t)));
+        c.set_size = static_cast<uint32_t*>(dev_alloc(c, c.n * sizeof(uint32_t)));
+        c.set_maxslot = static_cast<uint32_t*>(dev_alloc(c, c.n * sizeof(uint32_t)));
+        c.set_bound = static_cast<float*>(dev_alloc(c, c.n * sizeof(float)));
+    } catch (...) {  // all of them or none
+        free_sets(c);
+        throw;
+    }
     launch_reset_sets(c);
 }
 
@@ -426,8 +431,13 @@ void load_points(Context& c, const float* pts, uint32_t n, uint32_t d, uint64_t 
         c.n = n;
         c.d = d;
         c.ld = d;  // supported dims are multiples of 4: rows stay 16-byte aligned
-        c.indices = static_cast<uint32_t*>(dev_alloc(c, static_cast<size_t>(n) * sizeof(uint32_t)));
-        c.indices_tmp = static_cast<uint32_t*>(dev_alloc(c, static_cast<size_t>(n) * sizeof(uint32_t)));
+        try {
+            c.indices = static_cast<uint32_t*>(dev_alloc(c, static_cast<size_t>(n) * sizeof(uint32_t)));
+            c.indices_tmp = static_cast<uint32_t*>(dev_alloc(c, static_cast<size_t>(n) * sizeof(uint32_t)));
+        } catch (...) {
+            release_all(c);
+            throw;
+        }
         if (had_sets) c.k = k;
     }
     const size_t row = static_cast<size_t>(d) * sizeof(float);

@@ -156,3 +156,31 @@ def test_a_repetition_that_found_no_room_leaves_nothing_half_made(knng_lib):
                     ctx.run_rep(129, 1, 3000, seed=3, rep_index=0)
                 assert e.value.status == 4
             assert np.array_equal(ctx.build(pts, few), want)
+
+
+def test_sets_that_found_no_room_are_not_there(knng_lib):
+    """A budget that holds some of the sets' arrays: the call is refused, stage calls
+    then answer that there are no sets, and shorter lists that fit run."""
+    n, d = 6_000, 64
+    pts = workloads.gaussian_mixture(n=n, d=d, clusters=8, sigma=0.2, seed=36)
+    with KnngContext(0) as ref:
+        ref.load_points(pts)
+        ref.reset_sets(10)
+        ref.run_rep(129, 1, 3000, seed=3, rep_index=0)
+        want = ref.sets()
+    # The distances fit, then the ids, the sizes, the slots too; never the bounds.
+    for part in (4 * 128, 8 * 128, 8 * 128 + 4, 8 * 128 + 8):
+        with KnngContext(0, n * (4 * d + 8 + part) + n * 2) as ctx:
+            ctx.load_points(pts)
+            for _ in range(2):
+                with pytest.raises(KnngError) as e:
+                    ctx.reset_sets(128)
+                assert e.value.status == 4
+                for call in (lambda: ctx.run_rep(129, 1, 3000, seed=3, rep_index=0), ctx.refine,
+                             lambda: ctx.process_leaves([0], [n])):
+                    with pytest.raises(KnngError) as e:
+                        call()
+                    assert e.value.status in (1, 5)
+            ctx.reset_sets(10)
+            ctx.run_rep(129, 1, 3000, seed=3, rep_index=0)
+            assert _same_sets(want, ctx.sets())
