@@ -107,3 +107,25 @@ def test_kd_sums_at_batch_and_chunk_edges(oracle_lib, knng_lib, n, nd, leaf):
         ctx.reset_sets(10)
         ctx.run_rep_kd(leaf, nd, 99, 0)
         np.testing.assert_array_equal(ctx.indices(), o.indices())
+
+
+def test_list_lengths_in_turn_on_one_context(knng_lib):
+    """The captured repetition is kept by the arrays it was captured with: lists of
+    several lengths in turn, the sets' arrays allocated anew each time and other
+    memory taken between, give the lists of fresh contexts."""
+    from sigmod23ann_b200 import default_params
+
+    pts = workloads.gaussian_mixture(n=7000, d=64, clusters=8, sigma=0.2, seed=41)
+
+    def params(k: int):
+        return default_params(k=k, reps=2, refine=1, max_leaf=257, max_leaf_odd=0, lloyd_iters=1, seed=2)
+
+    want = {}
+    for k in (100, 10, 77, 99):
+        with KnngContext(0) as c:
+            want[k] = c.build(pts, params(k), want_dists=True)
+    with KnngContext(0) as c:
+        for k in (100, 10, 100, 77, 99, 10, 100, 99, 77, 100):
+            ids, dists = c.build(pts, params(k), want_dists=True)
+            assert np.array_equal(ids, want[k][0]), k
+            assert np.array_equal(dists.view(np.uint32), want[k][1].view(np.uint32)), k
