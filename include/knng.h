@@ -103,7 +103,8 @@ typedef struct knng_stats {
     uint64_t refine_overflow; /* points whose candidates a warp's tables did not hold (redone by a CTA) */
     double ms_refine_prep;    /* refinement: snapshot, reverse lists, scans */
     uint64_t refine_join_launches; /* join-kernel launches (one per range of points) */
-    uint64_t refine_lost;     /* points redone by the per-point pass (past a CTA's tables) */
+    uint64_t refine_lost;     /* points redone by the per-point pass (past a CTA's tables, or a range's
+                                 join gave up) */
     uint64_t refine_passes_done; /* neighbour-of-neighbour passes run, whichever kernel ran them */
     double recall_estimate;   /* knng_build_adaptive: recall on its sample at the end */
     uint64_t estimate_queries;/* knng_build_adaptive: sampled points */
@@ -402,7 +403,9 @@ typedef struct knng_job_info {
 } knng_job_info;
 
 /* HBM a job of n points, d dims, k neighbours reserves: points, order, sets,
- * refinement lists and survivor storage, plus fixed scratch. */
+ * a pass's snapshots and 96 bytes per neighbour-list entry for its other lists
+ * and the finished ones, plus fixed scratch.  It is more than a build holds
+ * (about 2.2 times at 2,000,000 x 100, k = 100). */
 uint64_t knng_job_reservation(uint32_t n, uint32_t d, uint32_t k);
 
 /* A server on `device` with an HBM budget (0: 80% of the device's memory) and

@@ -12,8 +12,10 @@
 // Distances are computed for the full b x b matrix (both triangles); each
 // (i, j) and (j, i) evaluation gives the same bits.
 // k_leaf_tc makes the same offers but computes distances only for the pairs
-// a tensor-core filter cannot rule out (see below); it is the slower of the
-// two at 10M points, where the sequential set updates dominate.
+// a tensor-core filter cannot rule out (see below).  It is the slower of the two
+// (139 ms against 85 a repetition at 10M points): it has a CTA per bucket, blocks
+// of 64 x 64 with a conversion and an MMA round trip each, and a containment
+// check in every offer, none of which k_leaf has.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -817,7 +819,8 @@ namespace {
 // Rows of a block of the FP32 pass: 32 (two a warp) once the points make a block
 // for each of two CTAs an SM, else 16.  64 loads the fewest column tiles per
 // pair, but four sets a warp spill and short buckets waste rows: 2M x 100
-// 130 ms against 125 (four repetitions), 100k x 100 5.6 against 4.7 (eight).
+// 130 ms against 125 (four repetitions), 100k x 100 5.6 against 4.7 (eight), both
+// measured with blocks of 64 columns and not again with the 128 of now.
 uint32_t leaf_rows(const Context& c) { return c.n >= 2u * c.sms * 2u * kLeafWarps ? 2u * kLeafWarps : kLeafWarps; }
 
 // The bucket pass over the buckets [0, count) or [0, *dcount): its items, then

@@ -153,7 +153,10 @@ uint64_t knng_job_reservation(uint32_t n, uint32_t d, uint32_t k) {
     const uint64_t order = N * 8;                   // permutation + scatter buffer
     const uint64_t sets = N * (K * 8 + 12);         // distances, ids, size, max slot, bound
     const uint64_t refine = N * K * 8 + N * 40;     // snapshot, reverse lists, counts and offsets
-    const uint64_t survivors = N * K * 96;          // per-point slots and pool of the join
+    // 96 bytes an entry: a pass's own lists take 24 (edges' bits and reverse
+    // entries, distances) and the finished lists 8; the rest is slack, from a join
+    // that wrote its survivors out as records.
+    const uint64_t survivors = N * K * 96;
     const uint64_t fixed = 256ull << 20;            // split, leaf and scan scratch
     return points + order + sets + refine + survivors + fixed;
 }
