@@ -409,6 +409,7 @@ void alloc_sets(Context& c, uint32_t k) {
         c.set_bound = static_cast<float*>(dev_alloc(c, c.n * sizeof(float)));
     } catch (...) {  // all of them or none
         free_sets(c);
+        c.k = 0;
         throw;
     }
     launch_reset_sets(c);

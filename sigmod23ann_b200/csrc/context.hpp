@@ -34,8 +34,8 @@ struct DeviceBuffer {
 // that the budget has no other room for.
 enum SpareBuffer {
     kSpareLeafLists,  // work items of a bucket pass over a host list (and norms)
-    // A join pass: list distances, counts, cursors and offsets of the reverse
-    // lists, these, the edges' bits, the queues of the replay.
+    // A join pass: the snapshot's distances; the reverse lists' counts, cursors,
+    // offsets and entries; the edges' bits; the replay's two queues.
     kSpareSnapD,
     kSpareRevCount,
     kSpareRevCursor,

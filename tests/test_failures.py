@@ -181,6 +181,7 @@ def test_sets_that_found_no_room_are_not_there(knng_lib):
                     with pytest.raises(KnngError) as e:
                         call()
                     assert e.value.status in (1, 5)
+                ctx.load_points(pts)  # brings back no sets, and is not refused for them
             ctx.reset_sets(10)
             ctx.run_rep(129, 1, 3000, seed=3, rep_index=0)
             assert _same_sets(want, ctx.sets())
